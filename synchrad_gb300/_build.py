@@ -26,6 +26,8 @@ SOURCES = {
     "sr_far_mixed.cu": [],
     "sr_far_df.cu": [],
     "sr_near_mixed.cu": [],
+    "sr_fast_far.cu": [],
+    "sr_fast_near.cu": [],
     "sr_far_adjoint.cu": [],
     "sr_diag.cu": [],
     "sr_noalloc.cu": [],

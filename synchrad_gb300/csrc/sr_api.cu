@@ -3,6 +3,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <set>
+#include <tuple>
 
 #include "sr_common.cuh"
 #include "sr_internal.h"
@@ -125,6 +128,20 @@ FarMixedParams make_far_mixed_params(const sr_tracks *t, const sr_grid *g, int c
   return far_mixed_params(t, g, comp, out);
 }
 int device_sm_count() { return n_sm_of_current_device(); }
+
+cudaError_t allow_smem(const void *kernel, int bytes) {
+  static std::mutex mu;
+  static std::set<std::tuple<int, const void *, int>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, kernel, bytes);
+  if (done.count(key)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.insert(key);
+  return e;
+}
 
 }  // namespace sr
 

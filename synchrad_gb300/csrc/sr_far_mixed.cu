@@ -59,6 +59,7 @@ namespace {
 // ------------------------------------------------------------------------
 template <typename TT>
 __global__ void far_prepass_kernel(FarMixedParams p) {
+  fast_tables(p);
   const TT *X = (const TT *)p.x, *Y = (const TT *)p.y, *Z = (const TT *)p.z;
   const TT *UX = (const TT *)p.ux, *UY = (const TT *)p.uy, *UZ = (const TT *)p.uz;
   const double dtInv = 1.0 / p.dt;
@@ -154,6 +155,7 @@ struct SmemFixed {
 // rotation chains of K/2), L lanes per direction, 32/L directions per warp.
 template <int K, int W>
 __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) {
+  if (by_transform(p)) return;
   static_assert(K % 4 == 0 && K >= 4 && K <= 32, "K");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SmemFixed<W> &sm = *reinterpret_cast<SmemFixed<W> *>(smem_raw);
@@ -790,8 +792,7 @@ int launch_main(const FarMixedParams &p, int grid, cudaStream_t s) {
                 "work shape needs %zu bytes of shared memory per CTA (at most %zu): fewer "
                 "steps per stage or more lanes per direction",
                 smem, kMaxSmemPerCta);
-  cudaError_t e = cudaFuncSetAttribute(far_mixed_kernel<K, kW>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem((const void *)far_mixed_kernel<K, kW>, (int)kMaxSmemPerCta);
   if (e != cudaSuccess) return cuda_fail(e, "far_mixed smem attribute");
   far_mixed_kernel<K, kW><<<grid, kW * 32, smem, s>>>(p);
   return cuda_fail(cudaGetLastError(), "far_mixed kernel launch");
@@ -829,6 +830,11 @@ FarMixedConfig far_mixed_make(uint32_t n_omega, uint32_t n_dirs, uint32_t n_trac
   FarMixedConfig c;
   c.W = kW;
   c.ctas_per_sm = 1;
+  c.direct = false;
+  c.n_omega = n_omega;
+  c.n_dirs = n_dirs;
+  c.n_tracks = n_tracks;
+  c.n_sm = n_sm;
   c.K = K;
   c.L = L;
   c.dpw = 32 / L;
@@ -863,9 +869,11 @@ size_t far_mixed_workspace(int64_t total_steps, uint64_t n_points, int n_out, ui
                            const FarMixedConfig &cfg) {
   size_t b = 256;                                                    // status word
   b += ((size_t)total_steps * kRecBytes + 255) / 256 * 256;          // step records
-  b += ((size_t)cfg.n_sub * n_out * n_snaps * n_points * 8 + 255) / 256 * 256;  // partials
+  const FastLayout l = fast_layout(cfg, false, total_steps, n_out, n_snaps);
+  b += ((size_t)std::max((uint32_t)cfg.n_sub, l.n_sub) * n_out * n_snaps * n_points * 8 + 255) /
+       256 * 256;  // partials
   b += (size_t)cfg.grid * cfg.W * cfg.K * 8 * 32 * sizeof(float);   // compensated sums
-  return b;
+  return (b + 255) / 256 * 256 + fast_workspace(l);
 }
 
 int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size_t ws_bytes,
@@ -880,11 +888,16 @@ int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size
   size_t off = 256;
   p.status = (int *)w;
   p.queue = (unsigned int *)(w + 128);  // in the zeroed 256-byte status block
+  const FastLayout fl = fast_layout(cfg, false, p.total_steps, p.n_out, p.n_snaps);
+  p.partial = (double *)(w + off);
+  const size_t partial_bytes =
+      (size_t)std::max((uint32_t)cfg.n_sub, fl.n_sub) * p.n_out * p.n_snaps * P * 8;
+  off += (partial_bytes + 255) / 256 * 256;
   p.records = (float4 *)(w + off);
   off += ((size_t)p.total_steps * kRecBytes + 255) / 256 * 256;
-  p.partial = (double *)(w + off);
-  off += ((size_t)cfg.n_sub * p.n_out * p.n_snaps * P * 8 + 255) / 256 * 256;
   p.outer = (float *)(w + off);
+  off += ((size_t)cfg.grid * cfg.W * cfg.K * 8 * 32 * sizeof(float) + 255) / 256 * 256;
+  fast_bind(p, fl, false, w + off, w);
   p.dpw = (uint32_t)cfg.dpw;
   p.n_wtiles = (p.n_omega + (uint32_t)(cfg.L * cfg.K) - 1) / (uint32_t)(cfg.L * cfg.K);
   const uint32_t n_dirs = p.n_theta * p.n_phi;
@@ -897,10 +910,9 @@ int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size
   p.stage_steps = (uint32_t)cfg.stage;
   p.fold_stages = (uint32_t)std::max(1, 2048 / cfg.stage);  // fold about every 2048 steps
 
-  cudaError_t e = cudaMemsetAsync(w, 0, 256, stream);
-  if (e != cudaSuccess) return cuda_fail(e, "status reset");
-  e = cudaMemsetAsync(p.partial, 0, (size_t)p.n_sub * p.n_out * p.n_snaps * P * 8, stream);
-  if (e != cudaSuccess) return cuda_fail(e, "partial reset");
+  // status block and partial spectra, one after the other
+  cudaError_t e = cudaMemsetAsync(w, 0, 256 + partial_bytes, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "status and partial reset");
 
   int dev = 0, n_sm = 0;
   cudaGetDevice(&dev);
@@ -909,6 +921,7 @@ int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size
     const int blk = 256;
     int64_t nb = (p.total_steps + blk - 1) / blk;
     if (nb > 8 * n_sm * 16) nb = 8 * n_sm * 16;
+    if (nb < 16) nb = 16;  // the tables' FP64 functions spread over the SMs
     if (p.track_f32)
       far_prepass_kernel<float><<<(int)nb, blk, 0, stream>>>(p);
     else
@@ -918,7 +931,8 @@ int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size
   }
   void *tok = nullptr;
   timing_record(stream, true, &tok);
-  int rc = dispatch_k(cfg.K, p, cfg.grid, stream);
+  int rc = fl.on ? launch_fast_far(p, fl, stream) : SR_OK;
+  if (rc == SR_OK) rc = dispatch_k(cfg.K, p, cfg.grid, stream);
   timing_record(stream, false, &tok);
   if (rc) return rc;
   const uint64_t total = (uint64_t)p.n_out * p.n_snaps * P;

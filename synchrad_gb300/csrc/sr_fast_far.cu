@@ -1,0 +1,141 @@
+// Far-field instances of the summation by transforms, and its work split.
+#include <algorithm>
+#include <cmath>
+
+#include "sr_fast_sum.cuh"
+
+namespace sr {
+
+namespace {
+size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+constexpr size_t kTables = (kFastMaxBand + 2) * 8 + 1024 * 16;
+}  // namespace
+
+FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
+                       uint32_t n_snaps) {
+  FastLayout l{};
+  if (c.direct || c.n_omega < 4 || c.n_dirs == 0 || c.n_tracks == 0 || n_snaps == 0 ||
+      total_steps <= 0)
+    return l;
+  const uint64_t mean = (uint64_t)total_steps / c.n_tracks;
+  // The term-by-term kernel walks a track's steps one after the other, this
+  // sum splits them; below some hundred steps its extra launches and circles
+  // cost more than that.  Measured on one undulator track, 16 directions, 64
+  // frequencies (us, transforms / term by term): far 87 / 76 at 200 steps,
+  // 109 / 353 at 2000; near 128 / 92 and 263 / 440.  From 64 tracks on the
+  // transforms win at 200 steps too (147 / 243, 232 / 293 with 200 tracks),
+  // and in the far field with 129 to 256 frequencies (118 / 143), where the
+  // term-by-term work has doubled and the circles are still small.
+  const uint64_t least = near ? 512 : c.n_omega > 128 && c.n_omega <= 256 ? 160 : 320;
+  if (c.n_tracks < 64 && mean < least) return l;
+  l.on = true;
+  const int np = near ? 3 : 1;
+  l.n_bands = (c.n_omega + kFastMaxBand - 1) / kFastMaxBand;
+  l.nb = (c.n_omega + l.n_bands - 1) / l.n_bands;
+  l.M = 128;
+  while (l.M < 2 * l.nb) l.M *= 2;
+  l.n_dwb = (c.n_dirs + 31) / 32 * l.n_bands;
+  l.slice_bytes = up256((size_t)32 * (np * (size_t)(l.M + 2 * l.nb) * 16 +
+                                      kFastList * (16 + 8 * (size_t)np)));
+  // Steps between two writes of the whole window: 128, fewer where they could
+  // lap the circle (a step moves by up to M / (2 nb) cells).
+  l.block = 128;
+  while (l.block > 32 && (uint64_t)l.block * l.M + 16ull * l.nb > 2ull * l.nb * l.M) l.block /= 2;
+  const uint64_t resident = (uint64_t)c.n_sm * (near ? 2 : 3) * kFastWarps;
+  const uint64_t units = (uint64_t)c.n_tracks * l.n_dwb;
+  l.dirs_per_warp = std::max(1u, 512u / l.M);
+  const uint64_t P = (uint64_t)c.n_omega * c.n_dirs;
+  // Few (track, 32 directions) units: their steps are split in segments of a
+  // block, after which a whole track's window is written out too, so that the
+  // sums come out the same either way (a batch streamed in chunks
+  // gives what one call gives).  Larger circles take longer segments: each one
+  // is cleared and read once per segment (~4 TB/s) while a step takes ~0.4 us,
+  // shortest together at sqrt(steps x bytes / (4e12 x 0.4e-6)).  Where that
+  // leaves more than four units per resident warp or 4 GiB, segments grow for
+  // the few long tracks that would not fill the SMs, else tracks stay whole.
+  if (n_snaps == 1 && units <= resident) {
+    const uint64_t all = (uint64_t)total_steps * l.n_dwb;
+    const uint64_t room = (4ull << 30) / l.slice_bytes;
+    uint64_t seg = l.block;
+    if (l.M >= 512)
+      seg = std::max<uint64_t>(
+          seg, (uint64_t)(std::sqrt((double)all * (2.0 * np * l.M * 512.0) / 1.6e6) / 128.0) * 128);
+    bool split = true;
+    if (all / seg + units > room) {
+      split = 2 * units < resident || l.M >= 512;
+      const uint64_t most =
+          std::max<uint64_t>(2 * resident, std::min<uint64_t>(4 * resident, room));
+      seg = std::max<uint64_t>(seg, (all / (most - units) / 128 + 1) * 128);
+    }
+    if (split && (uint64_t)total_steps > seg) {
+      l.split = true;
+      l.seg_steps = (uint32_t)std::min<uint64_t>(seg, 0xffffff00u);
+      l.n_segs = (uint32_t)((uint64_t)total_steps / seg + c.n_tracks);
+    }
+  }
+  // Several snapshots: a unit per interval between them; a snapshot's
+  // transform adds up the circles of the intervals before it.
+  if (n_snaps > 1 && n_snaps <= 16 && units <= resident &&
+      units * n_snaps * l.slice_bytes <= (4ull << 30)) {
+    l.split = true;
+    l.seg_steps = 0;
+    l.n_segs = c.n_tracks * n_snaps;
+  }
+  uint64_t subs;
+  if (l.split) {
+    const uint64_t groups = (uint64_t)l.n_dwb * (32u / l.dirs_per_warp) * n_snaps;
+    subs = (resident + groups - 1) / groups;
+  } else {
+    subs = (8 * resident + l.n_dwb - 1) / l.n_dwb;
+  }
+  // partial spectra of at most 1 GiB, or one
+  const uint64_t room = (1ull << 30) / std::max<uint64_t>(1, P * n_out * n_snaps * 8);
+  subs = std::max<uint64_t>(1, std::min({subs, room, (uint64_t)c.n_tracks}));
+  l.n_sub = (uint32_t)subs;
+  const uint64_t warps = l.split ? (uint64_t)l.n_segs * l.n_dwb : std::min(resident, l.n_dwb * subs);
+  l.slices = (uint32_t)((warps + kFastWarps - 1) / kFastWarps * kFastWarps);
+  return l;
+}
+
+size_t fast_workspace(const FastLayout &l) {
+  if (!l.on) return 0;
+  return up256(kTables) + up256((size_t)l.slices * 4) + (size_t)l.slices * l.slice_bytes;
+}
+
+void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
+               unsigned char *status) {
+  FastParams &f = p.fast;
+  if (!l.on) {
+    f.uneven = nullptr;
+    return;
+  }
+  f.uneven = (unsigned int *)(status + 64);
+  f.queue = (unsigned int *)(status + 192);
+  f.deconv = (double *)base;
+  f.twiddle = (float4 *)(base + (kFastMaxBand + 2) * 8);
+  base += up256(kTables);
+  f.dirty = (unsigned int *)base;
+  base += up256((size_t)l.slices * 4);
+  f.scratch = base;
+  f.slice_bytes = l.slice_bytes;
+  f.n_bands = l.n_bands;
+  f.nb = l.nb;
+  f.M = l.M;
+  f.n_dwb = l.n_dwb;
+  f.n_sub = l.n_sub;
+  f.n_segs = l.n_segs;
+  f.seg_steps = l.seg_steps;
+  f.block = l.block;
+  f.dirs_per_warp = l.dirs_per_warp;
+  // phi nodes spanned by 32 consecutive directions, and the steps whose turned
+  // records of all of them fit the staging buffer (128 records)
+  f.n_phik = near ? 1u : std::min(p.n_phi, (p.n_theta + 30u) / p.n_theta + 1u);
+  f.chunk = 32u;
+  while (!near && f.chunk * f.n_phik > 128u) f.chunk /= 2u;
+}
+
+int launch_fast_far(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
+  return launch_fast<false>(p, l, s);
+}
+
+}  // namespace sr

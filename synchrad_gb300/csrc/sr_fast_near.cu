@@ -1,0 +1,10 @@
+// Near-field instances of the summation by transforms.
+#include "sr_fast_sum.cuh"
+
+namespace sr {
+
+int launch_fast_near(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
+  return launch_fast<true>(p, l, s);
+}
+
+}  // namespace sr

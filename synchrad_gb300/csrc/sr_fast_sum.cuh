@@ -1,0 +1,1168 @@
+// Spectral sums over track steps on an evenly spaced omega axis through a
+// transform over the steps: the kernels shared by the mixed-precision far and
+// near fields.
+//
+// Both fields need, per direction (screen point) and track,
+//     A_j = sum_s v_s exp(i omega_j tau_s),  omega_j = omega_0 + j d_omega,
+// a discrete Fourier sum with uneven times tau_s.  Term by term it costs
+// N x steps products; here each step is spread with a smooth kernel of kTaps
+// cells onto a circle of M >= 2 N cells of the phase d_omega tau mod 2 pi,
+// one M-point FFT per (track, direction, component) turns the cells into the
+// sums and a division by the kernel's transform undoes the spreading (the
+// nonuniform FFT of Dutt & Rokhlin, SIAM J. Sci. Comput. 14 (1993), with the
+// Kaiser-Bessel kernel of Jackson et al., IEEE TMI 10 (1991), beta from Beatty
+// et al., IEEE TMI 24 (2005)).  The kernel's aliasing is below 3e-8 of the sum
+// at kTaps = 8 and M = 2 N, under the rounding of the FP32 terms.
+//
+// tau grows along a track, so the steps of a direction sweep the circle: a
+// lane owns one direction and holds the kTaps cells around the current step
+// in registers; when the step moves on by one cell the oldest one is complete
+// and leaves for the lane's circle in global memory (red.v4.f32: the lane is
+// the only writer of its circle, so the order of the sums is fixed).  The
+// per-(direction, step) values (double-float tau, amplitudes) are computed
+// once for all frequencies, by the lane itself.
+//
+// A step enters when omega |dtau| < pi at every frequency of the band with the
+// guard band to spare (kPiLo).  A step that the rule cuts inside the band, or
+// whose band edge lies in the guard band, goes to a short list per lane; the
+// warp empties the lists by direct sums over the included frequencies, with
+// the exact FP64 test in the guard band.
+#pragma once
+
+#include "sr_mixed_common.cuh"
+
+namespace sr {
+namespace {
+
+constexpr int kTaps = 8;
+constexpr int kFastList = 96;     // list entries per lane (a chunk adds at most 32)
+constexpr int kFastWarps = 4;     // warps per CTA
+// Per-warp shared memory: step records of the current chunk while spreading,
+// the transpose buffer of the FFT otherwise; the first field's outputs; the
+// cos/sin phi of the warp's directions.
+struct FastSmem {
+  union {
+    float4 rec[8704 / 16];
+    float2 tr[32 * 33];
+  };
+  float2 out[kFastMaxBand];
+  float4 phic[32];
+};
+
+// Taps phi(f + 3.5 - l), l = 0..7, for f in [-1/2, 1/2]: degree-8 Chebyshev
+// fits of the Kaiser-Bessel kernel on each cell, even and odd parts shared by
+// the mirrored taps.
+__device__ __forceinline__ void kb_taps(float f, float (&w)[kTaps]) {
+  const float g = f * f;
+  auto pair = [&](int l, float e0, float o0, float e1, float o1, float e2, float o2, float e3,
+                  float o3, float e4) {
+    float e = __fmaf_rn(e4, g, e3);
+    e = __fmaf_rn(e, g, e2);
+    e = __fmaf_rn(e, g, e1);
+    e = __fmaf_rn(e, g, e0);
+    float o = __fmaf_rn(o3, g, o2);
+    o = __fmaf_rn(o, g, o1);
+    o = __fmaf_rn(o, g, o0);
+    w[l] = __fmaf_rn(o, f, e);
+    w[kTaps - 1 - l] = __fmaf_rn(-o, f, e);
+  };
+  pair(0, 9.660679643e-05f, -7.671282510e-04f, 2.600571373e-03f, -4.920937587e-03f,
+       5.659276154e-03f, -3.947199788e-03f, 1.406157040e-03f, 9.299917292e-05f, -2.649927337e-04f);
+  pair(1, 1.900451072e-02f, -6.841991097e-02f, 1.010312214e-01f, -7.361625135e-02f,
+       1.998347044e-02f, 7.933221757e-03f, -7.344931830e-03f, 9.507333161e-04f, 7.229428156e-04f);
+  pair(2, 2.666729093e-01f, -4.878970087e-01f, 2.578946948e-01f, 5.260234699e-02f,
+       -9.378349781e-02f, 1.511092298e-02f, 1.341344323e-02f, -4.336146638e-03f,
+       -9.862204315e-04f);
+  pair(3, 8.674505353e-01f, -4.952890873e-01f, -3.615280092e-01f, 2.447273135e-01f,
+       6.815172732e-02f, -5.749912560e-02f, -7.492190693e-03f, 8.106620982e-03f,
+       4.874356382e-04f);
+}
+
+// One cell's sums added to the lane's circle (no return value, no ordering
+// against other lanes: each circle has one writer).
+__device__ __forceinline__ void red_f4(float4 *p, float2 a, float2 b) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
+                   __cvta_generic_to_global(p)),
+               "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
+               : "memory");
+}
+
+// A term of a partial spectrum (one writer per subset and point: the order of
+// the sum is the order of the tracks).
+__device__ __forceinline__ void red_f64(double *p, double v) {
+  asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+               "d"(v)
+               : "memory");
+}
+__device__ __forceinline__ df df_square(df a) {
+  const float p = a.hi * a.hi;
+  return df{p, __fmaf_rn(a.hi + a.hi, a.lo, __fmaf_rn(a.hi, a.hi, -p))};
+}
+// |x|^2 + |y|^2 of two complex FP32 values, exact to about 2^-46.
+__device__ __forceinline__ df df_norm2(float2 x, float2 y) {
+  const float a = x.x * x.x, b = x.y * x.y, c = y.x * y.x, d = y.y * y.y;
+  const float l = (__fmaf_rn(x.x, x.x, -a) + __fmaf_rn(x.y, x.y, -b)) +
+                  (__fmaf_rn(y.x, y.x, -c) + __fmaf_rn(y.y, y.y, -d));
+  const df s = two_sum(a, b), t = two_sum(c, d);
+  const df r = two_sum(s.hi, t.hi);
+  return df{r.hi, r.lo + ((s.lo + t.lo) + l)};
+}
+
+// exp(2 pi i w tau) as phasor_rev, with the FP32 library's sin and cos: one
+// seed serves every frequency of the band, so the hardware functions' error
+// (~4e-7) would not average over seeds as it does term by term.
+__device__ __forceinline__ void phasor_exact(float wh, float wl, float th, float tl, float &s,
+                                             float &c) {
+  const float p = wh * th;
+  float e = __fmaf_rn(wh, th, -p);
+  e = __fmaf_rn(wh, tl, e);
+  e = __fmaf_rn(wl, th, e);
+  const float f = (p - rintf(p)) + e;
+  sincospif(f + f, &s, &c);
+}
+
+// cos(2 pi k / 32) as hi + lo.
+__device__ __forceinline__ df cos32(int k) {
+  constexpr float h[9] = {1.f, 0.980785251f, 0.923879504f,
+                          0.831469595f, 0.707106769f, 0.555570245f,
+                          0.382683426f, 0.195090324f, 0.f};
+  constexpr float l[9] = {0.f, 2.97394731e-08f, 2.83074897e-08f,
+                          1.68702634e-08f, 1.21016175e-08f, -1.17695214e-08f,
+                          6.22335072e-09f, -1.67047143e-09f, 0.f};
+  k &= 31;
+  if (k > 16) k = 32 - k;
+  return k <= 8 ? df{h[k], l[k]} : df{-h[16 - k], -l[16 - k]};
+}
+
+// d (c + i s), the factor given as hi + lo: the twiddles are the same for
+// every track, so their rounding would not average over the tracks.
+__device__ __forceinline__ float2 mul_df(float2 d, float ch, float sh, float cl, float sl) {
+  return make_float2(__fmaf_rn(d.x, ch, __fmaf_rn(-d.y, sh, __fmaf_rn(d.x, cl, -d.y * sl))),
+                     __fmaf_rn(d.x, sh, __fmaf_rn(d.y, ch, __fmaf_rn(d.x, sl, d.y * cl))));
+}
+
+// In-place DFT with exp(+2 pi i j k / N) of N = 4, 8, 16 or 32 register
+// values, decimation in frequency; output k is left at index bitrev(k).
+template <int N>
+__device__ __forceinline__ void fft_reg(float2 (&x)[N]) {
+#pragma unroll
+  for (int len = N; len > 1; len >>= 1) {
+#pragma unroll
+    for (int b = 0; b < N; b += len) {
+#pragma unroll
+      for (int j = 0; j < len / 2; ++j) {
+        const float2 u = x[b + j], v = x[b + j + len / 2];
+        x[b + j] = make_float2(u.x + v.x, u.y + v.y);
+        const float2 d = make_float2(u.x - v.x, u.y - v.y);
+        const int k = j * (32 / len);  // twiddle exp(2 pi i k / 32)
+        float2 r;
+        if (k == 0) {
+          r = d;
+        } else if (k == 8) {
+          r = make_float2(-d.y, d.x);
+        } else {
+          const df c = cos32(k), s = cos32(k - 8);
+          r = mul_df(d, c.hi, s.hi, c.lo, s.lo);
+        }
+        x[b + j + len / 2] = r;
+      }
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ constexpr int bitrev(int k) {
+  int r = 0;
+  for (int n = N; n > 1; n >>= 1) {
+    r = (r << 1) | (k & 1);
+    k >>= 1;
+  }
+  return r;
+}
+
+// Second half of the transform of the fields in x: NF fields of M = 32 R1
+// cells (cell 32 i + lane in x[.][i]).  Writes the N band sums of field q to
+// dst[q][j], j = frequency index + N/2 (not yet divided by the kernel's
+// transform).
+template <int R1, int NF>
+__device__ __forceinline__ void fft_band(float2 (&x)[NF][R1], float2 *tr, const float4 *tw,
+                                         int lane, int n, float2 *dst) {
+  static_assert(R1 * NF == 32, "one warp holds 1024 cells");
+#pragma unroll
+  for (int q = 0; q < NF; ++q) {
+    fft_reg<R1>(x[q]);
+#pragma unroll
+    for (int a = 0; a < R1; ++a) {
+      const float2 v = x[q][bitrev<R1>(a)];
+      float2 r = v;
+      if (a) {
+        const float4 t = __ldg(tw + a * 32 + lane);  // exp(2 pi i a lane / M)
+        r = mul_df(v, t.x, t.y, t.z, t.w);
+      }
+      tr[(q * R1 + a) * 33 + lane] = r;
+    }
+  }
+  __syncwarp();
+  float2 y[32];
+#pragma unroll
+  for (int l = 0; l < 32; ++l) y[l] = tr[lane * 33 + l];
+  __syncwarp();
+  fft_reg<32>(y);
+  const int q = lane / R1, a = lane % R1;
+#pragma unroll
+  for (int b = 0; b < 32; ++b) {
+    const int k = a + R1 * b;
+    const int j = (b < 16 ? k : k - 32 * R1) + n / 2;
+    if (j >= 0 && j < n) dst[q * n + j] = y[bitrev<32>(b)];
+  }
+  __syncwarp();
+}
+
+// Values of a direction (far) or screen point (near) that its lane keeps.
+template <bool NEAR>
+struct LaneDir;
+template <>
+struct LaneDir<false> {
+  float dc_h, dc_l, st_h, st_l;  // 1 - cos(theta), sin(theta) as double-floats
+  float f_dc, f_st, f_ct;
+};
+template <>
+struct LaneDir<true> {
+  float X_h, X_l, Y_h, Y_l, L_h, L_l;
+};
+
+// The part of a warp's scratch slice.
+template <bool NEAR>
+struct FastSlice {
+  static constexpr int NP = NEAR ? 3 : 1;  // pairs of complex fields
+  unsigned char *base;
+  __device__ FastSlice(const FastParams &f, size_t i) : base(f.scratch + i * f.slice_bytes) {}
+  // [NP][32][M] cells (X re, X im, Y re, Y im)
+  __device__ float4 *grid() const { return (float4 *)base; }
+  // [NP][32][2][nb] direct sums of the listed steps: sums, then low parts
+  __device__ float4 *part(const FastParams &f) const { return grid() + (size_t)NP * 32 * f.M; }
+  // [32][kFastList] tau.hi, tau.lo, first | last << 16
+  __device__ float4 *lhead(const FastParams &f) const {
+    return grid() + (size_t)NP * 32 * (f.M + 2 * f.nb);
+  }
+  // [NP][32][kFastList] amplitudes X, Y
+  __device__ float2 *lamp(const FastParams &f) const {
+    return (float2 *)(lhead(f) + kFastList * 32);
+  }
+};
+
+// State of one warp's unit of work: 32 directions x one omega band.
+template <bool NEAR>
+struct FastUnit {
+  static constexpr int NP = NEAR ? 3 : 1;
+  uint32_t slot0;      // first direction
+  uint32_t j0;         // first frequency of the band
+  int nb;              // its frequencies
+  df f_c, f_d;         // (centre frequency, d_omega) / 2 pi
+  float wmax, wmin;    // largest and smallest |omega| of the band
+  LaneDir<NEAR> ld;
+  uint32_t dir;
+  bool active;
+  int kphi;            // phi of the lane among the warp's (far)
+};
+
+template <bool NEAR>
+__device__ void unit_init(const FarMixedParams &p, uint32_t dwb, int lane, FastSmem &sm,
+                          FastUnit<NEAR> &u) {
+  const FastParams &f = p.fast;
+  const uint32_t nT = p.n_theta, n_dirs = nT * p.n_phi;
+  const uint32_t band = dwb % f.n_bands;
+  u.slot0 = (dwb / f.n_bands) * 32u;
+  u.j0 = band * f.nb;
+  u.nb = (int)min(f.nb, p.n_omega - u.j0);
+  const double w0 = p.omega[0];
+  const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
+  const double inv2pi = 0.15915494309189533577;
+  u.f_c = df_from_double((w0 + (double)(u.j0 + u.nb / 2) * dw) * inv2pi);
+  u.f_d = df_from_double(dw * inv2pi);
+  const double wa = w0 + (double)u.j0 * dw, wb = w0 + (double)(u.j0 + u.nb - 1) * dw;
+  u.wmax = (float)fmax(fabs(wa), fabs(wb));
+  u.wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
+  u.active = u.slot0 + lane < n_dirs;
+  u.dir = u.active ? u.slot0 + lane : n_dirs - 1;
+  const uint32_t iT = u.dir % nT, iP = u.dir / nT, iP0 = u.slot0 / nT;
+  u.kphi = (int)(iP - iP0);
+  if constexpr (!NEAR) {
+    const df c = df_from_double(1.0 - p.cos_theta[iT]), s = df_from_double(p.sin_theta[iT]);
+    u.ld.dc_h = c.hi; u.ld.dc_l = c.lo; u.ld.st_h = s.hi; u.ld.st_l = s.lo;
+    u.ld.f_dc = (float)(1.0 - p.cos_theta[iT]);
+    u.ld.f_st = (float)p.sin_theta[iT];
+    u.ld.f_ct = (float)p.cos_theta[iT];
+    const uint32_t k = iP0 + lane;
+    if (lane < (int)f.n_phik) {
+      const df cp = df_from_double(p.cos_phi[min(k, p.n_phi - 1)]);
+      const df sp = df_from_double(p.sin_phi[min(k, p.n_phi - 1)]);
+      sm.phic[lane] = make_float4(cp.hi, cp.lo, sp.hi, sp.lo);
+    }
+  } else {
+    const df x = df_from_double(p.sin_theta[iT] * p.cos_phi[iP]);
+    const df y = df_from_double(p.sin_theta[iT] * p.sin_phi[iP]);
+    const df L = df_from_double(p.L_screen);
+    u.ld.X_h = x.hi; u.ld.X_l = x.lo; u.ld.Y_h = y.hi; u.ld.Y_l = y.lo;
+    u.ld.L_h = L.hi; u.ld.L_l = L.lo;
+  }
+  __syncwarp();
+}
+
+// The chunk's step records in shared memory.  Far: per (phi of the warp,
+// step) the record turned into the plane of that phi, so that a lane's
+// tau and amplitudes take its theta alone:
+//   (q.hi, q.lo, z.hi, z.lo) (rho.hi, rho.lo, b_rho, b_z) (1 - b_z, b_phi, a_rho, a_z) (a_phi)
+// with rho = cos(phi) x + sin(phi) y.  Near: the records as they are.
+template <bool NEAR>
+__device__ __forceinline__ void stage_records(const FarMixedParams &p, int64_t g, uint32_t cnt,
+                                              int lane, FastSmem &sm) {
+  const uint32_t cs = p.fast.chunk;
+  const float4 *src = p.records + g * kRecF4;
+  if constexpr (NEAR) {
+    if ((uint32_t)lane < cnt) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sm.rec[lane * 3 + k] = __ldg(src + (size_t)lane * kRecF4 + k);
+    }
+  } else {
+    const uint32_t n = cs * p.fast.n_phik;
+    for (uint32_t i = lane; i < n; i += 32u) {
+      const uint32_t k = i / cs, s = i % cs;
+      if (s >= cnt) continue;
+      const float4 *r = src + (size_t)s * kRecF4;
+      const float4 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2), r3 = __ldg(r + 3);
+      const float4 ph = sm.phic[k];
+      const df rho = df_add(df_mul(df{ph.x, ph.y}, df{r0.z, r0.w}),
+                            df_mul(df{ph.z, ph.w}, df{r1.x, r1.y}));
+      float4 *d = sm.rec + k * (cs * 4u + 1u) + s * 4u;
+      d[0] = make_float4(r0.x, r0.y, r1.z, r1.w);
+      d[1] = make_float4(rho.hi, rho.lo, ph.x * r2.x + ph.z * r2.y, r2.z);
+      d[2] = make_float4(r2.w, ph.x * r2.y - ph.z * r2.x, ph.x * r3.x + ph.z * r3.y, r3.z);
+      d[3] = make_float4(ph.x * r3.y - ph.z * r3.x, 0.f, 0.f, 0.f);
+    }
+  }
+  __syncwarp();
+}
+
+// 1/d to FP32 rounding: the hardware estimate and one Newton step.
+__device__ __forceinline__ float rcp_newton(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float e = __fmaf_rn(-d, r, 1.0f);
+  // an overflowed or zero estimate (d subnormal, 0 or infinite) stands as it is
+  return fabsf(e) < 1.0f ? __fmaf_rn(r, e, r) : r;
+}
+
+// tau (near: tau - L) of step i of the chunk for the lane's direction, and
+// its amplitudes: far X = A_theta, Y = A_phi; near X_c, Y_c of component c
+// with A_c = Y_c + i omega X_c.
+template <bool NEAR>
+__device__ __forceinline__ df step_values(const FastUnit<NEAR> &u, const FastSmem &sm,
+                                          uint32_t rec0, uint32_t i, float (&X)[NEAR ? 3 : 1],
+                                          float (&Y)[NEAR ? 3 : 1]) {
+  if constexpr (!NEAR) {
+    const float4 *r = sm.rec + rec0 + i * 4u;
+    const float4 a = r[0], b = r[1], c = r[2];
+    const float aphi = r[3].x;
+    // tau = q + (1 - cos th) z - sin th rho  (double-float)
+    const df p1 = df_mul_raw(df{u.ld.dc_h, u.ld.dc_l}, df{a.z, a.w});
+    const df p2 = df_mul_raw(df{u.ld.st_h, u.ld.st_l}, df{b.x, b.y});
+    const df s1 = two_sum(a.x, p1.hi);
+    const df s2 = two_sum(s1.hi, -p2.hi);
+    const df tau = fast_two_sum(s2.hi, ((a.y + p1.lo) - p2.lo) + (s1.lo + s2.lo));
+    const float D = c.x + u.ld.f_dc * b.w - u.ld.f_st * b.z;
+    const float c2 = rcp_newton(D);
+    const float an = u.ld.f_st * c.z + u.ld.f_ct * c.w;
+    const float c1 = an * c2 * c2;
+    const float tb = u.ld.f_ct * b.z - u.ld.f_st * b.w;
+    const float ta = u.ld.f_ct * c.z - u.ld.f_st * c.w;
+    X[0] = -(c1 * tb + c2 * ta);
+    Y[0] = -(c1 * c.y + c2 * aphi);
+    return tau;
+  } else {
+    const float4 *r = sm.rec + i * 3u;
+    const float4 r0 = r[0], r1 = r[1], r2 = r[2];
+    // tau - L = (t - z) + rho^2 / (r + L - z)
+    const df ddx = df_sub(df{u.ld.X_h, u.ld.X_l}, df{r0.z, r0.w});
+    const df ddy = df_sub(df{u.ld.Y_h, u.ld.Y_l}, df{r1.x, r1.y});
+    const df D = df_sub(df{u.ld.L_h, u.ld.L_l}, df{r1.z, r1.w});
+    const df rho2 = df_add(df_mul(ddx, ddx), df_mul(ddy, ddy));
+    const df rr = df_sqrt(df_add(rho2, df_mul(D, D)));
+    const df F = (D.hi > 0.f) ? df_div(rho2, df_add(rr, D)) : df_sub(rr, D);
+    const float rinv = __frcp_rn(rr.hi + rr.lo);
+    const float nx = (ddx.hi + ddx.lo) * rinv, ny = (ddy.hi + ddy.lo) * rinv;
+    const float nz = (D.hi + D.lo) * rinv;
+    const float omn = (F.hi + F.lo) * rinv;  // 1 - n_z
+    X[0] = (r2.x - nx) * rinv;
+    X[1] = (r2.y - ny) * rinv;
+    X[2] = (omn - r2.w) * rinv;
+    const float q = rinv * rinv;
+    Y[0] = nx * q; Y[1] = ny * q; Y[2] = nz * q;
+    return df_add(df{r0.x, r0.y}, F);
+  }
+}
+
+// Per-lane sweep state along one track.
+template <bool NEAR>
+struct Sweep {
+  static constexpr int NP = NEAR ? 3 : 1;
+  float2 gx[NP][kTaps], gy[NP][kTaps];  // cells cur-3 .. cur+4
+  int cur;          // cell of the last included step (mod M)
+  bool live;        // the window holds something
+  float tp_h, tp_l; // tau of the previous step
+  int n_list;       // entries of the lane's list
+  bool dirty;       // the lane's direct sums hold something
+};
+
+template <bool NEAR>
+__device__ __forceinline__ void window_clear(Sweep<NEAR> &w) {
+#pragma unroll
+  for (int c = 0; c < Sweep<NEAR>::NP; ++c)
+#pragma unroll
+    for (int l = 0; l < kTaps; ++l) w.gx[c][l] = w.gy[c][l] = make_float2(0.f, 0.f);
+}
+
+// The whole window to the lane's circle.
+template <bool NEAR>
+__device__ __forceinline__ void window_flush(Sweep<NEAR> &w, float4 *cells, int M) {
+#pragma unroll
+  for (int c = 0; c < Sweep<NEAR>::NP; ++c)
+#pragma unroll
+    for (int l = 0; l < kTaps; ++l)
+      red_f4(cells + (size_t)c * 32 * M + ((w.cur - 3 + l) & (M - 1)), w.gx[c][l], w.gy[c][l]);
+  window_clear(w);
+}
+
+// The included frequencies [jf, jl] of a step whose rule cuts the band: the
+// certain interval (kPiLo), extended by the exact FP64 test through the
+// guard band (up to kPiHi), as jf | jl << 16.  Empty: jf > jl.
+template <bool NEAR>
+__device__ __forceinline__ uint32_t cut_interval(const FarMixedParams &p, uint32_t j0, int nb,
+                                              float w0f, float dwf, uint32_t dir, int64_t base, uint32_t s,
+                                              uint32_t it_start, float adt) {
+  const float inv_dw = 1.0f / dwf, inv_adt = __frcp_rn(adt);
+  const uint32_t iT = dir % p.n_theta, iP = dir / p.n_theta;
+  auto inside = [&](int j) -> bool {
+    const double w = p.omega[j0 + j];
+    if constexpr (NEAR)
+      return exact_mask_near(p, base, s, it_start, w, p.sin_theta[iT] * p.cos_phi[iP],
+                             p.sin_theta[iT] * p.sin_phi[iP]);
+    else
+      return exact_mask(p, base, s, it_start, w, p.sin_theta[iT] * p.cos_phi[iP],
+                        p.sin_theta[iT] * p.sin_phi[iP], p.cos_theta[iT]);
+  };
+  int uf, ul, jf, jl;
+  omega_interval(w0f, dwf, inv_dw, kPiLo * inv_adt, nb, jf, jl);
+  omega_interval(w0f, dwf, inv_dw, kPiHi * inv_adt, nb, uf, ul);
+  if (jf > jl) {  // no certain point: the first and last that pass the test
+    jf = 1;
+    jl = 0;
+    for (int j = uf; j <= ul; ++j)
+      if (inside(j)) {
+        if (jf > jl) jf = j;
+        jl = j;
+      }
+    return (uint32_t)jf | ((uint32_t)jl << 16);
+  }
+  while (jl + 1 <= ul && inside(jl + 1)) ++jl;
+  while (jf - 1 >= uf && inside(jf - 1)) --jf;
+  return (uint32_t)jf | ((uint32_t)jl << 16);
+}
+
+// Direct sums of the listed steps of every lane, by the whole warp: point
+// j = lane + 32 k, seeded by sin/cos and rotated by exp(32 i d_omega tau).
+// Two entries at a time share the packed FP32 operations (their chains are
+// independent; one at a time the sums waited for the rotations).  At most 8
+// blocks of 32 points per pass, so that the pair sums stay in registers.
+template <bool NEAR, int NK>
+__device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<NEAR> sl, uint32_t slot0,
+                                         uint32_t j0, int nb, int64_t base, uint32_t it_start,
+                                         int n_list, bool dirty, int lane) {
+  constexpr int NP = NEAR ? 3 : 1;
+  constexpr int KB = NK < 8 ? NK : 8;
+  __syncwarp();
+  const uint32_t has = __ballot_sync(0xffffffffu, n_list > 0);
+  const uint32_t old = __ballot_sync(0xffffffffu, dirty);
+  const double w0 = p.omega[0];
+  const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
+  const double inv2pi = 0.15915494309189533577;
+  const df f32 = df_from_double(32.0 * dw * inv2pi);
+  const float w0f = (float)(w0 + (double)j0 * dw), dwf = (float)dw;
+  float4 *lhead = sl.lhead(p.fast), *part = sl.part(p.fast);
+  const float2 *lamp = sl.lamp(p.fast);
+  // the included frequencies of each entry, in place of its |dtau|
+  for (uint32_t m = has; m; m &= m - 1) {
+    const int d = __ffs(m) - 1;
+    const int n = __shfl_sync(0xffffffffu, n_list, d);
+    for (int e = lane; e < n; e += 32) {
+      float4 *h = lhead + d * kFastList + e;
+      const float adt = __ldcg(&h->z);
+      const uint32_t s = __float_as_uint(__ldcg(&h->w));
+      const uint32_t r =
+          cut_interval<NEAR>(p, j0, nb, w0f, dwf, slot0 + d, base, s, it_start, adt);
+      h->z = __uint_as_float(r);
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int h0 = 0; h0 < NK; h0 += KB) {
+    if (32 * h0 >= nb) break;
+    const df fl = df_from_double((w0 + (double)(j0 + 32 * h0 + lane) * dw) * inv2pi);
+#pragma unroll 1
+    for (uint32_t m = has; m; m &= m - 1) {
+      const int d = __ffs(m) - 1;
+      const int n = __shfl_sync(0xffffffffu, n_list, d);
+#pragma unroll 1
+      for (int c = 0; c < NP; ++c) {
+        float2 xr[KB], xi[KB], yr[KB], yi[KB];  // .x: even entries, .y: odd entries
+#pragma unroll
+        for (int k = 0; k < KB; ++k) xr[k] = xi[k] = yr[k] = yi[k] = make_float2(0.f, 0.f);
+        for (int e0 = 0; e0 < n; e0 += 32) {
+          // a lane loads one entry and its rotation; the warp then takes the
+          // entries in order
+          const int ne = min(32, n - e0), el = e0 + min(lane, ne - 1);
+          const float4 h = __ldcg(lhead + d * kFastList + el);
+          float2 am = __ldcg(lamp + ((size_t)c * 32 + d) * kFastList + el);
+          if (lane >= ne) am = make_float2(0.f, 0.f);
+          float hs, hc;
+          phasor_rev(f32.hi, f32.lo, h.x, h.y, hs, hc);
+          for (int e = 0; e < ne; e += 2) {
+            auto two = [&](float v) {
+              return make_float2(__shfl_sync(0xffffffffu, v, e), __shfl_sync(0xffffffffu, v, e + 1));
+            };
+            const float2 th = two(h.x), tl = two(h.y), r = two(h.z);
+            const float2 vx = two(am.x), vy = two(am.y), rc = two(hc), rs = two(hs);
+            const float2 nrs = make_float2(-rs.x, -rs.y);
+            const uint32_t ra = __float_as_uint(r.x), rb = __float_as_uint(r.y);
+            const int fa = (int)(ra & 0xffffu) - 32 * h0, la = (int)(ra >> 16) - 32 * h0;
+            const int fb = (int)(rb & 0xffffu) - 32 * h0, lb = (int)(rb >> 16) - 32 * h0;
+            // an entry without frequencies (fa > la) adds nothing below: its
+            // block range is empty or masked
+            const int last = max(la, lb);
+            if (last < 0) continue;
+            // blocks below kw are included whole by both
+            const int kw = max(fa, fb) <= 0 ? (min(la, lb) + 1) >> 5 : 0;
+            float2 zc, zs;
+            phasor_rev(fl.hi, fl.lo, th.x, tl.x, zs.x, zc.x);
+            phasor_rev(fl.hi, fl.lo, th.y, tl.y, zs.y, zc.y);
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+              if (32 * k > last) break;
+              float2 px = vx, py = vy;
+              if (k >= kw) {
+                const int j = lane + 32 * k;
+                if (j < fa || j > la) px.x = py.x = 0.f;
+                if (j < fb || j > lb) px.y = py.y = 0.f;
+              }
+              xr[k] = __ffma2_rn(px, zc, xr[k]);
+              xi[k] = __ffma2_rn(px, zs, xi[k]);
+              yr[k] = __ffma2_rn(py, zc, yr[k]);
+              yi[k] = __ffma2_rn(py, zs, yi[k]);
+              rot2p(zc, zs, rc, rs, nrs, zc, zs);
+            }
+          }
+        }
+        // compensated: a track can empty its lists a thousand times
+        float4 *a = part + ((size_t)c * 32 + d) * 2 * p.fast.nb + 32 * h0;
+        float4 *al = a + p.fast.nb;
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+          const int j = lane + 32 * k;
+          if (j + 32 * h0 < nb) {
+            float4 v = make_float4(xr[k].x + xr[k].y, xi[k].x + xi[k].y, yr[k].x + yr[k].y,
+                                   yi[k].x + yi[k].y);
+            float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
+            if ((old >> d) & 1u) {
+              const float4 o = a[j];
+              l = al[j];
+              df t = two_sum(o.x, v.x);
+              v.x = t.hi; l.x += t.lo;
+              t = two_sum(o.y, v.y);
+              v.y = t.hi; l.y += t.lo;
+              t = two_sum(o.z, v.z);
+              v.z = t.hi; l.z += t.lo;
+              t = two_sum(o.w, v.w);
+              v.w = t.hi; l.w += t.lo;
+            }
+            a[j] = v;
+            al[j] = l;
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// Spread steps [a, b) of a track into the lane's circle (steps before `from`
+// only give the previous tau).
+template <bool NEAR, int NK>
+__device__ __forceinline__ void spread_steps(const FarMixedParams &p, const FastUnit<NEAR> &u,
+                                             const FastSlice<NEAR> &sl, FastSmem &sm,
+                                             Sweep<NEAR> &w, int64_t base, uint32_t it_start,
+                                             uint32_t a, uint32_t b, uint32_t from, int lane) {
+  constexpr int NP = NEAR ? 3 : 1;
+  const int M = (int)p.fast.M;
+  const float Mf = (float)M;
+  const uint32_t cs = p.fast.chunk;
+  float4 *cells = sl.grid() + (size_t)lane * M;
+  const uint32_t rec0 = NEAR ? 0u : (uint32_t)u.kphi * (cs * 4u + 1u);
+  for (uint32_t s0 = a, cnt = 0; s0 < b; s0 += cnt) {
+    // the step before `from` stands alone, so that chunks start at `from`
+    cnt = s0 < from ? 1u : min(cs, b - s0);
+    __syncwarp();
+    stage_records<NEAR>(p, base + s0, cnt, lane, sm);
+#pragma unroll 1
+    for (uint32_t i = 0; i < cnt; ++i) {
+      const uint32_t s = s0 + i;
+      float X[NP], Y[NP];
+      const df tau = step_values<NEAR>(u, sm, rec0, i, X, Y);
+      // the track's first step compares its whole phase with zero
+      // (synchrad/kernel_farfield.cl:49, kernel_nearfield.cl:48)
+      float dt0 = (tau.hi - w.tp_h) + (tau.lo - w.tp_l);
+      if (s == 0) {
+        dt0 = tau.hi + tau.lo;
+        if constexpr (NEAR) dt0 += u.ld.L_h + u.ld.L_l;
+      }
+      const float adt = fabsf(dt0);
+      w.tp_h = tau.hi;
+      w.tp_l = tau.lo;
+      const bool mine = u.active && s >= from;
+      if (mine && u.wmax * adt < kPiLo) {
+        // phase of the band's centre, whole turns dropped
+        float zs, zc;
+        phasor_exact(u.f_c.hi, u.f_c.lo, tau.hi, tau.lo, zs, zc);
+        // cell of the step: d_omega tau / 2 pi turns of M cells
+        const float pr = u.f_d.hi * tau.hi;
+        float e = __fmaf_rn(u.f_d.hi, tau.hi, -pr);
+        e = __fmaf_rn(u.f_d.hi, tau.lo, e);
+        e = __fmaf_rn(u.f_d.lo, tau.hi, e);
+        const float uh = (pr - rintf(pr)) * Mf, ul = e * Mf;
+        const float rm = rintf((uh - 0.5f) + ul);
+        const float f = ((uh - rm) - 0.5f) + ul;
+        const int m = (int)rm;
+        int adv = ((m - w.cur + M / 2) & (M - 1)) - M / 2;
+        float t[kTaps];
+        kb_taps(f, t);
+        const float2 z = make_float2(zc, zs);
+        // more than one cell on: all but the last plainly (each cell leaves once)
+        while (w.live && adv > 1 && adv < kTaps) {
+#pragma unroll
+          for (int c = 0; c < NP; ++c) {
+            red_f4(cells + (size_t)c * 32 * M + ((w.cur - 3) & (M - 1)), w.gx[c][0], w.gy[c][0]);
+#pragma unroll
+            for (int l = 0; l + 1 < kTaps; ++l) {
+              w.gx[c][l] = w.gx[c][l + 1];
+              w.gy[c][l] = w.gy[c][l + 1];
+            }
+            w.gx[c][kTaps - 1] = w.gy[c][kTaps - 1] = make_float2(0.f, 0.f);
+          }
+          ++w.cur;
+          --adv;
+        }
+        if (w.live && adv == 1) {
+#pragma unroll
+          for (int c = 0; c < NP; ++c) {
+            red_f4(cells + (size_t)c * 32 * M + ((w.cur - 3) & (M - 1)), w.gx[c][0], w.gy[c][0]);
+            const float2 vx = __fmul2_rn(make_float2(X[c], X[c]), z);
+            const float2 vy = __fmul2_rn(make_float2(Y[c], Y[c]), z);
+#pragma unroll
+            for (int l = 0; l + 1 < kTaps; ++l) {
+              w.gx[c][l] = __ffma2_rn(make_float2(t[l], t[l]), vx, w.gx[c][l + 1]);
+              w.gy[c][l] = __ffma2_rn(make_float2(t[l], t[l]), vy, w.gy[c][l + 1]);
+            }
+            w.gx[c][kTaps - 1] = __fmul2_rn(make_float2(t[kTaps - 1], t[kTaps - 1]), vx);
+            w.gy[c][kTaps - 1] = __fmul2_rn(make_float2(t[kTaps - 1], t[kTaps - 1]), vy);
+          }
+          w.cur = m;
+        } else {
+          if (!w.live) {
+            w.cur = m;
+            w.live = true;
+          } else if (adv != 0) {
+            if (adv == -1) {
+#pragma unroll
+              for (int c = 0; c < NP; ++c) {
+                red_f4(cells + (size_t)c * 32 * M + ((w.cur + 4) & (M - 1)), w.gx[c][kTaps - 1],
+                       w.gy[c][kTaps - 1]);
+#pragma unroll
+                for (int l = kTaps - 1; l > 0; --l) {
+                  w.gx[c][l] = w.gx[c][l - 1];
+                  w.gy[c][l] = w.gy[c][l - 1];
+                }
+                w.gx[c][0] = w.gy[c][0] = make_float2(0.f, 0.f);
+              }
+            } else {
+              window_flush(w, cells, M);
+            }
+            w.cur = m;
+          }
+#pragma unroll
+          for (int c = 0; c < NP; ++c) {
+            const float2 vx = __fmul2_rn(make_float2(X[c], X[c]), z);
+            const float2 vy = __fmul2_rn(make_float2(Y[c], Y[c]), z);
+#pragma unroll
+            for (int l = 0; l < kTaps; ++l) {
+              w.gx[c][l] = __ffma2_rn(make_float2(t[l], t[l]), vx, w.gx[c][l]);
+              w.gy[c][l] = __ffma2_rn(make_float2(t[l], t[l]), vy, w.gy[c][l]);
+            }
+          }
+        }
+      } else if (mine && !(u.wmin * adt > kPiHi)) {
+        const int k = w.n_list++;
+        sl.lhead(p.fast)[lane * kFastList + k] =
+            make_float4(tau.hi, tau.lo, adt, __uint_as_float(s));
+#pragma unroll
+        for (int c = 0; c < NP; ++c)
+          sl.lamp(p.fast)[((size_t)c * 32 + lane) * kFastList + k] = make_float2(X[c], Y[c]);
+      }
+    }
+    // cells that stay in the window for long would gather hundreds of terms:
+    // started afresh every 128 steps (fewer where a sweep would lap the circle), their FP32 sums round a fifth as much
+    const bool drain = __any_sync(0xffffffffu, w.n_list > kFastList - 32);
+    if (drain || ((s0 + cnt - from) & (p.fast.block - 1u)) == 0u) {
+      if (w.live) window_flush(w, cells, M);
+      if (drain) {
+        drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, lane);
+        w.dirty = w.dirty || w.n_list > 0;
+        w.n_list = 0;
+        window_clear(w);
+      }
+    }
+  }
+}
+
+// Steps [a, b) of a track into the warp's circles and direct sums, nothing
+// left in registers; returns whether the lane's direct sums hold something.
+// A function of its own: its loop keeps its registers whatever the transforms
+// need.
+template <bool NEAR, int NK>
+__device__ __forceinline__ bool spread_range(const FarMixedParams &p, const FastUnit<NEAR> &uref,
+                                          FastSlice<NEAR> sl, FastSmem &sm, int64_t base,
+                                          uint32_t it_start, uint32_t a, uint32_t b, bool dirty,
+                                          int lane) {
+  const FastUnit<NEAR> u = uref;
+  Sweep<NEAR> w;
+  window_clear(w);
+  w.cur = 0;
+  w.live = false;
+  w.dirty = dirty;
+  w.tp_h = w.tp_l = 0.f;
+  w.n_list = 0;
+  spread_steps<NEAR, NK>(p, u, sl, sm, w, base, it_start, a ? a - 1 : 0u, b, a, lane);
+  if (w.live) window_flush(w, sl.grid() + (size_t)lane * p.fast.M, (int)p.fast.M);
+  if (__any_sync(0xffffffffu, w.n_list > 0)) {
+    drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, lane);
+    w.dirty = w.dirty || w.n_list > 0;
+  }
+  __threadfence();
+  __syncwarp();
+  return w.dirty;
+}
+
+// The spectrum of one pair of fields, X and Y (band sums xs, ys, undivided),
+// added to the partial spectrum of track subset `sub`; A is also kept for
+// the adjoints where asked.
+template <bool NEAR>
+__device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUnit<NEAR> &u,
+                                          uint32_t dir, int d, int c, const float2 *xs,
+                                          const float2 *ys, const float4 *part, int n_seg,
+                                          const uint32_t *dirty, uint32_t t, uint32_t ksnap, uint32_t sub, int lane) {
+  const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
+  const double wp = p.weight[t];
+  const double wpdt2 = wp * p.dt * p.dt, wpdt = sqrt(wp) * p.dt;
+  double *out = p.partial + (uint64_t)sub * p.n_out * p.n_snaps * P;
+  const uint32_t iT = dir % p.n_theta, iP = dir / p.n_theta;
+  bool listed = p.save_A != nullptr;
+  for (int i = 0; i < n_seg; ++i) listed = listed || ((dirty[(size_t)i * p.fast.n_dwb] >> d) & 1u);
+  const uint64_t g0 = (uint64_t)u.j0 + (uint64_t)p.n_omega * dir;
+  if (!listed && p.comp == SR_COMP_TOTAL) {
+    // |A|^2 from the FP32 sums in double-float (exact products), scaled and
+    // added in FP64: a third of the FP64 operations of the general form below
+    double *o = out + (uint64_t)ksnap * P + g0;
+    for (int m = lane; m < u.nb; m += 32) {
+      const double dv = p.fast.deconv[m - u.nb / 2 + kFastMaxBand / 2];
+      const float2 x = xs[m], y = ys[m];
+      df q;
+      if constexpr (!NEAR) {
+        q = df_norm2(x, y);
+      } else {
+        const double w = p.omega[u.j0 + m];
+        const df wd = df_from_double(w);
+        const df a = df_mul_raw(wd, df{-x.y, 0.f}), b = df_mul_raw(wd, df{x.x, 0.f});
+        q = df_add(df_square(df_add(df{y.x, 0.f}, a)), df_square(df_add(df{y.y, 0.f}, b)));
+      }
+      red_f64(o + m, (wpdt2 * dv * dv) * ((double)q.hi + (double)q.lo));
+    }
+    return;
+  }
+  for (int m = lane; m < u.nb; m += 32) {
+    const double dv = p.fast.deconv[m - u.nb / 2 + kFastMaxBand / 2];
+    const float2 x = xs[m], y = ys[m];
+    double Ar = (double)x.x * dv, Ai = (double)x.y * dv;
+    double Br = (double)y.x * dv, Bi = (double)y.y * dv;
+    for (int i = 0; i < n_seg; ++i)
+      if ((dirty[(size_t)i * p.fast.n_dwb] >> d) & 1u) {  // direct sums of the listed steps
+        const float4 *q = part + (size_t)i * (p.fast.slice_bytes * p.fast.n_dwb / 16) + m;
+        const float4 v = q[0], l = q[p.fast.nb];
+        Ar += (double)v.x + (double)l.x;
+        Ai += (double)v.y + (double)l.y;
+        Br += (double)v.z + (double)l.z;
+        Bi += (double)v.w + (double)l.w;
+      }
+    const uint64_t gti = g0 + m;
+    auto add = [&](int o, double v) {
+      red_f64(out + ((uint64_t)o * p.n_snaps + ksnap) * P + gti, v);
+    };
+    if constexpr (!NEAR) {
+      if (p.save_A != nullptr)
+        reinterpret_cast<float4 *>(p.save_A)[((uint64_t)t * p.n_snaps + ksnap) * P + gti] =
+            make_float4((float)Ar, (float)Ai, (float)Br, (float)Bi);
+      if (p.comp == SR_COMP_TOTAL) {
+        add(0, wpdt2 * (Ar * Ar + Ai * Ai + Br * Br + Bi * Bi));
+      } else if (p.comp == SR_COMP_SPHERIC) {
+        add(1, wpdt2 * (Ar * Ar + Ai * Ai));
+        add(2, wpdt2 * (Br * Br + Bi * Bi));
+      } else if (p.comp == SR_COMP_SPHERIC_COMPLEX) {
+        add(2, wpdt * Ar);
+        add(3, wpdt * Ai);
+        add(4, wpdt * Br);
+        add(5, wpdt * Bi);
+      } else {
+        const double cT = p.cos_theta[iT], sT = p.sin_theta[iT];
+        const double cP = p.cos_phi[iP], sP = p.sin_phi[iP];
+        const double hx = cT * cP, hy = cT * sP;
+        const double xr = hx * Ar - sP * Br, xi = hx * Ai - sP * Bi;
+        const double yr = hy * Ar + cP * Br, yi = hy * Ai + cP * Bi;
+        const double zr = -sT * Ar, zi = -sT * Ai;
+        if (p.comp == SR_COMP_CARTESIAN) {
+          add(0, wpdt2 * (xr * xr + xi * xi));
+          add(1, wpdt2 * (yr * yr + yi * yi));
+          add(2, wpdt2 * (zr * zr + zi * zi));
+        } else {
+          const double f = wpdt * p.form_factor[u.j0 + m];
+          add(0, f * xr);
+          add(1, f * xi);
+          add(2, f * yr);
+          add(3, f * yi);
+          add(4, f * zr);
+          add(5, f * zi);
+        }
+      }
+    } else {
+      const double w = p.omega[u.j0 + m];
+      const double Er = Br - w * Ai, Ei = Bi + w * Ar;  // Y + i omega X
+      if (p.save_A != nullptr) {
+        float *sa = p.save_A + 8 * (((uint64_t)t * p.n_snaps + ksnap) * P + gti);
+        reinterpret_cast<float2 *>(sa)[c] = make_float2((float)Er, (float)Ei);
+        if (c == 2) reinterpret_cast<float2 *>(sa)[3] = make_float2(0.f, 0.f);
+      }
+      if (p.comp == SR_COMP_TOTAL) {
+        add(0, wpdt2 * (Er * Er + Ei * Ei));
+      } else if (p.comp == SR_COMP_CARTESIAN) {
+        add(c, wpdt2 * (Er * Er + Ei * Ei));
+      } else {  // cartesian_complex (FormFactor not applied)
+        double sL, cL;
+        sincos(w * p.L_screen, &sL, &cL);
+        add(2 * c, wpdt * (Er * cL - Ei * sL));
+        add(2 * c + 1, wpdt * (Er * sL + Ei * cL));
+      }
+    }
+  }
+}
+
+// Transforms and emits the pairs [pr0, pr1) (pair = local direction x NP + c)
+// of one track, summing the circles of n_seg slices (slice stride in bytes).
+template <bool NEAR, int R1>
+__device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const FastUnit<NEAR> &u,
+                                                const unsigned char *slice0, int n_seg,
+                                                const uint32_t *dirty, FastSmem &sm, int pr0,
+                                                int pr1, uint32_t t, uint32_t ksnap,
+                                                uint32_t sub, int lane) {
+  constexpr int NP = NEAR ? 3 : 1;
+  constexpr int NF = 32 / R1, M = 32 * R1;
+  const uint32_t n_dirs = p.n_theta * p.n_phi;
+  const size_t stride = p.fast.slice_bytes * p.fast.n_dwb;  // between a track's segments
+  const float4 *grid = (const float4 *)slice0;
+  const float4 *parts = grid + (size_t)NP * 32 * M;
+  auto emit = [&](int pr, const float2 *xs, const float2 *ys) {
+    const int d = pr / NP, c = pr % NP;
+    emit_pair<NEAR>(p, u, u.slot0 + d, d, c, xs, ys, parts + ((size_t)c * 32 + d) * 2 * p.fast.nb,
+                    n_seg, dirty, t, ksnap, sub, lane);
+  };
+  if constexpr (R1 == 32) {
+    for (int pr = pr0; pr < pr1; ++pr) {
+      const int d = pr / NP, c = pr % NP;
+      if (u.slot0 + d >= n_dirs) break;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {  // field X, then Y
+        float2 x[1][32];
+        const float2 *g = (const float2 *)(grid + ((size_t)c * 32 + d) * M) + h;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[0][i] = __ldcg(g + 2 * (32 * i + lane));
+        for (int sg = 1; sg < n_seg; ++sg) {
+          const float2 *gs = g + (size_t)sg * (stride / 8);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float2 v = __ldcg(gs + 2 * (32 * i + lane));
+            x[0][i].x += v.x;
+            x[0][i].y += v.y;
+          }
+        }
+        fft_band<32, 1>(x, sm.tr, p.fast.twiddle, lane, u.nb, h ? sm.tr : sm.out);
+      }
+      emit(pr, sm.out, sm.tr);
+      __syncwarp();
+    }
+  } else {
+    for (int q0 = pr0; q0 < pr1; q0 += NF / 2) {
+      if (u.slot0 + q0 / NP >= n_dirs) break;
+      float2 x[NF][R1];
+#pragma unroll
+      for (int k = 0; k < NF / 2; ++k) {
+        const int pr = min(q0 + k, pr1 - 1), d = pr / NP, c = pr % NP;
+        const float4 *g = grid + ((size_t)c * 32 + d) * M;
+#pragma unroll
+        for (int i = 0; i < R1; ++i) {
+          const float4 v = __ldcg(g + 32 * i + lane);
+          x[2 * k][i] = make_float2(v.x, v.y);
+          x[2 * k + 1][i] = make_float2(v.z, v.w);
+        }
+        for (int sg = 1; sg < n_seg; ++sg) {
+          const float4 *gs = g + (size_t)sg * (stride / 16);
+#pragma unroll
+          for (int i = 0; i < R1; ++i) {
+            const float4 v = __ldcg(gs + 32 * i + lane);
+            x[2 * k][i].x += v.x;
+            x[2 * k][i].y += v.y;
+            x[2 * k + 1][i].x += v.z;
+            x[2 * k + 1][i].y += v.w;
+          }
+        }
+      }
+      fft_band<R1, NF>(x, sm.tr, p.fast.twiddle, lane, u.nb, sm.out);
+#pragma unroll 1
+      for (int k = 0; k < NF / 2; ++k) {
+        const int pr = q0 + k;
+        if (pr >= pr1 || u.slot0 + pr / NP >= n_dirs) break;
+        emit(pr, sm.out + (2 * k) * u.nb, sm.out + (2 * k + 1) * u.nb);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// Tracks of subset `sub`: one each when there are as many subsets as tracks.
+__device__ __forceinline__ void fast_tracks_of(const FarMixedParams &p, uint32_t sub, uint32_t &t0,
+                                               uint32_t &t1) {
+  if (p.fast.n_sub == p.n_tracks) {
+    t0 = sub;
+    t1 = sub + 1;
+  } else {
+    subset_range(p, sub, p.fast.n_sub, t0, t1);
+  }
+}
+
+// Whole tracks: a warp takes (32 directions x band, track subset) items from
+// a queue, and for each track spreads its steps, transforms the 32 circles
+// and adds the spectra at every snapshot.
+template <bool NEAR, int R1>
+__global__ void __launch_bounds__(kFastWarps * 32, NEAR ? 2 : 3)
+fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
+  if (*p.fast.uneven) return;
+  constexpr int NP = NEAR ? 3 : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  FastSmem &sm = reinterpret_cast<FastSmem *>(smem_raw)[warp];
+  const FastParams &f = p.fast;
+  const uint32_t wid = blockIdx.x * kFastWarps + warp;
+  const FastSlice<NEAR> sl(f, wid);
+  const uint32_t n_items = f.n_dwb * f.n_sub;
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(f.queue, 1u);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= n_items) return;
+    const uint32_t sub = item / f.n_dwb;
+    FastUnit<NEAR> u;
+    __syncwarp();
+    unit_init<NEAR>(p, item % f.n_dwb, lane, sm, u);
+    uint32_t t0, t1;
+    fast_tracks_of(p, sub, t0, t1);
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t n_body = track_body(p, t);
+      const uint32_t it_start = p.it_start[t], it_end = p.it_end[t];
+      const uint32_t *snaps = p.snap_its + (size_t)t * p.snap_stride;
+      SnapState snap;
+      snap.init(it_start, it_end, snaps, p.n_snaps);
+      if (snap.fire_it == SnapState::NEVER) continue;  // nothing of the track is written
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint32_t i = lane; i < (uint32_t)(NP * 32 * 32 * R1); i += 32u) __stcg(sl.grid() + i, zero);
+      __threadfence();
+      __syncwarp();
+      bool dirty_l = false;
+      const int64_t base = p.offsets[t];
+      uint32_t s = 0;
+      // steps up to each snapshot's write; those due after the last body step
+      // repeat the same amplitudes; steps after the last write enter nothing
+      while (snap.fire_it != SnapState::NEVER) {
+        const uint32_t e = (uint32_t)min((int64_t)n_body, snap.fire_it + 1);
+        if (e > s) {
+          dirty_l = spread_range<NEAR, R1 / 2>(p, u, sl, sm, base, it_start, s, e, dirty_l, lane);
+          s = e;
+        }
+        const uint32_t dirty = __ballot_sync(0xffffffffu, dirty_l);
+        transform_pairs<NEAR, R1>(p, u, sl.base, 1, &dirty, sm, 0, 32 * NP,
+                                  t, snap.k, sub, lane);
+        snap.advance(it_start, it_end, snaps, p.n_snaps);
+      }
+    }
+  }
+}
+
+// Few tracks: first the steps, each unit into its own slice, so that every SM
+// has work.  A unit is a segment of f.seg_steps steps (one snapshot; track t's
+// segments start at first_segment(t), one number spare per track) or the
+// steps between two snapshots (f.seg_steps = 0) ...
+__device__ __forceinline__ uint32_t first_segment(const FarMixedParams &p, uint32_t t) {
+  return (uint32_t)((uint64_t)p.offsets[t] / p.fast.seg_steps) + t;
+}
+// The track's k-th snapshot write, and the first step that the one before it
+// does not enter; false if there is none.
+__device__ __forceinline__ bool nth_snapshot(const FarMixedParams &p, uint32_t t, uint32_t k,
+                                             SnapState &snap, uint64_t &from) {
+  const uint32_t *snaps = p.snap_its + (size_t)t * p.snap_stride;
+  snap.init(p.it_start[t], p.it_end[t], snaps, p.n_snaps);
+  from = 0;
+  for (uint32_t i = 0; i < k && snap.fire_it != SnapState::NEVER; ++i) {
+    from = (uint64_t)snap.fire_it + 1;
+    snap.advance(p.it_start[t], p.it_end[t], snaps, p.n_snaps);
+  }
+  return snap.fire_it != SnapState::NEVER;
+}
+
+template <bool NEAR, int R1>
+__global__ void __launch_bounds__(kFastWarps * 32, NEAR ? 2 : 3)
+fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
+  if (*p.fast.uneven) return;
+  constexpr int NP = NEAR ? 3 : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  FastSmem &sm = reinterpret_cast<FastSmem *>(smem_raw)[warp];
+  const FastParams &f = p.fast;
+  const uint32_t unit = blockIdx.x * kFastWarps + warp;
+  if (unit >= f.n_segs * f.n_dwb) return;
+  const uint32_t gs = unit / f.n_dwb, dwb = unit % f.n_dwb;
+  uint32_t t;
+  uint64_t a, b;
+  if (f.seg_steps == 0) {  // the steps between two snapshots
+    t = gs / p.n_snaps;
+    SnapState snap;
+    if (!nth_snapshot(p, t, gs % p.n_snaps, snap, a)) return;
+    b = (uint64_t)min((int64_t)track_body(p, t), snap.fire_it + 1);
+    a = min(a, b);
+  } else {
+    uint32_t lo = 0, hi = p.n_tracks;  // the segment's track
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (first_segment(p, mid) <= gs) lo = mid; else hi = mid;
+    }
+    t = lo;
+    a = (uint64_t)(gs - first_segment(p, t)) * f.seg_steps;
+    SnapState snap;
+    uint64_t from;
+    if (!nth_snapshot(p, t, 0, snap, from)) return;
+    const uint64_t n = (uint64_t)min((int64_t)track_body(p, t), snap.fire_it + 1);
+    if (a >= n && a > 0) return;  // no segment of the track
+    b = min(n, a + f.seg_steps);
+  }
+  const FastSlice<NEAR> sl(f, unit);
+  FastUnit<NEAR> u;
+  unit_init<NEAR>(p, dwb, lane, sm, u);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t i = lane; i < NP * 32u * f.M; i += 32u) __stcg(sl.grid() + i, zero);
+  __threadfence();
+  __syncwarp();
+  bool dirty_l = false;
+  if (b > a)
+    dirty_l = spread_range<NEAR, R1 / 2>(p, u, sl, sm, p.offsets[t], p.it_start[t], (uint32_t)a,
+                                         (uint32_t)b, false, lane);
+  const uint32_t dirty = __ballot_sync(0xffffffffu, dirty_l);
+  if (lane == 0) f.dirty[unit] = dirty;
+}
+
+// ... then, a few directions per warp and its track subset, the transforms of
+// the summed circles.
+template <bool NEAR, int R1>
+__global__ void __launch_bounds__(kFastWarps * 32, 4)
+fast_transform_kernel(const __grid_constant__ FarMixedParams p) {
+  if (*p.fast.uneven) return;
+  constexpr int NP = NEAR ? 3 : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  FastSmem &sm = reinterpret_cast<FastSmem *>(smem_raw)[warp];
+  const FastParams &f = p.fast;
+  uint32_t item = blockIdx.x * kFastWarps + warp;
+  const uint32_t per = f.dirs_per_warp, n_g = 32u / per;
+  if (item >= f.n_dwb * n_g * f.n_sub * p.n_snaps) return;
+  const uint32_t g = item % n_g;
+  item /= n_g;
+  const uint32_t dwb = item % f.n_dwb;
+  item /= f.n_dwb;
+  const uint32_t k = item % p.n_snaps, sub = item / p.n_snaps;
+  FastUnit<NEAR> u;
+  unit_init<NEAR>(p, dwb, lane, sm, u);
+  uint32_t t0, t1;
+  fast_tracks_of(p, sub, t0, t1);
+  for (uint32_t t = t0; t < t1; ++t) {
+    SnapState snap;
+    uint64_t from;
+    if (!nth_snapshot(p, t, k, snap, from)) continue;
+    size_t unit0;
+    int n_seg;
+    if (f.seg_steps == 0) {
+      unit0 = (size_t)t * p.n_snaps;
+      n_seg = (int)k + 1;
+    } else {
+      const uint64_t n = (uint64_t)min((int64_t)track_body(p, t), snap.fire_it + 1);
+      unit0 = first_segment(p, t);
+      n_seg = n ? (int)((n + f.seg_steps - 1) / f.seg_steps) : 1;
+    }
+    unit0 = unit0 * f.n_dwb + dwb;
+    transform_pairs<NEAR, R1>(p, u, f.scratch + unit0 * f.slice_bytes, n_seg, f.dirty + unit0, sm,
+                              (int)(g * per) * NP, (int)((g + 1) * per) * NP, t, snap.k, sub, lane);
+  }
+}
+
+// ------------------------------------------------------------------ host side
+template <bool NEAR, int R1>
+int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
+  constexpr int smem = (int)sizeof(FastSmem) * kFastWarps;
+  const unsigned threads = kFastWarps * 32;
+  cudaError_t e;
+  if (!l.split) {
+    e = allow_smem((const void *)fast_tracks_kernel<NEAR, R1>, smem);
+    if (e != cudaSuccess) return cuda_fail(e, "fast sum smem attribute");
+    fast_tracks_kernel<NEAR, R1><<<l.slices / kFastWarps, threads, smem, s>>>(p);
+    return cuda_fail(cudaGetLastError(), "fast sum launch");
+  }
+  e = allow_smem((const void *)fast_spread_kernel<NEAR, R1>, smem);
+  if (e == cudaSuccess) e = allow_smem((const void *)fast_transform_kernel<NEAR, R1>, smem);
+  if (e != cudaSuccess) return cuda_fail(e, "fast sum smem attribute");
+  fast_spread_kernel<NEAR, R1><<<l.slices / kFastWarps, threads, smem, s>>>(p);
+  const uint32_t items = l.n_dwb * (32u / l.dirs_per_warp) * l.n_sub * p.n_snaps;
+  fast_transform_kernel<NEAR, R1><<<(items + kFastWarps - 1) / kFastWarps, threads, smem, s>>>(p);
+  return cuda_fail(cudaGetLastError(), "fast sum launch");
+}
+
+template <bool NEAR>
+int launch_fast(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
+  switch (l.M) {
+    case 128: return launch_fast_r<NEAR, 4>(p, l, s);
+    case 256: return launch_fast_r<NEAR, 8>(p, l, s);
+    case 512: return launch_fast_r<NEAR, 16>(p, l, s);
+    default: return launch_fast_r<NEAR, 32>(p, l, s);
+  }
+}
+
+}  // namespace
+}  // namespace sr

@@ -34,6 +34,28 @@ void timing_record(cudaStream_t s, bool start, void **token);
 int launch_port(const PortParams &p, int mode, int comp, int dtype, bool native,
                 cudaStream_t stream);
 
+// Arguments of the summation by transforms (sr_fast_sum.cuh), for evenly
+// spaced omega axes.
+struct FastParams {
+  unsigned int *uneven;  // set by the record pass when the axis is not evenly spaced
+  unsigned int *queue;   // next work item (zeroed per launch)
+  double *deconv;        // 1 / transform of the spreading kernel, per frequency index
+  float4 *twiddle;       // [M/32][32] exp(2 pi i a l / M): cos, sin, and their low parts
+  unsigned int *dirty;   // per slice: directions whose direct sums hold something
+  unsigned char *scratch;
+  unsigned long long slice_bytes;
+  uint32_t n_bands, nb;  // omega bands and the frequencies of one
+  uint32_t M;            // cells of a circle
+  uint32_t n_dwb;        // (32 directions) x bands
+  uint32_t n_sub;        // track subsets
+  uint32_t n_segs;       // few tracks: segments of seg_steps steps, of all tracks
+  uint32_t seg_steps;
+  uint32_t block;        // steps after which the window is written out (a power of two)
+  uint32_t n_phik;       // phi nodes a warp's 32 directions span at most (far field)
+  uint32_t chunk;        // steps staged at a time
+  uint32_t dirs_per_warp;  // of the separate transform kernel
+};
+
 // Arguments of the mixed-precision far-field path.
 struct FarMixedParams {
   // tracks
@@ -73,6 +95,7 @@ struct FarMixedParams {
   unsigned int *queue;   // work items handed out after each CTA's first (zeroed per launch)
   // outputs
   double *out[6];
+  FastParams fast;       // fast.uneven == nullptr: term by term only
 };
 
 struct FarMixedConfig {
@@ -84,7 +107,28 @@ struct FarMixedConfig {
   int ctas_per_sm;
   int grid;     // CTAs of the persistent launch
   int stage;    // step records per TMA stage (far field; multiple of 32, <= 512)
+  bool direct;  // term by term on every axis (a pinned or tuned shape, no scratch to spare)
+  uint32_t n_omega, n_dirs, n_tracks;  // the problem the shape was made for
+  int n_sm;
 };
+
+// Work split of the summation by transforms.
+struct FastLayout {
+  bool on;     // worth it for these sizes
+  bool split;  // steps and transforms in two kernels (few tracks, one snapshot)
+  uint32_t n_bands, nb, M, n_dwb, n_sub, n_segs, seg_steps, block, slices, dirs_per_warp;
+  size_t slice_bytes;
+};
+FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
+                       uint32_t n_snaps);
+// Bytes of the tables and scratch behind the other parts of a workspace.
+size_t fast_workspace(const FastLayout &l);
+// Sets p.fast from the layout (workspace part at `base`, counters in the
+// status block at `status`).
+void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
+               unsigned char *status);
+int launch_fast_far(const FarMixedParams &p, const FastLayout &l, cudaStream_t s);
+int launch_fast_near(const FarMixedParams &p, const FastLayout &l, cudaStream_t s);
 
 FarMixedConfig far_mixed_make(uint32_t n_omega, uint32_t n_dirs, uint32_t n_tracks, int n_sm,
                               int K, int L, int stage, int n_sub);
@@ -126,6 +170,9 @@ int validate_spectrum_args(const sr_tracks *t, const sr_grid *g, int comp,
 FarMixedParams make_far_mixed_params(const sr_tracks *t, const sr_grid *g,
                                      int comp, void *const *out);
 int device_sm_count();
+// Lets a kernel use `bytes` of dynamic shared memory on the current device
+// (set once per kernel and device, not at every launch).
+cudaError_t allow_smem(const void *kernel, int bytes);
 
 // sr_noalloc.cu: the status word of the allocation-free entry point's static
 // scratch array on the current device.

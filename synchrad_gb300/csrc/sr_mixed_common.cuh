@@ -30,14 +30,17 @@ __device__ __forceinline__ uint32_t lower_bound_i64(const int64_t *a, uint32_t n
 
 // Track range [t0, t1) of subset `sub`: tracks whose first step lies in
 // [sub*total/n_sub, (sub+1)*total/n_sub), so subsets carry equal step counts.
+__device__ __forceinline__ void subset_range(const FarMixedParams &p, uint32_t sub,
+                                             uint32_t n_sub, uint32_t &t0, uint32_t &t1) {
+  const int64_t tot = p.total_steps;
+  t0 = (sub == 0) ? 0u : lower_bound_i64(p.offsets, p.n_tracks, (tot * (int64_t)sub) / n_sub);
+  t1 = (sub + 1 == n_sub)
+           ? p.n_tracks
+           : lower_bound_i64(p.offsets, p.n_tracks, (tot * (int64_t)(sub + 1)) / n_sub);
+}
 __device__ __forceinline__ void subset_tracks(const FarMixedParams &p, uint32_t sub,
                                               uint32_t &t0, uint32_t &t1) {
-  const int64_t tot = p.total_steps;
-  t0 = (sub == 0) ? 0u
-                  : lower_bound_i64(p.offsets, p.n_tracks, (tot * (int64_t)sub) / p.n_sub);
-  t1 = (sub + 1 == p.n_sub)
-           ? p.n_tracks
-           : lower_bound_i64(p.offsets, p.n_tracks, (tot * (int64_t)(sub + 1)) / p.n_sub);
+  subset_range(p, sub, p.n_sub, t0, t1);
 }
 
 __device__ __forceinline__ uint32_t track_body(const FarMixedParams &p, uint32_t t) {
@@ -183,17 +186,62 @@ __device__ __forceinline__ void cmul(float ar, float ai, float br, float bi, flo
   ci = ar * bi + ai * br;
 }
 
+// Whether this launch's axis is summed by transforms (sr_fast_sum.cuh): the
+// kernels that sum term by term leave at once then, and the other way round.
+__device__ __forceinline__ bool by_transform(const FarMixedParams &p) {
+  return p.fast.uneven != nullptr && *p.fast.uneven == 0u;
+}
+
+// Tables of the summation by transforms, made beside the step records: the
+// test of the omega axis (omega_j = omega_0 + j d_omega to 1e-12), the
+// reciprocal transform of the Kaiser-Bessel spreading kernel,
+// phi^(xi) = 8 sinh(s) / (s I0(beta)), s = sqrt(beta^2 - (8 pi xi)^2) at
+// xi = i / M, and the twiddle factors.
+constexpr int kFastMaxBand = 512;             // frequencies per band (M = 1024 cells)
+constexpr double kKbBeta = 18.638939747698778;  // pi sqrt((8/2)^2 (2 - 1/2)^2 - 0.8)
+constexpr double kKbI0 = 11574003.318462234;        // I0(kKbBeta)
+__device__ __forceinline__ void fast_tables(const FarMixedParams &p) {
+  const FastParams &f = p.fast;
+  if (f.uneven == nullptr) return;
+  const uint32_t nt = gridDim.x * blockDim.x, gt = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t n = p.n_omega;
+  const double w0 = p.omega[0], dw = (p.omega[n - 1] - w0) / (double)(n - 1);
+  bool bad = !(fabs(dw) > 0.0) || !isfinite(dw);
+  for (uint32_t j = gt; j < n; j += nt) {
+    const double wj = p.omega[j];
+    if (!(fabs(wj - (w0 + (double)j * dw)) <= 1e-12 * fabs(wj) + 1e-300)) bad = true;
+  }
+  if (bad) atomicOr(f.uneven, 1u);
+  if (threadIdx.x < 32u)  // one warp of each block: FP64 functions spread over the SMs
+    for (uint32_t i = blockIdx.x * 32u + threadIdx.x; i < f.M; i += gridDim.x * 32u) {
+      double sn, cn;  // f.M = 32 (M / 32) twiddles
+      sincospi(2.0 * (double)((i / 32u) * (i % 32u)) / (double)f.M, &sn, &cn);
+      const df c = df_from_double(cn), s = df_from_double(sn);
+      f.twiddle[i] = make_float4(c.hi, s.hi, c.lo, s.lo);
+    }
+  else if (threadIdx.x < 64u)
+    for (uint32_t i = blockIdx.x * 32u + threadIdx.x - 32u; i <= f.nb / 2u;
+         i += gridDim.x * 32u) {
+      const double x = 8.0 * M_PI * (double)i / (double)f.M;
+      const double s = sqrt(kKbBeta * kKbBeta - x * x);
+      const double v = s * kKbI0 / (8.0 * sinh(s));
+      f.deconv[kFastMaxBand / 2 - i] = v;
+      if (i < kFastMaxBand / 2) f.deconv[kFastMaxBand / 2 + i] = v;
+    }
+}
+
 // out[c][k*P + g] += sum over subsets (fixed order) of partial[sub][c][k][g]
 __global__ void mixed_reduce_kernel(FarMixedParams p) {
   const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
   const uint64_t per = (uint64_t)p.n_snaps * P;
   const uint64_t total = per * p.n_out;
+  const uint32_t n_sub = by_transform(p) ? p.fast.n_sub : p.n_sub;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t c = (uint32_t)(i / per);
     const uint64_t r = i - (uint64_t)c * per;
     double acc = 0.0;
-    for (uint32_t s = 0; s < p.n_sub; ++s) acc += p.partial[((uint64_t)s * p.n_out + c) * per + r];
+    for (uint32_t s = 0; s < n_sub; ++s) acc += p.partial[((uint64_t)s * p.n_out + c) * per + r];
     p.out[c][r] += acc;
   }
 }

@@ -42,6 +42,7 @@ constexpr int kNSetupF4 = 8;    // float4 per (screen point, step) in the setup
 //   r3 = r4 = 0 (padding: an 80-byte record stride spreads per-lane reads over the banks)
 template <typename TT>
 __global__ void near_prepass_kernel(FarMixedParams p) {
+  fast_tables(p);
   const TT *X = (const TT *)p.x, *Y = (const TT *)p.y, *Z = (const TT *)p.z;
   const TT *UX = (const TT *)p.ux, *UY = (const TT *)p.uy, *UZ = (const TT *)p.uz;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < p.total_steps;
@@ -120,6 +121,7 @@ __device__ __forceinline__ void near_accumulate(NearAcc<K> &a, int q, float2 zr,
 
 template <int K, int W>
 __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p) {
+  if (by_transform(p)) return;
   static_assert(K == 8 || K == 16, "K");
   constexpr int KP = K / 2, HP = KP / 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -576,8 +578,7 @@ int launch_near_main(const FarMixedParams &p, int grid, cudaStream_t s) {
   if (smem > kMaxSmemPerCta)
     return fail(SR_ERR_INVALID, "work shape needs %zu bytes of shared memory per CTA (at most %zu)",
                 smem, kMaxSmemPerCta);
-  cudaError_t e = cudaFuncSetAttribute(near_mixed_kernel<K, kNW>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem((const void *)near_mixed_kernel<K, kNW>, (int)kMaxSmemPerCta);
   if (e != cudaSuccess) return cuda_fail(e, "near_mixed smem attribute");
   near_mixed_kernel<K, kNW><<<grid, kNW * 32, smem, s>>>(p);
   return cuda_fail(cudaGetLastError(), "near_mixed kernel launch");
@@ -593,6 +594,11 @@ FarMixedConfig near_mixed_make(uint32_t n_omega, uint32_t n_screen, uint32_t n_t
   FarMixedConfig c;
   c.W = kNW;
   c.ctas_per_sm = 1;
+  c.direct = false;
+  c.n_omega = n_omega;
+  c.n_dirs = n_screen;
+  c.n_tracks = n_tracks;
+  c.n_sm = n_sm;
   c.K = K;
   c.stage = kStage;
   c.L = L;
@@ -636,9 +642,11 @@ size_t near_mixed_workspace(int64_t total_steps, uint64_t n_points, int n_out, u
                             const FarMixedConfig &cfg) {
   size_t b = 256;
   b += ((size_t)total_steps * kRecBytes + 255) / 256 * 256;
-  b += ((size_t)cfg.n_sub * n_out * n_snaps * n_points * 8 + 255) / 256 * 256;
+  const FastLayout l = fast_layout(cfg, true, total_steps, n_out, n_snaps);
+  b += ((size_t)std::max((uint32_t)cfg.n_sub, l.n_sub) * n_out * n_snaps * n_points * 8 + 255) /
+       256 * 256;
   b += (size_t)cfg.grid * cfg.W * cfg.K * kNOuter * 32 * sizeof(float);
-  return b;
+  return (b + 255) / 256 * 256 + fast_workspace(l);
 }
 
 int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size_t ws_bytes,
@@ -653,11 +661,16 @@ int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, siz
   size_t off = 256;
   p.status = (int *)w;
   p.queue = (unsigned int *)(w + 128);  // in the zeroed 256-byte status block
+  const FastLayout fl = fast_layout(cfg, true, p.total_steps, p.n_out, p.n_snaps);
+  p.partial = (double *)(w + off);
+  const size_t partial_bytes =
+      (size_t)std::max((uint32_t)cfg.n_sub, fl.n_sub) * p.n_out * p.n_snaps * P * 8;
+  off += (partial_bytes + 255) / 256 * 256;
   p.records = (float4 *)(w + off);
   off += ((size_t)p.total_steps * kRecBytes + 255) / 256 * 256;
-  p.partial = (double *)(w + off);
-  off += ((size_t)cfg.n_sub * p.n_out * p.n_snaps * P * 8 + 255) / 256 * 256;
   p.outer = (float *)(w + off);
+  off += ((size_t)cfg.grid * cfg.W * cfg.K * kNOuter * 32 * sizeof(float) + 255) / 256 * 256;
+  fast_bind(p, fl, true, w + off, w);
   p.dpw = (uint32_t)cfg.dpw;
   p.n_wtiles = (p.n_omega + (uint32_t)(cfg.L * cfg.K) - 1) / (uint32_t)(cfg.L * cfg.K);
   const uint32_t n_dirs = p.n_theta * p.n_phi;
@@ -666,10 +679,10 @@ int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, siz
   p.n_sub = (uint32_t)cfg.n_sub;
   p.n_items = p.n_groups * p.n_sub;
 
-  cudaError_t e = cudaMemsetAsync(w, 0, 256, stream);
-  if (e != cudaSuccess) return cuda_fail(e, "status reset");
-  e = cudaMemsetAsync(p.partial, 0, (size_t)p.n_sub * p.n_out * p.n_snaps * P * 8, stream);
-  if (e != cudaSuccess) return cuda_fail(e, "partial reset");
+  // status block and partial spectra, one after the other
+  cudaError_t e = cudaMemsetAsync(w, 0, 256 + partial_bytes, stream);
+  if (e != cudaSuccess) return cuda_fail(e, "status and partial reset");
+
   int dev = 0, n_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -677,6 +690,7 @@ int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, siz
     const int blk = 256;
     int64_t nb = (p.total_steps + blk - 1) / blk;
     if (nb > 8 * n_sm * 16) nb = 8 * n_sm * 16;
+    if (nb < 16) nb = 16;  // the tables' FP64 functions spread over the SMs
     if (p.track_f32)
       near_prepass_kernel<float><<<(int)nb, blk, 0, stream>>>(p);
     else
@@ -688,8 +702,10 @@ int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, siz
     return fail(SR_ERR_INVALID, "near field: points per lane %d (8 or 16)", cfg.K);
   void *tok = nullptr;
   timing_record(stream, true, &tok);
-  int rc = (cfg.K == 16) ? launch_near_main<16>(p, cfg.grid, stream)
-                         : launch_near_main<8>(p, cfg.grid, stream);
+  int rc = fl.on ? launch_fast_near(p, fl, stream) : SR_OK;
+  if (rc == SR_OK)
+    rc = (cfg.K == 16) ? launch_near_main<16>(p, cfg.grid, stream)
+                       : launch_near_main<8>(p, cfg.grid, stream);
   timing_record(stream, false, &tok);
   if (rc) return rc;
   const uint64_t total = (uint64_t)p.n_out * p.n_snaps * P;

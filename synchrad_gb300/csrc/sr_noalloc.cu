@@ -103,6 +103,7 @@ extern "C" int sr_spectrum_noalloc(const sr_tracks *t, const sr_grid *g, int com
   FarMixedConfig cfg =
       far_mixed_choose(g->n_omega, g->n_theta * g->n_phi, t->n_tracks, device_sm_count());
   cfg.n_sub = 1;
+  cfg.direct = true;  // the static array has no room for the transforms' circles
   const uint32_t n_wtiles = (g->n_omega + (uint32_t)(cfg.L * cfg.K) - 1) / (uint32_t)(cfg.L * cfg.K);
   const uint64_t dgroups = ((uint64_t)g->n_theta * g->n_phi + cfg.dpw - 1) / cfg.dpw;
   const uint64_t groups = (dgroups * n_wtiles + cfg.W - 1) / cfg.W;

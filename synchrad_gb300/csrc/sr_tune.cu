@@ -161,11 +161,12 @@ extern "C" int sr_config_set(const sr_tracks *t, const sr_grid *g, int comp, int
   if (c->track_subsets < 0 || c->track_subsets > 64)
     return fail(SR_ERR_INVALID, "track subsets %d (0: default, at most 64)", c->track_subsets);
   const uint32_t n_dirs = g->n_theta * g->n_phi;
-  const FarMixedConfig cfg =
+  FarMixedConfig cfg =
       far ? far_mixed_make(g->n_omega, n_dirs, t->n_tracks, device_sm_count(), K, L, st,
                            c->track_subsets)
           : near_mixed_make(g->n_omega, n_dirs, t->n_tracks, device_sm_count(), K, L,
                             c->track_subsets);
+  cfg.direct = true;  // a shape is that of the term-by-term kernels
   std::lock_guard<std::mutex> lk(g_tmu);
   g_cache[key_of(t, g, comp)] = cfg;
   return SR_OK;
