@@ -155,7 +155,7 @@ struct SmemFixed {
 // rotation chains of K/2), L lanes per direction, 32/L directions per warp.
 template <int K, int W>
 __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) {
-  if (by_transform(p)) return;
+  if (*p.fast.uneven != 0u) return;  // uneven_axis_kernel's
   static_assert(K % 4 == 0 && K >= 4 && K <= 32, "K");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SmemFixed<W> &sm = *reinterpret_cast<SmemFixed<W> *>(smem_raw);
@@ -189,15 +189,9 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
   const double inv2pi = 0.15915494309189533577;
   float *outer = p.outer + ((size_t)blockIdx.x * W + warp) * K * 8 * 32;
   uint32_t stage_no = 0;  // running stage counter (mbarrier phase bookkeeping)
-  // A uniform omega axis (omega_j = omega_0 + j d_omega to 1e-12): the points of
-  // a (direction, step) that pass the mask form one index interval, found once
+  // The axis is even (uneven_axis_kernel takes the others): the points of a
+  // (direction, step) that pass the mask form one index interval, found once
   // per (direction, step) in the setup and shared by the lanes.
-  bool axis_ok = nO < 65535u;
-  for (uint32_t j = threadIdx.x; j < nO && axis_ok; j += blockDim.x) {
-    const double wj = p.omega[j];
-    if (fabs(wj - (p.omega[0] + (double)j * dw_glob)) > 1e-12 * fabs(wj) + 1e-300) axis_ok = false;
-  }
-  const bool iv = __syncthreads_and(axis_ok) != 0;
   const float w0g = nO > 0 ? (float)p.omega[0] : 0.f;
   const float dwg = (float)dw_glob, inv_dwg = (dwg != 0.f) ? 1.0f / dwg : 0.f;
 
@@ -241,22 +235,11 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
       d.phx = (float)(-d.sPh); d.phy = (float)d.cPh;
     }
 
-    // Lane omega constants (revolutions) and uniformity of its chunk.
+    // Lane omega constants (revolutions).
     const double w0d = nv > 0 ? p.omega[j0] : 0.0;
     const df d_w0 = df_from_double(w0d * inv2pi);
-    const float w0f = (float)w0d, dwf = (float)dw_glob;
-    const float inv_dwf = (dwf != 0.f) ? 1.0f / dwf : 0.f;
-    bool uniform = true;
-    float wabs_min = 3.0e38f, wabs_max = 0.f;
-    for (int m = 0; m < nv; ++m) {
-      const double wm = p.omega[j0 + m];
-      const double pred = w0d + (double)m * dw_glob;
-      if (fabs(wm - pred) > 1e-12 * fabs(wm) + 1e-300) uniform = false;
-      const float a = (float)fabs(wm);
-      wabs_min = fminf(wabs_min, a);
-      wabs_max = fmaxf(wabs_max, a);
-    }
-    if (nv == 0) { wabs_min = 0.f; wabs_max = 0.f; }
+    float wabs_max = 0.f;
+    for (int m = 0; m < nv; ++m) wabs_max = fmaxf(wabs_max, (float)fabs(p.omega[j0 + m]));
     __syncwarp();
 
     uint32_t t0, t1;
@@ -414,7 +397,7 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
         if (active_w) {
           for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
             const uint32_t mcnt = min(32u, cnt - c0);
-            // Classes of the chunk's steps on a uniform axis, one bit per step:
+            // Classes of the chunk's steps, one bit per step:
             // every point of the warp's omega tile included (for all of its
             // directions), or none possibly included.
             uint32_t fast_bits = 0u, out_bits = 0u;
@@ -486,7 +469,7 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
                 // the mask's index intervals over the whole omega axis: points
                 // certainly included (below kPiLo) and possibly included (kPiHi)
                 int jfc = 1, jlc = 0, jfu = 1, jlu = 0;
-                if (iv) {
+                {
                   const float inv_adt = __frcp_rn(fabsf(dtau));
                   omega_interval(w0g, dwg, inv_dwg, kPiLo * inv_adt, (int)nO, jfc, jlc);
                   omega_interval(w0g, dwg, inv_dwg, kPiHi * inv_adt, (int)nO, jfu, jlu);
@@ -505,13 +488,13 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
                 __syncwarp();
                 if (lane == 0) { d.tprev_h = th_last; d.tprev_l = tl_last; d.adt_max = amax; }
               }
-              fast_bits = __ballot_sync(0xffffffffu, iv && (uint32_t)lane < mcnt && in_all);
-              out_bits = __ballot_sync(0xffffffffu, iv && (uint32_t)lane < mcnt && out_all && !in_all);
+              fast_bits = __ballot_sync(0xffffffffu, (uint32_t)lane < mcnt && in_all);
+              out_bits = __ballot_sync(0xffffffffu, (uint32_t)lane < mcnt && out_all && !in_all);
             }
             __syncwarp();
             // ---- the points: K per lane as two packed rotation chains ----
             // A chunk whose steps are all included for this lane's omega range,
-            // with a uniform axis and no snapshot write, runs the tight loop.
+            // and without a snapshot write, runs the tight loop.
             const bool fire_here = snap.fire_it >= (int64_t)(s0 + c0) &&
                                    snap.fire_it < (int64_t)(s0 + c0 + mcnt);
             // The first pair's phasors of one step: the reseed e^{i omega_0 tau}
@@ -524,7 +507,7 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
               ZrA = make_float2(zc, zc * A.z - zs * A.w);
               ZiA = make_float2(zs, zc * A.w + zs * A.z);
             };
-            // One fully included step on a uniform axis: two packed chains.
+            // One fully included step: two packed chains.
             auto step_fast = [&](const float4 *st, float2 ZrA, float2 ZiA) {
               const float4 AT = st[1 * 32], R2 = st[2 * 32], X = st[3 * 32], Y = st[4 * 32];
               const float2 at = make_float2(AT.x, AT.y), ap = make_float2(AT.z, AT.w);
@@ -550,7 +533,7 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
               }
             };
             // warp-uniform choices (lanes of a warp never diverge between paths)
-            if (__all_sync(0xffffffffu, uniform && !fire_here &&
+            if (__all_sync(0xffffffffu, !fire_here &&
                            wabs_max * sm.dc[warp][dsub].adt_max < kPiLo)) {
               // every step of the chunk included for every point: the tight loop
               const float4 *st = setup + (size_t)dsub * kSetupStride;
@@ -559,8 +542,8 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
                 step_seed(st + i, i, zr, zi);
                 step_fast(st + i, zr, zi);
               }
-            } else if (iv && __all_sync(0xffffffffu, uniform)) {
-              // Uniform axis: each step's class comes from the setup's ballots
+            } else {
+              // Each step's class comes from the setup's ballots
               // (no per-step vote). Runs of included steps go through the
               // straight-line loop; a step that is neither fully included nor
               // fully excluded for the warp takes the masked step (its points'
@@ -636,116 +619,6 @@ __global__ void __launch_bounds__(W * 32, 1) far_mixed_kernel(FarMixedParams p) 
                   snap.advance(it_start, it_end, snaps, p.n_snaps);
                 }
                 ++i;
-              }
-            } else {
-              // General loop (an omega axis that is not uniform as a whole):
-              // per-step vote, per-lane index interval on uniform lanes and a
-              // per-point test with one reseed per point on the others.
-#pragma unroll 1
-              for (uint32_t i = 0; i < mcnt; ++i) {
-                const float4 *st = setup + (size_t)dsub * kSetupStride + i;
-                const float adt = st[5 * 32].x;
-                const uint32_t s = s0 + c0 + i;
-                // a lane is all in (out) when its largest (smallest) |omega|
-                // passes (fails) the rule with the guard band
-                const bool all_in = wabs_max * adt < kPiLo;
-                const bool all_out = wabs_min * adt > kPiHi;
-                if (__all_sync(0xffffffffu, uniform && (all_in || nv == 0))) {
-                  // every point of the warp included: the straight-line step
-                  // (the same products as the masked path with a full mask)
-                  float2 zr, zi;
-                  step_seed(st, i, zr, zi);
-                  step_fast(st, zr, zi);
-                } else if (!__all_sync(0xffffffffu, all_out || nv == 0)) {
-                  // one masked path for every lane of the warp (excluded lanes
-                  // carry a zero mask); skipped only when the whole warp is out
-                  const float4 A = st[0], AT = st[1 * 32], R2 = st[2 * 32], X = st[3 * 32],
-                               Y = st[4 * 32];
-                  uint32_t mask = (all_out || nv == 0) ? 0u : 0xffffffffu;
-                  if (!all_in && !all_out && nv > 0) {
-                    const DirConst &d = sm.dc[warp][dsub];
-                    if (uniform) {
-                      // included points form an index interval; only points
-                      // inside the guard band need the exact FP64 test
-                      const float inv_adt = __frcp_rn(adt);  // adt > 0 here
-                      mask = omega_range_bits_r(w0f, dwf, inv_dwf, kPiLo * inv_adt, nv);
-                      uint32_t unc =
-                          omega_range_bits_r(w0f, dwf, inv_dwf, kPiHi * inv_adt, nv) & ~mask;
-                      while (unc) {
-                        const int m = __ffs(unc) - 1;
-                        unc &= unc - 1u;
-                        if (exact_mask(p, base, s, it_start, p.omega[j0 + m], d.n0, d.n1, d.cT))
-                          mask |= 1u << m;
-                      }
-                    } else {
-                      mask = 0;
-#pragma unroll 1
-                      for (int m = 0; m < nv; ++m) {
-                        const double wm = p.omega[j0 + m];
-                        const float ph = (float)fabs(wm) * adt;
-                        bool inc;
-                        if (ph < kPiLo) inc = true;
-                        else if (ph > kPiHi) inc = false;
-                        else inc = exact_mask(p, base, s, it_start, wm, d.n0, d.n1, d.cT);
-                        mask |= (uint32_t)inc << m;
-                      }
-                    }
-                  }
-                  // phasors as two packed chains from the reseeded first point
-                  // (uniform axis) or one reseed per point (non-uniform axis);
-                  // amplitudes zeroed per point where the step is masked out
-                  float2 ZrA, ZiA;
-                  step_seed(st, i, ZrA, ZiA);
-                  float2 ZrB, ZiB;
-                  rot2p(ZrA, ZiA, make_float2(X.z, X.w), make_float2(Y.x, Y.y),
-                        make_float2(Y.z, Y.w), ZrB, ZiB);
-#pragma unroll
-                  for (int q = 0; q < HP; ++q) {
-                    if (!uniform) {
-#pragma unroll
-                      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                          const int m = h * (K / 2) + 2 * q + e;
-                          const df wr = df_from_double(p.omega[j0 + min(m, max(nv - 1, 0))] * inv2pi);
-                          float ss, cc;
-                          phasor_rev(wr.hi, wr.lo, A.x, A.y, ss, cc);
-                          float2 &zr = h ? ZrB : ZrA;
-                          float2 &zi = h ? ZiB : ZiA;
-                          if (e == 0) { zr.x = cc; zi.x = ss; } else { zr.y = cc; zi.y = ss; }
-                        }
-                      }
-                    }
-                    // masked points: their phasors (not the amplitudes) are
-                    // zeroed, one packed product per chain and component
-                    const int mA = 2 * q, mB = K / 2 + 2 * q;
-                    const float2 gA = make_float2(((mask >> mA) & 1u) ? 1.f : 0.f,
-                                                  ((mask >> (mA + 1)) & 1u) ? 1.f : 0.f);
-                    const float2 gB = make_float2(((mask >> mB) & 1u) ? 1.f : 0.f,
-                                                  ((mask >> (mB + 1)) & 1u) ? 1.f : 0.f);
-                    const float2 at = make_float2(AT.x, AT.y), ap = make_float2(AT.z, AT.w);
-                    const float2 mrA = __fmul2_rn(ZrA, gA), miA = __fmul2_rn(ZiA, gA);
-                    const float2 mrB = __fmul2_rn(ZrB, gB), miB = __fmul2_rn(ZiB, gB);
-                    aTr[q] = __ffma2_rn(mrA, at, aTr[q]);
-                    aTi[q] = __ffma2_rn(miA, at, aTi[q]);
-                    aPr[q] = __ffma2_rn(mrA, ap, aPr[q]);
-                    aPi[q] = __ffma2_rn(miA, ap, aPi[q]);
-                    aTr[HP + q] = __ffma2_rn(mrB, at, aTr[HP + q]);
-                    aTi[HP + q] = __ffma2_rn(miB, at, aTi[HP + q]);
-                    aPr[HP + q] = __ffma2_rn(mrB, ap, aPr[HP + q]);
-                    aPi[HP + q] = __ffma2_rn(miB, ap, aPi[HP + q]);
-                    if (q + 1 < HP && uniform) {
-                      rot2p(ZrA, ZiA, make_float2(R2.x, R2.y), make_float2(R2.z, R2.w),
-                            make_float2(X.x, X.y), ZrA, ZiA);
-                      rot2p(ZrB, ZiB, make_float2(R2.x, R2.y), make_float2(R2.z, R2.w),
-                            make_float2(X.x, X.y), ZrB, ZiB);
-                    }
-                  }
-                }
-                if ((int64_t)s == snap.fire_it) {  // uniform over the CTA
-                  flush(snap.k);
-                  snap.advance(it_start, it_end, snaps, p.n_snaps);
-                }
               }
             }
             __syncwarp();
@@ -931,8 +804,8 @@ int launch_far_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size
   }
   void *tok = nullptr;
   timing_record(stream, true, &tok);
-  int rc = fl.on ? launch_fast_far(p, fl, stream) : SR_OK;
-  if (rc == SR_OK) rc = dispatch_k(cfg.K, p, cfg.grid, stream);
+  int rc = fl.on ? launch_fast_far(p, fl, stream) : dispatch_k(cfg.K, p, cfg.grid, stream);
+  if (rc == SR_OK) rc = launch_uneven_far(p, n_sm, stream);
   timing_record(stream, false, &tok);
   if (rc) return rc;
   const uint64_t total = (uint64_t)p.n_out * p.n_snaps * P;

@@ -105,11 +105,9 @@ size_t fast_workspace(const FastLayout &l) {
 void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
                unsigned char *status) {
   FastParams &f = p.fast;
-  if (!l.on) {
-    f.uneven = nullptr;
-    return;
-  }
   f.uneven = (unsigned int *)(status + 64);
+  f.M = 0;
+  if (!l.on) return;
   f.queue = (unsigned int *)(status + 192);
   f.deconv = (double *)base;
   f.twiddle = (float4 *)(base + (kFastMaxBand + 2) * 8);
@@ -132,6 +130,10 @@ void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char 
   f.n_phik = near ? 1u : std::min(p.n_phi, (p.n_theta + 30u) / p.n_theta + 1u);
   f.chunk = 32u;
   while (!near && f.chunk * f.n_phik > 128u) f.chunk /= 2u;
+}
+
+int launch_uneven_far(const FarMixedParams &p, int n_sm, cudaStream_t s) {
+  return launch_uneven<false>(p, n_sm, s);
 }
 
 int launch_fast_far(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {

@@ -265,6 +265,27 @@ struct FastUnit {
   int kphi;            // phi of the lane among the warp's (far)
 };
 
+__device__ __forceinline__ void lane_dir(const FarMixedParams &p, uint32_t iT, uint32_t,
+                                         LaneDir<false> &ld) {
+  const df c = df_from_double(1.0 - p.cos_theta[iT]), s = df_from_double(p.sin_theta[iT]);
+  ld.dc_h = c.hi; ld.dc_l = c.lo; ld.st_h = s.hi; ld.st_l = s.lo;
+  ld.f_dc = (float)(1.0 - p.cos_theta[iT]);
+  ld.f_st = (float)p.sin_theta[iT];
+  ld.f_ct = (float)p.cos_theta[iT];
+}
+__device__ __forceinline__ void lane_dir(const FarMixedParams &p, uint32_t iR, uint32_t iP,
+                                         LaneDir<true> &ld) {
+  const df x = df_from_double(p.sin_theta[iR] * p.cos_phi[iP]);
+  const df y = df_from_double(p.sin_theta[iR] * p.sin_phi[iP]);
+  const df L = df_from_double(p.L_screen);
+  ld.X_h = x.hi; ld.X_l = x.lo; ld.Y_h = y.hi; ld.Y_l = y.lo;
+  ld.L_h = L.hi; ld.L_l = L.lo;
+}
+__device__ __forceinline__ float4 phi_pairs(const FarMixedParams &p, uint32_t iP) {
+  const df c = df_from_double(p.cos_phi[iP]), s = df_from_double(p.sin_phi[iP]);
+  return make_float4(c.hi, c.lo, s.hi, s.lo);
+}
+
 template <bool NEAR>
 __device__ void unit_init(const FarMixedParams &p, uint32_t dwb, int lane, FastSmem &sm,
                           FastUnit<NEAR> &u) {
@@ -286,24 +307,9 @@ __device__ void unit_init(const FarMixedParams &p, uint32_t dwb, int lane, FastS
   u.dir = u.active ? u.slot0 + lane : n_dirs - 1;
   const uint32_t iT = u.dir % nT, iP = u.dir / nT, iP0 = u.slot0 / nT;
   u.kphi = (int)(iP - iP0);
+  lane_dir(p, iT, iP, u.ld);
   if constexpr (!NEAR) {
-    const df c = df_from_double(1.0 - p.cos_theta[iT]), s = df_from_double(p.sin_theta[iT]);
-    u.ld.dc_h = c.hi; u.ld.dc_l = c.lo; u.ld.st_h = s.hi; u.ld.st_l = s.lo;
-    u.ld.f_dc = (float)(1.0 - p.cos_theta[iT]);
-    u.ld.f_st = (float)p.sin_theta[iT];
-    u.ld.f_ct = (float)p.cos_theta[iT];
-    const uint32_t k = iP0 + lane;
-    if (lane < (int)f.n_phik) {
-      const df cp = df_from_double(p.cos_phi[min(k, p.n_phi - 1)]);
-      const df sp = df_from_double(p.sin_phi[min(k, p.n_phi - 1)]);
-      sm.phic[lane] = make_float4(cp.hi, cp.lo, sp.hi, sp.lo);
-    }
-  } else {
-    const df x = df_from_double(p.sin_theta[iT] * p.cos_phi[iP]);
-    const df y = df_from_double(p.sin_theta[iT] * p.sin_phi[iP]);
-    const df L = df_from_double(p.L_screen);
-    u.ld.X_h = x.hi; u.ld.X_l = x.lo; u.ld.Y_h = y.hi; u.ld.Y_l = y.lo;
-    u.ld.L_h = L.hi; u.ld.L_l = L.lo;
+    if (lane < (int)f.n_phik) sm.phic[lane] = phi_pairs(p, min(iP0 + lane, p.n_phi - 1));
   }
   __syncwarp();
 }
@@ -315,8 +321,8 @@ __device__ void unit_init(const FarMixedParams &p, uint32_t dwb, int lane, FastS
 // with rho = cos(phi) x + sin(phi) y.  Near: the records as they are.
 template <bool NEAR>
 __device__ __forceinline__ void stage_records(const FarMixedParams &p, int64_t g, uint32_t cnt,
-                                              int lane, FastSmem &sm) {
-  const uint32_t cs = p.fast.chunk;
+                                              uint32_t cs, uint32_t n_phik, int lane,
+                                              FastSmem &sm) {
   const float4 *src = p.records + g * kRecF4;
   if constexpr (NEAR) {
     if ((uint32_t)lane < cnt) {
@@ -324,7 +330,7 @@ __device__ __forceinline__ void stage_records(const FarMixedParams &p, int64_t g
       for (int k = 0; k < 3; ++k) sm.rec[lane * 3 + k] = __ldg(src + (size_t)lane * kRecF4 + k);
     }
   } else {
-    const uint32_t n = cs * p.fast.n_phik;
+    const uint32_t n = cs * n_phik;
     for (uint32_t i = lane; i < n; i += 32u) {
       const uint32_t k = i / cs, s = i % cs;
       if (s >= cnt) continue;
@@ -356,7 +362,7 @@ __device__ __forceinline__ float rcp_newton(float d) {
 // its amplitudes: far X = A_theta, Y = A_phi; near X_c, Y_c of component c
 // with A_c = Y_c + i omega X_c.
 template <bool NEAR>
-__device__ __forceinline__ df step_values(const FastUnit<NEAR> &u, const FastSmem &sm,
+__device__ __forceinline__ df step_values(const LaneDir<NEAR> &ld, const FastSmem &sm,
                                           uint32_t rec0, uint32_t i, float (&X)[NEAR ? 3 : 1],
                                           float (&Y)[NEAR ? 3 : 1]) {
   if constexpr (!NEAR) {
@@ -364,17 +370,17 @@ __device__ __forceinline__ df step_values(const FastUnit<NEAR> &u, const FastSme
     const float4 a = r[0], b = r[1], c = r[2];
     const float aphi = r[3].x;
     // tau = q + (1 - cos th) z - sin th rho  (double-float)
-    const df p1 = df_mul_raw(df{u.ld.dc_h, u.ld.dc_l}, df{a.z, a.w});
-    const df p2 = df_mul_raw(df{u.ld.st_h, u.ld.st_l}, df{b.x, b.y});
+    const df p1 = df_mul_raw(df{ld.dc_h, ld.dc_l}, df{a.z, a.w});
+    const df p2 = df_mul_raw(df{ld.st_h, ld.st_l}, df{b.x, b.y});
     const df s1 = two_sum(a.x, p1.hi);
     const df s2 = two_sum(s1.hi, -p2.hi);
     const df tau = fast_two_sum(s2.hi, ((a.y + p1.lo) - p2.lo) + (s1.lo + s2.lo));
-    const float D = c.x + u.ld.f_dc * b.w - u.ld.f_st * b.z;
+    const float D = c.x + ld.f_dc * b.w - ld.f_st * b.z;
     const float c2 = rcp_newton(D);
-    const float an = u.ld.f_st * c.z + u.ld.f_ct * c.w;
+    const float an = ld.f_st * c.z + ld.f_ct * c.w;
     const float c1 = an * c2 * c2;
-    const float tb = u.ld.f_ct * b.z - u.ld.f_st * b.w;
-    const float ta = u.ld.f_ct * c.z - u.ld.f_st * c.w;
+    const float tb = ld.f_ct * b.z - ld.f_st * b.w;
+    const float ta = ld.f_ct * c.z - ld.f_st * c.w;
     X[0] = -(c1 * tb + c2 * ta);
     Y[0] = -(c1 * c.y + c2 * aphi);
     return tau;
@@ -382,9 +388,9 @@ __device__ __forceinline__ df step_values(const FastUnit<NEAR> &u, const FastSme
     const float4 *r = sm.rec + i * 3u;
     const float4 r0 = r[0], r1 = r[1], r2 = r[2];
     // tau - L = (t - z) + rho^2 / (r + L - z)
-    const df ddx = df_sub(df{u.ld.X_h, u.ld.X_l}, df{r0.z, r0.w});
-    const df ddy = df_sub(df{u.ld.Y_h, u.ld.Y_l}, df{r1.x, r1.y});
-    const df D = df_sub(df{u.ld.L_h, u.ld.L_l}, df{r1.z, r1.w});
+    const df ddx = df_sub(df{ld.X_h, ld.X_l}, df{r0.z, r0.w});
+    const df ddy = df_sub(df{ld.Y_h, ld.Y_l}, df{r1.x, r1.y});
+    const df D = df_sub(df{ld.L_h, ld.L_l}, df{r1.z, r1.w});
     const df rho2 = df_add(df_mul(ddx, ddx), df_mul(ddy, ddy));
     const df rr = df_sqrt(df_add(rho2, df_mul(D, D)));
     const df F = (D.hi > 0.f) ? df_div(rho2, df_add(rr, D)) : df_sub(rr, D);
@@ -610,12 +616,12 @@ __device__ __forceinline__ void spread_steps(const FarMixedParams &p, const Fast
     // the step before `from` stands alone, so that chunks start at `from`
     cnt = s0 < from ? 1u : min(cs, b - s0);
     __syncwarp();
-    stage_records<NEAR>(p, base + s0, cnt, lane, sm);
+    stage_records<NEAR>(p, base + s0, cnt, cs, p.fast.n_phik, lane, sm);
 #pragma unroll 1
     for (uint32_t i = 0; i < cnt; ++i) {
       const uint32_t s = s0 + i;
       float X[NP], Y[NP];
-      const df tau = step_values<NEAR>(u, sm, rec0, i, X, Y);
+      const df tau = step_values<NEAR>(u.ld, sm, rec0, i, X, Y);
       // the track's first step compares its whole phase with zero
       // (synchrad/kernel_farfield.cl:49, kernel_nearfield.cl:48)
       float dt0 = (tau.hi - w.tp_h) + (tau.lo - w.tp_l);
@@ -759,9 +765,78 @@ __device__ __forceinline__ bool spread_range(const FarMixedParams &p, const Fast
   return w.dirty;
 }
 
+// One pair of amplitudes A (X), B (Y) at frequency j of a direction, as the
+// comp wants it, added to the partial spectrum `out`; A is also kept for the
+// adjoints where asked.
+template <bool NEAR>
+__device__ __forceinline__ void emit_point(const FarMixedParams &p, uint32_t dir, int c, uint32_t j,
+                                           uint32_t t, uint32_t ksnap, double wpdt2, double wpdt,
+                                           double *out, double Ar, double Ai, double Br,
+                                           double Bi) {
+  const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
+  const uint64_t gti = (uint64_t)j + (uint64_t)p.n_omega * dir;
+  const uint32_t iT = dir % p.n_theta, iP = dir / p.n_theta;
+  auto add = [&](int o, double v) {
+    red_f64(out + ((uint64_t)o * p.n_snaps + ksnap) * P + gti, v);
+  };
+  if constexpr (!NEAR) {
+    if (p.save_A != nullptr)
+      reinterpret_cast<float4 *>(p.save_A)[((uint64_t)t * p.n_snaps + ksnap) * P + gti] =
+          make_float4((float)Ar, (float)Ai, (float)Br, (float)Bi);
+    if (p.comp == SR_COMP_TOTAL) {
+      add(0, wpdt2 * (Ar * Ar + Ai * Ai + Br * Br + Bi * Bi));
+    } else if (p.comp == SR_COMP_SPHERIC) {
+      add(1, wpdt2 * (Ar * Ar + Ai * Ai));
+      add(2, wpdt2 * (Br * Br + Bi * Bi));
+    } else if (p.comp == SR_COMP_SPHERIC_COMPLEX) {
+      add(2, wpdt * Ar);
+      add(3, wpdt * Ai);
+      add(4, wpdt * Br);
+      add(5, wpdt * Bi);
+    } else {
+      const double cT = p.cos_theta[iT], sT = p.sin_theta[iT];
+      const double cP = p.cos_phi[iP], sP = p.sin_phi[iP];
+      const double hx = cT * cP, hy = cT * sP;
+      const double xr = hx * Ar - sP * Br, xi = hx * Ai - sP * Bi;
+      const double yr = hy * Ar + cP * Br, yi = hy * Ai + cP * Bi;
+      const double zr = -sT * Ar, zi = -sT * Ai;
+      if (p.comp == SR_COMP_CARTESIAN) {
+        add(0, wpdt2 * (xr * xr + xi * xi));
+        add(1, wpdt2 * (yr * yr + yi * yi));
+        add(2, wpdt2 * (zr * zr + zi * zi));
+      } else {
+        const double f = wpdt * p.form_factor[j];
+        add(0, f * xr);
+        add(1, f * xi);
+        add(2, f * yr);
+        add(3, f * yi);
+        add(4, f * zr);
+        add(5, f * zi);
+      }
+    }
+  } else {
+    const double w = p.omega[j];
+    const double Er = Br - w * Ai, Ei = Bi + w * Ar;  // Y + i omega X
+    if (p.save_A != nullptr) {
+      float *sa = p.save_A + 8 * (((uint64_t)t * p.n_snaps + ksnap) * P + gti);
+      reinterpret_cast<float2 *>(sa)[c] = make_float2((float)Er, (float)Ei);
+      if (c == 2) reinterpret_cast<float2 *>(sa)[3] = make_float2(0.f, 0.f);
+    }
+    if (p.comp == SR_COMP_TOTAL) {
+      add(0, wpdt2 * (Er * Er + Ei * Ei));
+    } else if (p.comp == SR_COMP_CARTESIAN) {
+      add(c, wpdt2 * (Er * Er + Ei * Ei));
+    } else {  // cartesian_complex (FormFactor not applied)
+      double sL, cL;
+      sincos(w * p.L_screen, &sL, &cL);
+      add(2 * c, wpdt * (Er * cL - Ei * sL));
+      add(2 * c + 1, wpdt * (Er * sL + Ei * cL));
+    }
+  }
+}
+
 // The spectrum of one pair of fields, X and Y (band sums xs, ys, undivided),
-// added to the partial spectrum of track subset `sub`; A is also kept for
-// the adjoints where asked.
+// added to the partial spectrum of track subset `sub`.
 template <bool NEAR>
 __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUnit<NEAR> &u,
                                           uint32_t dir, int d, int c, const float2 *xs,
@@ -771,7 +846,6 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
   const double wp = p.weight[t];
   const double wpdt2 = wp * p.dt * p.dt, wpdt = sqrt(wp) * p.dt;
   double *out = p.partial + (uint64_t)sub * p.n_out * p.n_snaps * P;
-  const uint32_t iT = dir % p.n_theta, iP = dir / p.n_theta;
   bool listed = p.save_A != nullptr;
   for (int i = 0; i < n_seg; ++i) listed = listed || ((dirty[(size_t)i * p.fast.n_dwb] >> d) & 1u);
   const uint64_t g0 = (uint64_t)u.j0 + (uint64_t)p.n_omega * dir;
@@ -809,64 +883,7 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
         Br += (double)v.z + (double)l.z;
         Bi += (double)v.w + (double)l.w;
       }
-    const uint64_t gti = g0 + m;
-    auto add = [&](int o, double v) {
-      red_f64(out + ((uint64_t)o * p.n_snaps + ksnap) * P + gti, v);
-    };
-    if constexpr (!NEAR) {
-      if (p.save_A != nullptr)
-        reinterpret_cast<float4 *>(p.save_A)[((uint64_t)t * p.n_snaps + ksnap) * P + gti] =
-            make_float4((float)Ar, (float)Ai, (float)Br, (float)Bi);
-      if (p.comp == SR_COMP_TOTAL) {
-        add(0, wpdt2 * (Ar * Ar + Ai * Ai + Br * Br + Bi * Bi));
-      } else if (p.comp == SR_COMP_SPHERIC) {
-        add(1, wpdt2 * (Ar * Ar + Ai * Ai));
-        add(2, wpdt2 * (Br * Br + Bi * Bi));
-      } else if (p.comp == SR_COMP_SPHERIC_COMPLEX) {
-        add(2, wpdt * Ar);
-        add(3, wpdt * Ai);
-        add(4, wpdt * Br);
-        add(5, wpdt * Bi);
-      } else {
-        const double cT = p.cos_theta[iT], sT = p.sin_theta[iT];
-        const double cP = p.cos_phi[iP], sP = p.sin_phi[iP];
-        const double hx = cT * cP, hy = cT * sP;
-        const double xr = hx * Ar - sP * Br, xi = hx * Ai - sP * Bi;
-        const double yr = hy * Ar + cP * Br, yi = hy * Ai + cP * Bi;
-        const double zr = -sT * Ar, zi = -sT * Ai;
-        if (p.comp == SR_COMP_CARTESIAN) {
-          add(0, wpdt2 * (xr * xr + xi * xi));
-          add(1, wpdt2 * (yr * yr + yi * yi));
-          add(2, wpdt2 * (zr * zr + zi * zi));
-        } else {
-          const double f = wpdt * p.form_factor[u.j0 + m];
-          add(0, f * xr);
-          add(1, f * xi);
-          add(2, f * yr);
-          add(3, f * yi);
-          add(4, f * zr);
-          add(5, f * zi);
-        }
-      }
-    } else {
-      const double w = p.omega[u.j0 + m];
-      const double Er = Br - w * Ai, Ei = Bi + w * Ar;  // Y + i omega X
-      if (p.save_A != nullptr) {
-        float *sa = p.save_A + 8 * (((uint64_t)t * p.n_snaps + ksnap) * P + gti);
-        reinterpret_cast<float2 *>(sa)[c] = make_float2((float)Er, (float)Ei);
-        if (c == 2) reinterpret_cast<float2 *>(sa)[3] = make_float2(0.f, 0.f);
-      }
-      if (p.comp == SR_COMP_TOTAL) {
-        add(0, wpdt2 * (Er * Er + Ei * Ei));
-      } else if (p.comp == SR_COMP_CARTESIAN) {
-        add(c, wpdt2 * (Er * Er + Ei * Ei));
-      } else {  // cartesian_complex (FormFactor not applied)
-        double sL, cL;
-        sincos(w * p.L_screen, &sL, &cL);
-        add(2 * c, wpdt * (Er * cL - Ei * sL));
-        add(2 * c + 1, wpdt * (Er * sL + Ei * cL));
-      }
-    }
+    emit_point<NEAR>(p, dir, c, u.j0 + m, t, ksnap, wpdt2, wpdt, out, Ar, Ai, Br, Bi);
   }
 }
 
@@ -1133,6 +1150,167 @@ fast_transform_kernel(const __grid_constant__ FarMixedParams p) {
   }
 }
 
+// Axes that are not evenly spaced: a sine and a cosine per point and step.  A
+// warp takes (direction, 32 K frequencies, track subset) items; its lanes
+// compute tau and the amplitudes of 32 steps, one each, then every lane sums
+// its K frequencies lane + 32 m over them (the frequencies as double-floats in
+// registers; the FP32 sums fold into compensated pairs every 1024 steps).
+// Bound by the XU pipe: two hardware functions per point and step, 0.125
+// cycles per SM.
+template <bool NEAR, int K>
+__global__ void __launch_bounds__(kFastWarps * 32, 3)
+uneven_axis_kernel(const __grid_constant__ FarMixedParams p) {
+  if (*p.fast.uneven == 0u) return;
+  constexpr int NP = NEAR ? 3 : 1, NV = 4 * NP;  // pairs, real sums per point
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  FastSmem &sm = reinterpret_cast<FastSmem *>(smem_raw)[warp];
+  float4 *sv = sm.rec + 160;                           // tau.hi, tau.lo, |dtau| of a step
+  float2 *sa = reinterpret_cast<float2 *>(sm.rec + 192);  // [NP][32] amplitudes X, Y
+  const uint32_t n_dirs = p.n_theta * p.n_phi, nO = p.n_omega;
+  const uint64_t P = (uint64_t)nO * n_dirs;
+  const uint32_t tiles = (nO + 32 * K - 1) / (32 * K);
+  const uint64_t n_items = (uint64_t)n_dirs * tiles * p.n_sub;
+  const double inv2pi = 0.15915494309189533577;
+  for (;;) {
+    uint32_t item32 = 0;
+    if (lane == 0) item32 = atomicAdd(p.queue, 1u);
+    const uint64_t item = __shfl_sync(0xffffffffu, item32, 0);
+    if (item >= n_items) return;
+    const uint32_t sub = (uint32_t)(item / ((uint64_t)n_dirs * tiles));
+    const uint32_t rest = (uint32_t)(item % ((uint64_t)n_dirs * tiles));
+    const uint32_t dir = rest / tiles, j0 = (rest % tiles) * 32u * K + lane;
+    const uint32_t iT = dir % p.n_theta, iP = dir / p.n_theta;
+    LaneDir<NEAR> ld;
+    lane_dir(p, iT, iP, ld);
+    __syncwarp();
+    if constexpr (!NEAR) {
+      if (lane == 0) sm.phic[0] = phi_pairs(p, iP);
+    }
+    __syncwarp();
+    float wh[K], wl[K], wa[K];
+    float wmax = 0.f;
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      const double w = p.omega[min(j0 + 32u * m, nO - 1u)];
+      const df r = df_from_double(w * inv2pi);
+      wh[m] = r.hi;
+      wl[m] = r.lo;
+      wa[m] = (float)fabs(w);
+      wmax = wa[m] <= 3.0e38f ? fmaxf(wmax, wa[m]) : INFINITY;  // NaN and infinity too
+    }
+    double *out = p.partial + (uint64_t)sub * p.n_out * p.n_snaps * P;
+    uint32_t t0, t1;
+    subset_tracks(p, sub, t0, t1);
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t n_body = track_body(p, t);
+      const uint32_t it_start = p.it_start[t], it_end = p.it_end[t];
+      const uint32_t *snaps = p.snap_its + (size_t)t * p.snap_stride;
+      SnapState snap;
+      snap.init(it_start, it_end, snaps, p.n_snaps);
+      if (snap.fire_it == SnapState::NEVER) continue;
+      const int64_t base = p.offsets[t];
+      const double wpdt2 = p.weight[t] * p.dt * p.dt, wpdt = sqrt(p.weight[t]) * p.dt;
+      float acc[K][NV], hi[K][NV], lo[K][NV];
+#pragma unroll
+      for (int m = 0; m < K; ++m)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[m][v] = hi[m][v] = lo[m][v] = 0.f;
+      auto fold = [&]() {
+#pragma unroll
+        for (int m = 0; m < K; ++m)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            const df e = two_sum(hi[m][v], acc[m][v]);
+            hi[m][v] = e.hi;
+            lo[m][v] += e.lo;
+            acc[m][v] = 0.f;
+          }
+      };
+      auto flush = [&]() {
+        fold();
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+          const uint32_t j = j0 + 32u * m;
+          if (j < nO) {
+#pragma unroll
+            for (int c = 0; c < NP; ++c) {
+              auto val = [&](int v) { return (double)hi[m][4 * c + v] + (double)lo[m][4 * c + v]; };
+              emit_point<NEAR>(p, dir, c, j, t, snap.k, wpdt2, wpdt, out, val(0), val(1), val(2),
+                               val(3));
+            }
+          }
+        }
+        snap.advance(it_start, it_end, snaps, p.n_snaps);
+      };
+      float tp_h = 0.f, tp_l = 0.f;
+      for (uint32_t s0 = 0; s0 < n_body && snap.fire_it != SnapState::NEVER; s0 += 32) {
+        const uint32_t cnt = min(32u, n_body - s0);
+        __syncwarp();
+        stage_records<NEAR>(p, base + s0, cnt, 32u, 1u, lane, sm);
+        {
+          const uint32_t l = min((uint32_t)lane, cnt - 1);
+          float X[NP], Y[NP];
+          const df tau = step_values<NEAR>(ld, sm, 0u, l, X, Y);
+          float ph = __shfl_up_sync(0xffffffffu, tau.hi, 1);
+          float pl = __shfl_up_sync(0xffffffffu, tau.lo, 1);
+          if (lane == 0) { ph = tp_h; pl = tp_l; }
+          float dt0 = (tau.hi - ph) + (tau.lo - pl);
+          if (s0 + l == 0) {  // the first step's whole phase is compared with zero
+            dt0 = tau.hi + tau.lo;
+            if constexpr (NEAR) dt0 += ld.L_h + ld.L_l;
+          }
+          tp_h = __shfl_sync(0xffffffffu, tau.hi, cnt - 1);
+          tp_l = __shfl_sync(0xffffffffu, tau.lo, cnt - 1);
+          sv[lane] = make_float4(tau.hi, tau.lo, fabsf(dt0), 0.f);
+#pragma unroll
+          for (int c = 0; c < NP; ++c) sa[c * 32 + lane] = make_float2(X[c], Y[c]);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t i = 0; i < cnt; ++i) {
+          const float4 q = sv[i];
+          float2 am[NP];
+#pragma unroll
+          for (int c = 0; c < NP; ++c) am[c] = sa[c * 32 + i];
+          const bool all_in = __all_sync(0xffffffffu, wmax * q.z < kPiLo);
+#pragma unroll
+          for (int m = 0; m < K; ++m) {
+            bool in = true;
+            if (!all_in) {
+              const float ph = wa[m] * q.z;
+              if (ph < kPiLo) {
+                in = true;
+              } else if (ph > kPiHi) {
+                in = false;
+              } else {
+                const double w = p.omega[min(j0 + 32u * m, nO - 1u)];
+                const double n0 = p.sin_theta[iT] * p.cos_phi[iP];
+                const double n1 = p.sin_theta[iT] * p.sin_phi[iP];
+                in = NEAR ? exact_mask_near(p, base, s0 + i, it_start, w, n0, n1)
+                          : exact_mask(p, base, s0 + i, it_start, w, n0, n1, p.cos_theta[iT]);
+              }
+            }
+            float sn, cs;
+            phasor_rev(wh[m], wl[m], q.x, q.y, sn, cs);
+            if (!in) sn = cs = 0.f;
+#pragma unroll
+            for (int c = 0; c < NP; ++c) {
+              acc[m][4 * c + 0] = __fmaf_rn(am[c].x, cs, acc[m][4 * c + 0]);
+              acc[m][4 * c + 1] = __fmaf_rn(am[c].x, sn, acc[m][4 * c + 1]);
+              acc[m][4 * c + 2] = __fmaf_rn(am[c].y, cs, acc[m][4 * c + 2]);
+              acc[m][4 * c + 3] = __fmaf_rn(am[c].y, sn, acc[m][4 * c + 3]);
+            }
+          }
+          if ((int64_t)(s0 + i) == snap.fire_it) flush();  // uniform over the warp
+        }
+        if (((s0 + 32) & 1023u) == 0) fold();
+      }
+      while (snap.fire_it != SnapState::NEVER) flush();  // due after the last body step
+    }
+  }
+}
+
 // ------------------------------------------------------------------ host side
 template <bool NEAR, int R1>
 int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
@@ -1152,6 +1330,39 @@ int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) 
   const uint32_t items = l.n_dwb * (32u / l.dirs_per_warp) * l.n_sub * p.n_snaps;
   fast_transform_kernel<NEAR, R1><<<(items + kFastWarps - 1) / kFastWarps, threads, smem, s>>>(p);
   return cuda_fail(cudaGetLastError(), "fast sum launch");
+}
+
+template <bool NEAR, int K>
+int launch_uneven_k(const FarMixedParams &p, int n_sm, cudaStream_t s) {
+  constexpr int smem = (int)sizeof(FastSmem) * kFastWarps;
+  const cudaError_t e = allow_smem((const void *)uneven_axis_kernel<NEAR, K>, smem);
+  if (e != cudaSuccess) return cuda_fail(e, "uneven axis smem attribute");
+  uneven_axis_kernel<NEAR, K><<<(unsigned)n_sm * 3, kFastWarps * 32, smem, s>>>(p);
+  return cuda_fail(cudaGetLastError(), "uneven axis launch");
+}
+
+// The fewest tiles of at most 8 (near: 3) x 32 frequencies, and the fewest
+// frequencies per lane that fill them.
+template <bool NEAR>
+int launch_uneven(const FarMixedParams &p, int n_sm, cudaStream_t s) {
+  constexpr uint32_t most = NEAR ? 3 : 8;
+  const uint32_t tiles = (p.n_omega + 32 * most - 1) / (32 * most);
+  const uint32_t K = (p.n_omega + 32 * tiles - 1) / (32 * tiles);
+  switch (K) {
+    case 1: return launch_uneven_k<NEAR, 1>(p, n_sm, s);
+    case 2: return launch_uneven_k<NEAR, 2>(p, n_sm, s);
+    case 3: return launch_uneven_k<NEAR, 3>(p, n_sm, s);
+  }
+  if constexpr (!NEAR) {
+    switch (K) {
+      case 4: return launch_uneven_k<NEAR, 4>(p, n_sm, s);
+      case 5: return launch_uneven_k<NEAR, 5>(p, n_sm, s);
+      case 6: return launch_uneven_k<NEAR, 6>(p, n_sm, s);
+      case 7: return launch_uneven_k<NEAR, 7>(p, n_sm, s);
+      case 8: return launch_uneven_k<NEAR, 8>(p, n_sm, s);
+    }
+  }
+  return fail(SR_ERR_INVALID, "%u frequencies per lane", K);
 }
 
 template <bool NEAR>

@@ -35,7 +35,7 @@ int launch_port(const PortParams &p, int mode, int comp, int dtype, bool native,
                 cudaStream_t stream);
 
 // Arguments of the summation by transforms (sr_fast_sum.cuh), for evenly
-// spaced omega axes.
+// spaced omega axes, and the test of the axis.
 struct FastParams {
   unsigned int *uneven;  // set by the record pass when the axis is not evenly spaced
   unsigned int *queue;   // next work item (zeroed per launch)
@@ -45,7 +45,7 @@ struct FastParams {
   unsigned char *scratch;
   unsigned long long slice_bytes;
   uint32_t n_bands, nb;  // omega bands and the frequencies of one
-  uint32_t M;            // cells of a circle
+  uint32_t M;            // cells of a circle; 0: term by term
   uint32_t n_dwb;        // (32 directions) x bands
   uint32_t n_sub;        // track subsets
   uint32_t n_segs;       // few tracks: segments of seg_steps steps, of all tracks
@@ -95,7 +95,7 @@ struct FarMixedParams {
   unsigned int *queue;   // work items handed out after each CTA's first (zeroed per launch)
   // outputs
   double *out[6];
-  FastParams fast;       // fast.uneven == nullptr: term by term only
+  FastParams fast;       // fast.M == 0: no summation by transforms
 };
 
 struct FarMixedConfig {
@@ -127,6 +127,8 @@ size_t fast_workspace(const FastLayout &l);
 // status block at `status`).
 void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
                unsigned char *status);
+int launch_uneven_far(const FarMixedParams &p, int n_sm, cudaStream_t s);
+int launch_uneven_near(const FarMixedParams &p, int n_sm, cudaStream_t s);
 int launch_fast_far(const FarMixedParams &p, const FastLayout &l, cudaStream_t s);
 int launch_fast_near(const FarMixedParams &p, const FastLayout &l, cudaStream_t s);
 

@@ -186,14 +186,13 @@ __device__ __forceinline__ void cmul(float ar, float ai, float br, float bi, flo
   ci = ar * bi + ai * br;
 }
 
-// Whether this launch's axis is summed by transforms (sr_fast_sum.cuh): the
-// kernels that sum term by term leave at once then, and the other way round.
+// Whether this launch's axis is summed by transforms (sr_fast_sum.cuh).
 __device__ __forceinline__ bool by_transform(const FarMixedParams &p) {
-  return p.fast.uneven != nullptr && *p.fast.uneven == 0u;
+  return p.fast.M != 0u && *p.fast.uneven == 0u;
 }
 
-// Tables of the summation by transforms, made beside the step records: the
-// test of the omega axis (omega_j = omega_0 + j d_omega to 1e-12), the
+// The test of the omega axis (omega_j = omega_0 + j d_omega to 1e-12), made
+// beside the step records, and the tables of the summation by transforms: the
 // reciprocal transform of the Kaiser-Bessel spreading kernel,
 // phi^(xi) = 8 sinh(s) / (s I0(beta)), s = sqrt(beta^2 - (8 pi xi)^2) at
 // xi = i / M, and the twiddle factors.
@@ -205,13 +204,16 @@ __device__ __forceinline__ void fast_tables(const FarMixedParams &p) {
   if (f.uneven == nullptr) return;
   const uint32_t nt = gridDim.x * blockDim.x, gt = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t n = p.n_omega;
-  const double w0 = p.omega[0], dw = (p.omega[n - 1] - w0) / (double)(n - 1);
-  bool bad = !(fabs(dw) > 0.0) || !isfinite(dw);
+  const double w0 = p.omega[0], dw = n > 1 ? (p.omega[n - 1] - w0) / (double)(n - 1) : 0.0;
+  // the term-by-term kernels pack frequency indices in 16 bits
+  bool bad = (f.M == 0u && n >= 65535u) ||
+             (n > 1 && (!(fabs(dw) > 0.0) || !isfinite(dw)));
   for (uint32_t j = gt; j < n; j += nt) {
     const double wj = p.omega[j];
     if (!(fabs(wj - (w0 + (double)j * dw)) <= 1e-12 * fabs(wj) + 1e-300)) bad = true;
   }
   if (bad) atomicOr(f.uneven, 1u);
+  if (f.M == 0u) return;
   if (threadIdx.x < 32u)  // one warp of each block: FP64 functions spread over the SMs
     for (uint32_t i = blockIdx.x * 32u + threadIdx.x; i < f.M; i += gridDim.x * 32u) {
       double sn, cn;  // f.M = 32 (M / 32) twiddles

@@ -121,7 +121,7 @@ __device__ __forceinline__ void near_accumulate(NearAcc<K> &a, int q, float2 zr,
 
 template <int K, int W>
 __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p) {
-  if (by_transform(p)) return;
+  if (*p.fast.uneven != 0u) return;  // uneven_axis_kernel's
   static_assert(K == 8 || K == 16, "K");
   constexpr int KP = K / 2, HP = KP / 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -184,11 +184,9 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
     const double w0d = nv > 0 ? p.omega[j0] : 0.0;
     const df d_w0 = df_from_double(w0d * inv2pi);
     const float w0f = (float)w0d, dwf = (float)dw_glob;
-    bool uniform = true;
     float wabs_min = 3.0e38f, wabs_max = 0.f;
     for (int m = 0; m < nv; ++m) {
       const double wm = p.omega[j0 + m];
-      if (fabs(wm - (w0d + (double)m * dw_glob)) > 1e-12 * fabs(wm) + 1e-300) uniform = false;
       wabs_min = fminf(wabs_min, (float)fabs(wm));
       wabs_max = fmaxf(wabs_max, (float)fabs(wm));
     }
@@ -314,7 +312,7 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
         ZrA = make_float2(zc, zc * A.z - zs * A.w);
         ZiA = make_float2(zs, zc * A.w + zs * A.z);
       };
-      // One fully included step on a uniform axis: two packed chains of pairs.
+      // One fully included step: two packed chains of pairs.
       auto step_fast = [&](const float4 *st, float2 ZrA, float2 ZiA) {
         const float4 F1 = st[1 * 32], F2 = st[2 * 32], F3 = st[3 * 32], R2 = st[4 * 32],
                      X = st[5 * 32], Y = st[6 * 32];
@@ -438,7 +436,7 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
                                    snap.fire_it < (int64_t)(s0 + c0 + mcnt);
             // warp-uniform choice: the whole warp runs the tight loop or the
             // general one (lanes of a warp never diverge between the two)
-            if (__all_sync(0xffffffffu, uniform && !fire_here &&
+            if (__all_sync(0xffffffffu, !fire_here &&
                            wabs_max * sm.sc[warp][dsub].adt_max < kPiLo)) {
               const float4 *st = setup + (size_t)dsub * kNSetupF4 * 32;
               for (uint32_t i = 0; i < mcnt; ++i) {
@@ -454,7 +452,7 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
                 const uint32_t s = s0 + c0 + i;
                 const bool all_in = wabs_max * adt < kPiLo;
                 const bool all_out = wabs_min * adt > kPiHi;
-                if (__all_sync(0xffffffffu, uniform && (all_in || nv == 0))) {
+                if (__all_sync(0xffffffffu, all_in || nv == 0)) {
                   // every point of the warp included: the straight-line step
                   // (the same products as the masked path with a full mask)
                   float2 zr, zi;
@@ -463,41 +461,26 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
                 } else if (!__all_sync(0xffffffffu, all_out || nv == 0)) {
                   // one masked path for every lane of the warp (excluded lanes
                   // carry a zero mask); skipped only when the whole warp is out
-                  const float4 A = st[0], F1 = st[1 * 32], F2 = st[2 * 32], F3 = st[3 * 32],
+                  const float4 F1 = st[1 * 32], F2 = st[2 * 32], F3 = st[3 * 32],
                                R2 = st[4 * 32], X = st[5 * 32], Y = st[6 * 32];
                   uint32_t mask = (all_out || nv == 0) ? 0u : 0xffffffffu;
                   if (!all_in && !all_out && nv > 0) {
                     const ScreenConst &c = sm.sc[warp][dsub];
-                    if (uniform) {
-                      // included points form an index interval; only points
-                      // inside the guard band need the exact FP64 test
-                      const float inv_adt = __frcp_rn(adt);  // adt > 0 here
-                      const float inv_dwf = (dwf != 0.f) ? __frcp_rn(dwf) : 0.f;
-                      mask = omega_range_bits_r(w0f, dwf, inv_dwf, kPiLo * inv_adt, nv);
-                      uint32_t unc =
-                          omega_range_bits_r(w0f, dwf, inv_dwf, kPiHi * inv_adt, nv) & ~mask;
-                      while (unc) {
-                        const int m = __ffs(unc) - 1;
-                        unc &= unc - 1u;
-                        if (exact_mask_near(p, base, s, it_start, p.omega[j0 + m], c.P0, c.P1))
-                          mask |= 1u << m;
-                      }
-                    } else {
-                      mask = 0;
-#pragma unroll 1
-                      for (int m = 0; m < nv; ++m) {
-                        const double wm = p.omega[j0 + m];
-                        const float phd = (float)fabs(wm) * adt;
-                        bool inc;
-                        if (phd < kPiLo) inc = true;
-                        else if (phd > kPiHi) inc = false;
-                        else inc = exact_mask_near(p, base, s, it_start, wm, c.P0, c.P1);
-                        mask |= (uint32_t)inc << m;
-                      }
+                    // included points form an index interval; only points
+                    // inside the guard band need the exact FP64 test
+                    const float inv_adt = __frcp_rn(adt);  // adt > 0 here
+                    const float inv_dwf = (dwf != 0.f) ? __frcp_rn(dwf) : 0.f;
+                    mask = omega_range_bits_r(w0f, dwf, inv_dwf, kPiLo * inv_adt, nv);
+                    uint32_t unc =
+                        omega_range_bits_r(w0f, dwf, inv_dwf, kPiHi * inv_adt, nv) & ~mask;
+                    while (unc) {
+                      const int m = __ffs(unc) - 1;
+                      unc &= unc - 1u;
+                      if (exact_mask_near(p, base, s, it_start, p.omega[j0 + m], c.P0, c.P1))
+                        mask |= 1u << m;
                     }
                   }
-                  // phasors as two packed chains (uniform axis) or one reseed per
-                  // point (non-uniform axis); amplitudes zeroed where masked out
+                  // phasors as two packed chains, zeroed where masked out
                   float2 ZrA, ZiA;
                   step_seed(st, i, ZrA, ZiA);
                   float2 ZrB, ZiB;
@@ -510,16 +493,6 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
                       float2 &zr = h ? ZrB : ZrA;
                       float2 &zi = h ? ZiB : ZiA;
                       const int m0 = h * (K / 2) + 2 * q;
-                      if (!uniform) {
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                          const df wr =
-                              df_from_double(p.omega[j0 + min(m0 + e, max(nv - 1, 0))] * inv2pi);
-                          float ss, cc;
-                          phasor_rev(wr.hi, wr.lo, A.x, A.y, ss, cc);
-                          if (e == 0) { zr.x = cc; zi.x = ss; } else { zr.y = cc; zi.y = ss; }
-                        }
-                      }
                       // masked points: their phasors (not the six amplitudes)
                       // are zeroed, one packed product per component
                       const float2 g = make_float2(((mask >> m0) & 1u) ? 1.f : 0.f,
@@ -531,7 +504,7 @@ __global__ void __launch_bounds__(W * 32, 1) near_mixed_kernel(FarMixedParams p)
                       near_accumulate(acc, h * HP + q, __fmul2_rn(zr, g), __fmul2_rn(zi, g), bb,
                                       aa);
                     }
-                    if (q + 1 < HP && uniform) {
+                    if (q + 1 < HP) {
                       rot2p(ZrA, ZiA, make_float2(R2.x, R2.y), make_float2(R2.z, R2.w),
                             make_float2(X.x, X.y), ZrA, ZiA);
                       rot2p(ZrB, ZiB, make_float2(R2.x, R2.y), make_float2(R2.z, R2.w),
@@ -702,10 +675,10 @@ int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, siz
     return fail(SR_ERR_INVALID, "near field: points per lane %d (8 or 16)", cfg.K);
   void *tok = nullptr;
   timing_record(stream, true, &tok);
-  int rc = fl.on ? launch_fast_near(p, fl, stream) : SR_OK;
-  if (rc == SR_OK)
-    rc = (cfg.K == 16) ? launch_near_main<16>(p, cfg.grid, stream)
-                       : launch_near_main<8>(p, cfg.grid, stream);
+  int rc = fl.on         ? launch_fast_near(p, fl, stream)
+           : cfg.K == 16 ? launch_near_main<16>(p, cfg.grid, stream)
+                         : launch_near_main<8>(p, cfg.grid, stream);
+  if (rc == SR_OK) rc = launch_uneven_near(p, n_sm, stream);
   timing_record(stream, false, &tok);
   if (rc) return rc;
   const uint64_t total = (uint64_t)p.n_out * p.n_snaps * P;

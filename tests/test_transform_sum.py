@@ -117,6 +117,21 @@ def test_axes(mode, axis):
     _check(*_spectra(w, axis=f))
 
 
+@pytest.mark.parametrize("mode", ["far", "near"])
+@pytest.mark.parametrize("n_omega,periods", [(2, 10), (33, 10), (95, 40), (97, 10), (160, 70),
+                                             (192, 10), (224, 10), (257, 40), (600, 10)])
+def test_uneven_axis_sizes(mode, n_omega, periods):
+    """Axes that are not even, at the frequency counts where a lane takes one
+    more frequency or a warp one more tile; coarse tracks (many periods) are cut
+    by the |dphase| < pi rule.  One term is a hardware sine and cosine (2e-7
+    rad) of a phase good to 1e-7: 4e-7 of the amplitude's norm at most."""
+    _need_gpu()
+    make = wl.c2_far_mixed if mode == "far" else wl.c5_near_helical
+    w = make(n_tracks=3, n_steps=300, grid=(n_omega, 3, 3), n_periods=periods)
+    _check(*_spectra(w, snaps=2, axis=lambda o: np.sort(o[0] + (o[-1] - o[0]) * np.linspace(
+        0, 1, o.size) ** 1.5)))
+
+
 @pytest.mark.parametrize("mode,comp", [("far", "cartesian"), ("far", "cartesian_complex"),
                                        ("far", "spheric"), ("far", "spheric_complex"),
                                        ("near", "cartesian"), ("near", "cartesian_complex")])
