@@ -34,6 +34,7 @@
 
 #include "sr_common.cuh"
 #include "sr_internal.h"
+#include "sr_fast_sum.cuh"
 #include "sr_mixed_common.cuh"
 #include "sr_adjoint_common.cuh"
 
@@ -56,7 +57,11 @@ struct AdjParams {
   float4 *dirtab;              // [n_dirs][4] direction constants
   AdjGlobals *glob;
   int64_t *item_off;           // [n_tracks + 1] first work item of each track
-  double *gstep;               // [total_steps][kAG] per-step gradients (bbar, a form)
+  double *gstep;               // [n_split][total_steps][kAG] per-step gradients (bbar, a form)
+  uint32_t n_split;            // runs of directions summed apart
+  float4 *bandtab;             // [n_bands] centre frequency / 2 pi
+  float2 *fields;              // transforms' cells of a batch of tracks (see below)
+  uint32_t t_lo, t_hi;         // the batch
   double *grad[6];             // x, y, z, ux, uy, uz  [total_steps]
   double *grad_w;              // [n_tracks]
 };
@@ -143,6 +148,25 @@ __global__ void adj_prep_kernel(AdjParams a) {
     o[2] = make_float4((float)n1, (float)cT, (float)(cT * cPh), (float)(cT * sPh));
     o[3] = make_float4((float)(-sT), (float)(-sPh), (float)cPh, 0.f);
   }
+  if (p.fast.M != 0u) {
+    // behind it, per theta: (1 - cos hi, lo, sin hi, lo) (1 - cos, sin, cos, 0);
+    // per omega band: its centre frequency / 2 pi as a double-float
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nT; i += stride) {
+      const double sT = p.sin_theta[i], cT = p.cos_theta[i];
+      const df c = df_from_double(1.0 - cT), s = df_from_double(sT);
+      float4 *o = a.dirtab + 4 * n_dirs + 2 * i;
+      o[0] = make_float4(c.hi, c.lo, s.hi, s.lo);
+      o[1] = make_float4((float)(1.0 - cT), (float)sT, (float)cT, 0.f);
+    }
+    const double w0 = p.omega[0];
+    const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < p.fast.n_bands;
+         b += stride) {
+      const uint32_t j0 = (uint32_t)b * p.fast.nb, n = min(p.fast.nb, p.n_omega - j0);
+      const df c = df_from_double((w0 + (double)(j0 + n / 2) * dw) * 0.15915494309189533577);
+      a.bandtab[b] = make_float4(c.hi, c.lo, 0.f, 0.f);
+    }
+  }
 }
 
 
@@ -208,10 +232,13 @@ __global__ void adj_final_kernel(AdjParams a) {
     const int64_t s = g - p.offsets[t];
     const int64_t n_body = (int64_t)track_body(p, t);
     double cur[kAG] = {0}, prev[kAG] = {0};
-    if (s < n_body)
-      for (int c = 0; c < kAG; ++c) cur[c] = a.gstep[g * kAG + c];
-    if (s >= 1 && s - 1 < n_body)
-      for (int c = 3; c < kAG; ++c) prev[c] = a.gstep[(g - 1) * kAG + c];
+    for (uint32_t k = 0; k < a.n_split; ++k) {
+      const double *gs = a.gstep + (int64_t)k * p.total_steps * kAG;
+      if (s < n_body)
+        for (int c = 0; c < kAG; ++c) cur[c] += gs[g * kAG + c];
+      if (s >= 1 && s - 1 < n_body)
+        for (int c = 3; c < kAG; ++c) prev[c] += gs[(g - 1) * kAG + c];
+    }
     a.grad[0][g] = cur[0];
     a.grad[1][g] = cur[1];
     a.grad[2][g] = cur[2];
@@ -276,6 +303,7 @@ __device__ __forceinline__ df record_tau(const float4 *r, const float4 &d0, cons
 template <int W>
 __global__ void __launch_bounds__(W * 32, 2) adj_far_kernel(AdjParams a) {
   const FarMixedParams &p = a.f;
+  if (by_transform(p)) return;  // adj_interp_kernel's
   extern __shared__ __align__(128) unsigned char smem_raw[];
   AdjSmem &sm = *reinterpret_cast<AdjSmem *>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,11 +563,355 @@ __global__ void __launch_bounds__(W * 32, 2) adj_far_kernel(AdjParams a) {
   }
 }
 
+// ------------------------------------------------------------------------
+// Even omega axes: the sums over omega by transforms (the transpose of the
+// forward's, sr_fast_sum.cuh).  For a (track, direction) the sums
+//   H_c(tau) = sum_j conj(U_cj) exp(i omega_j tau),  K_c the same with omega_j U
+// are band-limited functions of tau: one FFT each of conj(U) divided by the
+// spreading kernel's transform gives cells on the circle of d_omega tau, and
+// every step takes 8 of them with the kernel's weights, whatever the number of
+// frequencies.  E_c = Re H_c, F_c = Im K_c.
+//
+// adj_fields_kernel: a warp per (track, snapshot segment, direction, band)
+// writes the cells of the four fields, [cell][H_th, H_ph, K_th, K_ph].
+// adj_interp_kernel: as below a CTA owns 256 steps of a track, a lane one step,
+// and loops over its directions; the records are turned into the plane of phi
+// once per phi.  Bound by the 16 cell loads of a (direction, step), 64 cycles
+// per warp and SM, and about as many for the arithmetic.
+// ------------------------------------------------------------------------
+
+// U of one point: summed over the snapshots k0..k1 that the steps enter.
+__device__ __forceinline__ float4 point_u(const AdjParams &a, uint32_t t, uint32_t k0, uint32_t k1,
+                                          uint64_t P, uint64_t gi, float wt, float swt) {
+  float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t k = k0; k <= k1; ++k) {
+    const float4 C = a.gcst[(uint64_t)k * P + gi];
+    if (a.linear) {
+      u.x += swt * C.x; u.y += swt * C.y;
+      u.z += swt * C.z; u.w += swt * C.w;
+    } else {
+      const float4 A = a.save_A[((uint64_t)t * a.f.n_snaps + k) * P + gi];
+      u.x += wt * (C.x * A.x + C.y * A.z);
+      u.y += wt * (C.x * A.y + C.y * A.w);
+      u.z += wt * (C.y * A.x + C.z * A.z);
+      u.w += wt * (C.y * A.y + C.z * A.w);
+    }
+  }
+  return u;
+}
+
+template <int R1>
+__global__ void __launch_bounds__(kFastWarps * 32, 3) adj_fields_kernel(
+    const __grid_constant__ AdjParams a) {
+  const FarMixedParams &p = a.f;
+  if (!by_transform(p)) return;
+  constexpr int NF = 32 / R1, M = 32 * R1;
+  constexpr int DP = NF > 4 ? NF / 4 : 1;     // directions per pass
+  constexpr int NPASS = 4 * DP / NF;
+  __shared__ float2 tr_all[kFastWarps][32 * 33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2 *tr = tr_all[warp];
+  const FastParams &f = p.fast;
+  const uint32_t n_dirs = p.n_theta * p.n_phi;
+  const uint64_t P = (uint64_t)p.n_omega * n_dirs;
+  const uint32_t dgroups = (n_dirs + DP - 1) / DP;
+  uint64_t task = (uint64_t)blockIdx.x * kFastWarps + warp;
+  const uint32_t band = (uint32_t)(task % f.n_bands);
+  task /= f.n_bands;
+  const uint32_t d0 = (uint32_t)(task % dgroups) * DP;
+  task /= dgroups;
+  const uint32_t k0 = (uint32_t)(task % p.n_snaps), t = a.t_lo + (uint32_t)(task / p.n_snaps);
+  if (t >= a.t_hi) return;
+  const uint32_t k1 = last_fired(p, t);
+  if (k1 == 0xffffffffu || k0 > k1) return;
+  const uint32_t j0 = band * f.nb;
+  const int nb = (int)min(f.nb, p.n_omega - j0);
+  const float wt = (float)p.weight[t], swt = (float)sqrt(p.weight[t]);
+#pragma unroll 1
+  for (int ps = 0; ps < NPASS; ++ps) {
+    float2 x[NF][R1], y[32];
+#pragma unroll
+    for (int dd = 0; dd < DP; ++dd) {
+      const uint32_t d = min(d0 + dd, n_dirs - 1);
+#pragma unroll
+      for (int i = 0; i < R1; ++i) {
+        const int n = 32 * i + lane;                        // frequency index mod M
+        const int j = (n < M / 2 ? n : n - M) + nb / 2;
+        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+        float dv = 0.f, w = 0.f;
+        if (j >= 0 && j < nb) {
+          u = point_u(a, t, k0, k1, P, (uint64_t)d * p.n_omega + j0 + j, wt, swt);
+          dv = (float)f.deconv[j - nb / 2 + kFastMaxBand / 2];
+          w = a.wtab[j0 + j].z;
+        }
+        const float2 th = make_float2(u.x * dv, -u.y * dv), ph = make_float2(u.z * dv, -u.w * dv);
+        auto field = [&](int q) {
+          const float2 b = (q & 1) ? ph : th;
+          return (q & 2) ? make_float2(b.x * w, b.y * w) : b;
+        };
+        if constexpr (NF >= 4) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[4 * dd + q][i] = field(q);
+        } else {
+#pragma unroll
+          for (int q = 0; q < NF; ++q) x[q][i] = field(ps * NF + q);
+        }
+      }
+    }
+    fft_fields<R1, NF>(x, y, tr, f.twiddle, lane);
+    const int q = lane / R1, al = lane % R1;
+    const int fq = ps * NF + q;                             // field of the pass's directions
+    const uint32_t d = d0 + fq / 4;
+    if (d < n_dirs) {
+      float2 *o = a.fields +
+                  ((((uint64_t)(t - a.t_lo) * p.n_snaps + k0) * n_dirs + d) * f.n_bands + band) *
+                      (4ull * M) + (fq & 3);
+#pragma unroll
+      for (int b = 0; b < 32; ++b) o[4 * (al + R1 * b)] = y[bitrev<32>(b)];
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
+    const __grid_constant__ AdjParams a) {
+  const FarMixedParams &p = a.f;
+  if (!by_transform(p)) return;
+  const FastParams &f = p.fast;
+  const int lane = threadIdx.x & 31;
+  const uint32_t nT = p.n_theta, n_dirs = nT * p.n_phi;
+  const uint64_t P = (uint64_t)p.n_omega * n_dirs;
+  const AdjGlobals G = *a.glob;
+  const int M = (int)f.M;
+  const float Mf = (float)M;
+  const double inv2pi = 0.15915494309189533577;
+  const double w0 = p.omega[0];
+  const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
+  const df f_d = df_from_double(dw * inv2pi);
+  const int64_t i_lo = a.item_off[a.t_lo], i_hi = a.item_off[a.t_hi];
+  const int64_t n_items = (i_hi - i_lo) * a.n_split;
+
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int64_t it = i_lo + item / a.n_split;
+    const uint32_t split = (uint32_t)(item % a.n_split);
+    const uint32_t dA = (uint32_t)((uint64_t)n_dirs * split / a.n_split);
+    const uint32_t dB = (uint32_t)((uint64_t)n_dirs * (split + 1) / a.n_split);
+    uint32_t lo = a.t_lo, hi = a.t_hi;  // last track with item_off[t] <= it
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (a.item_off[mid] <= it) lo = mid; else hi = mid;
+    }
+    const uint32_t t = lo;
+    const int64_t base = p.offsets[t];
+    SnapSegment seg{0, 0, 0, 0};
+    track_segments(p, t, (uint32_t)kASteps, (uint32_t)(it - a.item_off[t]), &seg);
+    const uint32_t s = seg.r0 + threadIdx.x;
+    const bool valid = s < seg.r1;
+    if (!__any_sync(0xffffffffu, valid)) continue;  // whole warps
+    const uint32_t sc = valid ? s : seg.r1 - 1;
+    const uint32_t it_start = p.it_start[t];
+    const float wt = (float)p.weight[t], swt = (float)sqrt(p.weight[t]);
+    const float4 *rp = p.records + (base + sc) * kRecF4;
+    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1), r2 = __ldg(rp + 2), r3 = __ldg(rp + 3);
+    // differences to the step before, for the quick test of the mask (the
+    // track's first step compares its whole phase with zero)
+    float dq = r0.x + r0.y, dz = r1.z + r1.w, dx = r0.z + r0.w, dy = r1.x + r1.y;
+    if (sc > 0) {
+      const float4 e0 = __ldg(rp - kRecF4), e1 = __ldg(rp - kRecF4 + 1);
+      dq = (r0.x - e0.x) + (r0.y - e0.y);
+      dx = (r0.z - e0.z) + (r0.w - e0.w);
+      dy = (r1.x - e1.x) + (r1.y - e1.y);
+      dz = (r1.z - e1.z) + (r1.w - e1.w);
+    }
+    double gD[kAG];
+#pragma unroll
+    for (int c = 0; c < kAG; ++c) gD[c] = 0.0;
+    float gF[kAG];   // x, bbar, a; within a phi: rho, phi, z of each
+#pragma unroll
+    for (int c = 0; c < kAG; ++c) gF[c] = 0.f;
+    const float2 *fld = a.fields +
+                        (((uint64_t)(t - a.t_lo) * p.n_snaps + seg.k0) * n_dirs) * f.n_bands *
+                            (4ull * M);
+    uint32_t d = dA;
+    while (d < dB) {
+      const uint32_t iP = d / nT, dE = min(dB, (iP + 1) * nT);
+      // the record in the plane of phi
+      const float4 ph = phi_pairs(p, iP);
+      const df rho = df_add(df_mul(df{ph.x, ph.y}, df{r0.z, r0.w}),
+                            df_mul(df{ph.z, ph.w}, df{r1.x, r1.y}));
+      const float b_r = ph.x * r2.x + ph.z * r2.y, b_p = ph.x * r2.y - ph.z * r2.x;
+      const float a_r = ph.x * r3.x + ph.z * r3.y, a_p = ph.x * r3.y - ph.z * r3.x;
+      const float drho = ph.x * dx + ph.z * dy;
+      float g_xr = 0.f, g_xz = 0.f, g_br = 0.f, g_bp = 0.f, g_bz = 0.f, g_ar = 0.f, g_ap = 0.f,
+            g_az = 0.f;
+#pragma unroll 1
+      for (; d < dE; ++d) {
+        // 1 - cos, sin, cos of theta: (dc hi, lo, sin hi, lo), (dc, sin, cos)
+        const float4 c0 = __ldg(a.dirtab + 4 * (uint64_t)nT * p.n_phi + 2 * (d - iP * nT));
+        const float4 c1v = __ldg(a.dirtab + 4 * (uint64_t)nT * p.n_phi + 2 * (d - iP * nT) + 1);
+        const df p1 = df_mul_raw(df{c0.x, c0.y}, df{r1.z, r1.w});
+        const df p2 = df_mul_raw(df{c0.z, c0.w}, rho);
+        const df s1 = two_sum(r0.x, p1.hi);
+        const df s2 = two_sum(s1.hi, -p2.hi);
+        const df tau = fast_two_sum(s2.hi, ((r0.y + p1.lo) - p2.lo) + (s1.lo + s2.lo));
+        // mask: certain where the FP32 difference leaves a 1e-3 margin, else from
+        // the double-float tau of both steps
+        int mode = valid ? 0 : 1;  // 0: every frequency enters, 1: none, 2: some
+        float et = 0.f, ep = 0.f, ft = 0.f, fp = 0.f;
+        const float quick = fabsf(dq + c1v.x * dz - c1v.y * drho);
+        if (__any_sync(0xffffffffu, valid && !(G.wabs_max * quick < 0.999f * kPiLo))) {
+          float dt0 = tau.hi + tau.lo;
+          if (sc > 0) {
+            const float4 e0 = __ldg(rp - kRecF4), e1 = __ldg(rp - kRecF4 + 1);
+            const df rb = df_add(df_mul(df{ph.x, ph.y}, df{e0.z, e0.w}),
+                                 df_mul(df{ph.z, ph.w}, df{e1.x, e1.y}));
+            const df q1 = df_mul_raw(df{c0.x, c0.y}, df{e1.z, e1.w});
+            const df q2 = df_mul_raw(df{c0.z, c0.w}, rb);
+            const df v1 = two_sum(e0.x, q1.hi);
+            const df v2 = two_sum(v1.hi, -q2.hi);
+            const df tb = fast_two_sum(v2.hi, ((e0.y + q1.lo) - q2.lo) + (v1.lo + v2.lo));
+            dt0 = (tau.hi - tb.hi) + (tau.lo - tb.lo);
+          }
+          const float adt = fabsf(dt0);
+          if (valid)
+            mode = G.wabs_max * adt < kPiLo ? 0 : (G.wabs_min * adt > kPiHi ? 1 : 2);
+          // cut steps, one after the other: the warp sums the included
+          // frequencies term by term
+          for (uint32_t cut = __ballot_sync(0xffffffffu, mode == 2); cut; cut &= cut - 1) {
+            const int b = __ffs(cut) - 1;
+            uint32_t r = 0;
+            if (lane == b)
+              r = cut_interval<false>(p, 0, (int)p.n_omega, G.w0f, G.dwf, d, base, s, it_start, adt);
+            r = __shfl_sync(0xffffffffu, r, b);
+            const float th = __shfl_sync(0xffffffffu, tau.hi, b);
+            const float tl = __shfl_sync(0xffffffffu, tau.lo, b);
+            const int jf = (int)(r & 0xffffu), jl = (int)(r >> 16);
+            float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+            for (int j = jf + lane; j <= jl; j += 32) {
+              const float4 u = point_u(a, t, seg.k0, seg.k1, P, (uint64_t)d * p.n_omega + j, wt, swt);
+              const float4 w = a.wtab[j];
+              float zs, zc;
+              phasor_rev(w.x, w.y, th, tl, zs, zc);
+              v0 += u.x * zc + u.y * zs;
+              v1 += u.z * zc + u.w * zs;
+              v2 += w.z * (u.x * zs - u.y * zc);
+              v3 += w.z * (u.z * zs - u.w * zc);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+              v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+              v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+              v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+              v3 += __shfl_xor_sync(0xffffffffu, v3, o);
+            }
+            if (lane == b) { et = v0; ep = v1; ft = v2; fp = v3; }
+          }
+        }
+        if (mode == 0) {
+          const float pr = f_d.hi * tau.hi;
+          float e = __fmaf_rn(f_d.hi, tau.hi, -pr);
+          e = __fmaf_rn(f_d.hi, tau.lo, e);
+          e = __fmaf_rn(f_d.lo, tau.hi, e);
+          const float uh = (pr - rintf(pr)) * Mf, ul = e * Mf;
+          const float rm = rintf((uh - 0.5f) + ul);
+          float wk[kTaps];
+          kb_taps(((uh - rm) - 0.5f) + ul, wk);
+          const int m = (int)rm - 3;
+          for (uint32_t band = 0; band < f.n_bands; ++band) {
+            const float4 *cell = reinterpret_cast<const float4 *>(
+                fld + ((uint64_t)d * f.n_bands + band) * (4ull * M));
+            float2 ht = make_float2(0.f, 0.f), hp = ht, kt = ht, kp = ht;
+#pragma unroll
+            for (int l = 0; l < kTaps; ++l) {
+              const float4 *q = cell + 2 * ((m + l) & (M - 1));
+              const float4 h = __ldg(q), k = __ldg(q + 1);
+              const float2 ww = make_float2(wk[l], wk[l]);
+              ht = __ffma2_rn(ww, make_float2(h.x, h.y), ht);
+              hp = __ffma2_rn(ww, make_float2(h.z, h.w), hp);
+              kt = __ffma2_rn(ww, make_float2(k.x, k.y), kt);
+              kp = __ffma2_rn(ww, make_float2(k.z, k.w), kp);
+            }
+            const float4 fc = __ldg(a.bandtab + band);  // its centre frequency / 2 pi
+            float zs, zc;
+            phasor_exact(fc.x, fc.y, tau.hi, tau.lo, zs, zc);
+            et += ht.x * zc - ht.y * zs;
+            ep += hp.x * zc - hp.y * zs;
+            ft += kt.x * zs + kt.y * zc;
+            fp += kp.x * zs + kp.y * zc;
+          }
+        }
+        if (mode != 1) {  // the chain rule, in the plane of phi
+          const float st = c1v.y, ct = c1v.z;
+          const float D = r2.w + c1v.x * r2.z - st * b_r;
+          const float c2 = rcp_newton(D);
+          const float an = st * a_r + ct * r3.z;
+          const float c22 = c2 * c2;
+          const float c1 = an * c22;
+          const float tb = ct * b_r - st * r2.z, ta = ct * a_r - st * r3.z;
+          const float amp_t = -(c1 * tb + c2 * ta), amp_p = -(c1 * b_p + c2 * a_p);
+          // x: n (amp_t F_t + amp_p F_p)
+          const float fx = amp_t * ft + amp_p * fp;
+          // bbar: -(2 an c2^3 e.b + c2^2 e.a) n E - c1 e E;  a: -(c2^2 e.b) n E - c2 e E
+          const float m3 = 2.f * c1 * c2;
+          const float kb = -(et * (m3 * tb + c22 * ta) + ep * (m3 * b_p + c22 * a_p));
+          const float ka = -c22 * (et * tb + ep * b_p);
+          const float er = et * ct, ez = -et * st;  // theta-hat = (cos, -sin) in (rho, z)
+          g_xr += st * fx;
+          g_xz += ct * fx;
+          g_br += kb * st - c1 * er;
+          g_bp -= c1 * ep;
+          g_bz += kb * ct - c1 * ez;
+          g_ar += ka * st - c2 * er;
+          g_ap -= c2 * ep;
+          g_az += ka * ct - c2 * ez;
+        }
+      }
+      gF[0] += ph.x * g_xr;
+      gF[1] += ph.z * g_xr;
+      gF[2] += g_xz;
+      gF[3] += ph.x * g_br - ph.z * g_bp;
+      gF[4] += ph.z * g_br + ph.x * g_bp;
+      gF[5] += g_bz;
+      gF[6] += ph.x * g_ar - ph.z * g_ap;
+      gF[7] += ph.z * g_ar + ph.x * g_ap;
+      gF[8] += g_az;
+      // FP32 over at least 32 directions, then FP64
+      if (nT >= 32 || d == dB || (iP & 7u) == 7u) {
+#pragma unroll
+        for (int c = 0; c < kAG; ++c) {
+          gD[c] += (double)gF[c];
+          gF[c] = 0.f;
+        }
+      }
+    }
+    if (valid) {
+#pragma unroll
+      for (int c = 0; c < kAG; ++c)
+        a.gstep[((uint64_t)split * p.total_steps + base + s) * kAG + c] = gD[c];
+    }
+  }
+}
+
 size_t adj_smem_bytes() { return sizeof(AdjSmem); }
 
+void launch_adj_fields(const AdjParams &a, uint64_t n_dirs, cudaStream_t s) {
+  const uint64_t dp = std::max(1u, 256u / a.f.fast.M);
+  const uint64_t warps = (uint64_t)(a.t_hi - a.t_lo) * a.f.n_snaps * ((n_dirs + dp - 1) / dp) *
+                         a.f.fast.n_bands;
+  const unsigned blocks = (unsigned)((warps + kFastWarps - 1) / kFastWarps);
+  switch (a.f.fast.M) {
+    case 128: adj_fields_kernel<4><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    case 256: adj_fields_kernel<8><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    case 512: adj_fields_kernel<16><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    default: adj_fields_kernel<32><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+  }
+}
+
 struct AdjLayout {
-  size_t records, gcst, wtab, dirtab, glob, item_off, gstep, wpart, total;
+  size_t records, gcst, wtab, dirtab, glob, item_off, gstep, wpart, tables, bandtab, fields, total;
   uint32_t w_chunks;
+  uint32_t n_split, batch;  // runs of directions; tracks per batch of fields (0: term by term)
+  uint32_t n_bands, nb, M;
 };
 
 AdjLayout adj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t n_dirs,
@@ -551,11 +923,35 @@ AdjLayout adj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t
   l.gcst = l.records + up((size_t)total_steps * kRecBytes);
   l.wtab = l.gcst + up((size_t)P * 16 * (n_snaps ? n_snaps : 1));
   l.dirtab = l.wtab + up((size_t)n_omega * 16);
-  l.glob = l.dirtab + up((size_t)n_dirs * 64);
+  l.glob = l.dirtab + up((size_t)n_dirs * 96);
+  // The transforms' cells: 32 bytes each for every (track, snapshot, direction),
+  // of as many tracks at a time as 2 GiB hold (at least what fills the SMs).
+  l.n_split = 1;
+  l.batch = 0;
+  l.n_bands = l.nb = l.M = 0;
+  if (n_omega >= 8 && n_omega < 65536u && n_tracks > 0 && n_snaps > 0 && total_steps > 0) {
+    l.n_bands = (n_omega + kFastMaxBand - 1) / kFastMaxBand;
+    l.nb = (n_omega + l.n_bands - 1) / l.n_bands;
+    l.M = fast_cells(l.nb);
+    const uint64_t per = (uint64_t)n_snaps * n_dirs * l.n_bands * l.M * 32;
+    const uint64_t fit = (2ull << 30) / per;
+    const uint64_t slots = 2ull * device_sm_count();
+    const uint64_t mean_items = (uint64_t)total_steps / n_tracks / kASteps + 1;
+    if (fit >= 1) {
+      l.batch = (uint32_t)std::min<uint64_t>(n_tracks, fit);
+      // few items: runs of at least 16 directions apart, so that the SMs fill
+      const uint64_t items = l.batch * mean_items;
+      l.n_split = (uint32_t)std::max<uint64_t>(
+          1, std::min<uint64_t>({(2 * slots + items - 1) / items, n_dirs / 16, 16}));
+    }
+  }
   l.item_off = l.glob + 256;
   l.gstep = l.item_off + up(((size_t)n_tracks + 1) * 8);
-  l.wpart = l.gstep + up((size_t)total_steps * kAG * 8);
-  l.total = l.wpart + up((size_t)n_tracks * l.w_chunks * 8);
+  l.wpart = l.gstep + up((size_t)total_steps * kAG * 8 * l.n_split);
+  l.tables = l.wpart + up((size_t)n_tracks * l.w_chunks * 8);
+  l.bandtab = l.tables + up(kFastTables);
+  l.fields = l.bandtab + up((size_t)l.n_bands * 16);
+  l.total = l.fields + (size_t)l.batch * n_snaps * n_dirs * l.n_bands * l.M * 32;
   return l;
 }
 
@@ -684,15 +1080,19 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   a.gstep = (double *)(w + lay.gstep);
   for (int i = 0; i < 6; ++i) a.grad[i] = grad_track[i];
   a.grad_w = grad_weight;
+  a.n_split = lay.n_split;
+  a.bandtab = (float4 *)(w + lay.bandtab);
+  a.fields = (float2 *)(w + lay.fields);
+  if (lay.batch) fast_tables_bind(a.f, lay.n_bands, lay.nb, lay.M, w + lay.tables, w);
 
   e = cudaMemsetAsync(w, 0, 256, s);
   if (e != cudaSuccess) return cuda_fail(e, "status reset");
   // steps that enter no snapshot (after the last one written) are not visited
-  e = cudaMemsetAsync(a.gstep, 0, (size_t)t->total_steps * kAG * 8, s);
+  e = cudaMemsetAsync(a.gstep, 0, (size_t)t->total_steps * kAG * 8 * lay.n_split, s);
   if (e != cudaSuccess) return cuda_fail(e, "gradient reset");
   const int n_sm = device_sm_count();
   const int64_t step_blocks = std::max<int64_t>(
-      1, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
+      16, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
   if (t->total_steps > 0) launch_far_prepass(a.f, (int)step_blocks, s);
   adj_globals_kernel<<<1, 256, 0, s>>>(a.f, a.wtab, a.glob);
   {
@@ -711,14 +1111,21 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   rc = cuda_fail(cudaGetLastError(), "adjoint prep launch");
   if (rc) return rc;
   const size_t smem = adj_smem_bytes();
-  e = cudaFuncSetAttribute(adj_far_kernel<kAW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
+  e = allow_smem((const void *)adj_far_kernel<kAW>, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "adjoint smem attribute");
   // upper bound of the work items (sum over tracks of ceil(n_body / 256))
-  const int64_t items_max = t->total_steps / kASteps + (int64_t)t->n_tracks;
+  const int64_t items_max = t->total_steps / kASteps + (int64_t)t->n_tracks * t->n_snaps;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items_max, 2 * (int64_t)n_sm));
   void *tok = nullptr;
   timing_record(s, true, &tok);
+  for (uint32_t lo = 0; lay.batch && lo < t->n_tracks; lo += lay.batch) {
+    a.t_lo = lo;
+    a.t_hi = std::min(t->n_tracks, lo + lay.batch);
+    launch_adj_fields(a, n_dirs, s);
+    const int64_t most = items_max * lay.n_split;
+    adj_interp_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm)),
+                        kASteps, 0, s>>>(a);
+  }
   adj_far_kernel<kAW><<<grid, kAW * 32, smem, s>>>(a);
   timing_record(s, false, &tok);
   rc = cuda_fail(cudaGetLastError(), "adjoint kernel launch");

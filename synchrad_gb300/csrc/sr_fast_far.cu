@@ -8,7 +8,6 @@ namespace sr {
 
 namespace {
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
-constexpr size_t kTables = (kFastMaxBand + 2) * 8 + 1024 * 16;
 }  // namespace
 
 FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
@@ -32,8 +31,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
   const int np = near ? 3 : 1;
   l.n_bands = (c.n_omega + kFastMaxBand - 1) / kFastMaxBand;
   l.nb = (c.n_omega + l.n_bands - 1) / l.n_bands;
-  l.M = 128;
-  while (l.M < 2 * l.nb) l.M *= 2;
+  l.M = fast_cells(l.nb);
   l.n_dwb = (c.n_dirs + 31) / 32 * l.n_bands;
   l.slice_bytes = up256((size_t)32 * (np * (size_t)(l.M + 2 * l.nb) * 16 +
                                       kFastList * (16 + 8 * (size_t)np)));
@@ -99,7 +97,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
 
 size_t fast_workspace(const FastLayout &l) {
   if (!l.on) return 0;
-  return up256(kTables) + up256((size_t)l.slices * 4) + (size_t)l.slices * l.slice_bytes;
+  return up256(kFastTables) + up256((size_t)l.slices * 4) + (size_t)l.slices * l.slice_bytes;
 }
 
 void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
@@ -109,16 +107,12 @@ void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char 
   f.M = 0;
   if (!l.on) return;
   f.queue = (unsigned int *)(status + 192);
-  f.deconv = (double *)base;
-  f.twiddle = (float4 *)(base + (kFastMaxBand + 2) * 8);
-  base += up256(kTables);
+  fast_tables_bind(p, l.n_bands, l.nb, l.M, base, status);
+  base += up256(kFastTables);
   f.dirty = (unsigned int *)base;
   base += up256((size_t)l.slices * 4);
   f.scratch = base;
   f.slice_bytes = l.slice_bytes;
-  f.n_bands = l.n_bands;
-  f.nb = l.nb;
-  f.M = l.M;
   f.n_dwb = l.n_dwb;
   f.n_sub = l.n_sub;
   f.n_segs = l.n_segs;

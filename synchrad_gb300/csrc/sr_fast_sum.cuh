@@ -179,13 +179,12 @@ __device__ __forceinline__ constexpr int bitrev(int k) {
   return r;
 }
 
-// Second half of the transform of the fields in x: NF fields of M = 32 R1
-// cells (cell 32 i + lane in x[.][i]).  Writes the N band sums of field q to
-// dst[q][j], j = frequency index + N/2 (not yet divided by the kernel's
-// transform).
+// The M-point transforms (exp(+2 pi i m k / M)) of NF fields, element
+// 32 i + lane of field q in x[q][i]; element a + R1 b of field q comes out in
+// y[bitrev(b)] of lane q R1 + a.
 template <int R1, int NF>
-__device__ __forceinline__ void fft_band(float2 (&x)[NF][R1], float2 *tr, const float4 *tw,
-                                         int lane, int n, float2 *dst) {
+__device__ __forceinline__ void fft_fields(float2 (&x)[NF][R1], float2 (&y)[32], float2 *tr,
+                                           const float4 *tw, int lane) {
   static_assert(R1 * NF == 32, "one warp holds 1024 cells");
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
@@ -202,11 +201,19 @@ __device__ __forceinline__ void fft_band(float2 (&x)[NF][R1], float2 *tr, const 
     }
   }
   __syncwarp();
-  float2 y[32];
 #pragma unroll
   for (int l = 0; l < 32; ++l) y[l] = tr[lane * 33 + l];
   __syncwarp();
   fft_reg<32>(y);
+}
+
+// The N band sums of the fields in x (cells) to dst[q][j], j = frequency index
+// + N/2 (not yet divided by the kernel's transform).
+template <int R1, int NF>
+__device__ __forceinline__ void fft_band(float2 (&x)[NF][R1], float2 *tr, const float4 *tw,
+                                         int lane, int n, float2 *dst) {
+  float2 y[32];
+  fft_fields<R1, NF>(x, y, tr, tw, lane);
   const int q = lane / R1, a = lane % R1;
 #pragma unroll
   for (int b = 0; b < 32; ++b) {
@@ -1312,6 +1319,25 @@ uneven_axis_kernel(const __grid_constant__ FarMixedParams p) {
 }
 
 // ------------------------------------------------------------------ host side
+inline uint32_t fast_cells(uint32_t nb) {
+  uint32_t M = 128;
+  while (M < 2 * nb) M *= 2;
+  return M;
+}
+constexpr size_t kFastTables = (kFastMaxBand + 2) * 8 + 1024 * 16;
+
+// p.fast's tables (made by the record pass) at `tables`, the axis test in the
+// status block.
+inline void fast_tables_bind(FarMixedParams &p, uint32_t n_bands, uint32_t nb, uint32_t M,
+                             unsigned char *tables, unsigned char *status) {
+  p.fast.uneven = (unsigned int *)(status + 64);
+  p.fast.deconv = (double *)tables;
+  p.fast.twiddle = (float4 *)(tables + (kFastMaxBand + 2) * 8);
+  p.fast.n_bands = n_bands;
+  p.fast.nb = nb;
+  p.fast.M = M;
+}
+
 template <bool NEAR, int R1>
 int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
   constexpr int smem = (int)sizeof(FastSmem) * kFastWarps;
