@@ -1,8 +1,11 @@
 // Pieces shared by the far- and near-field adjoint kernels.
 #pragma once
 
+#include <algorithm>
+
 #include "sr_common.cuh"
 #include "sr_internal.h"
+#include "sr_fast_sum.cuh"
 #include "sr_mixed_common.cuh"
 
 namespace sr {
@@ -17,7 +20,8 @@ struct AdjGlobals {
 };
 
 // Omega table, axis uniformity and |omega| range (one block).
-__global__ void adj_globals_kernel(FarMixedParams p, float4 *wtab, AdjGlobals *glob) {
+__device__ __forceinline__ void adj_globals(const FarMixedParams &p, float4 *wtab,
+                                            AdjGlobals *glob) {
   const uint32_t nO = p.n_omega;
   const double w0 = p.omega[0];
   const double dw = (nO > 1) ? (p.omega[nO - 1] - w0) / (double)(nO - 1) : 0.0;
@@ -32,7 +36,7 @@ __global__ void adj_globals_kernel(FarMixedParams p, float4 *wtab, AdjGlobals *g
     amin = fminf(amin, aw);
     amax = fmaxf(amax, aw);
   }
-  __shared__ float smin[256], smax[256];
+  __shared__ float smin[1024], smax[1024];
   smin[threadIdx.x] = amin;
   smax[threadIdx.x] = amax;
   const int all_uni = __syncthreads_and(uni ? 1 : 0);
@@ -118,7 +122,8 @@ __device__ __forceinline__ uint32_t track_segments(const FarMixedParams &p, uint
 // Work items per track (snapshot segments cut into runs of steps_per_item),
 // as an exclusive prefix (one block of 1024 threads, each scanning a
 // contiguous run of tracks).
-__global__ void adj_items_kernel(FarMixedParams p, int64_t *item_off, uint32_t steps_per_item) {
+__device__ __forceinline__ void adj_items(const FarMixedParams &p, int64_t *item_off,
+                                          uint32_t steps_per_item) {
   const uint32_t n = p.n_tracks;
   const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
   const uint32_t t0 = min(n, threadIdx.x * per), t1 = min(n, t0 + per);
@@ -141,10 +146,19 @@ __global__ void adj_items_kernel(FarMixedParams p, int64_t *item_off, uint32_t s
   if (threadIdx.x == blockDim.x - 1) item_off[n] = sums[blockDim.x - 1];
 }
 
+// The two one-block preparations in one launch (two blocks of 1024 threads).
+__global__ void adj_setup_kernel(FarMixedParams p, float4 *wtab, AdjGlobals *glob,
+                                 int64_t *item_off, uint32_t steps_per_item) {
+  if (blockIdx.x == 0)
+    adj_globals(p, wtab, glob);
+  else
+    adj_items(p, item_off, steps_per_item);
+}
+
 // Weight gradients are summed in two fixed-order stages: block (t, b) sums
 // chunk b of track t's points into wpart[t][b] by a fixed tree, then one
-// thread per track adds its chunks in order (sr_far_adjoint.cu,
-// sr_near_adjoint.cu).
+// thread of the last launch per track adds its chunks in order
+// (sr_far_adjoint.cu, sr_near_adjoint.cu).
 constexpr int kWeightThreads = 256;
 
 inline uint32_t adj_weight_chunks(uint64_t P, uint32_t n_tracks, int n_sm) {
@@ -153,6 +167,55 @@ inline uint32_t adj_weight_chunks(uint64_t P, uint32_t n_tracks, int n_sm) {
   if (c > cmax) c = cmax;
   if (c > 256) c = 256;
   return (uint32_t)(c < 1 ? 1 : c);
+}
+
+__device__ __forceinline__ void adj_weight_final(const FarMixedParams &p, const double *wpart,
+                                                 uint32_t n_chunks, int linear, double *grad_w) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < p.n_tracks;
+       t += gridDim.x * blockDim.x) {
+    double s = 0.0;
+    for (uint32_t b = 0; b < n_chunks; ++b) s += wpart[(uint64_t)t * n_chunks + b];
+    const double w = p.weight[t];
+    grad_w[t] = linear ? (w > 0.0 ? s / (2.0 * sqrt(w)) : 0.0) : 0.5 * s;
+  }
+}
+
+// The transforms' cells (`cell` bytes each) of every (track, snapshot,
+// direction, omega band), of as many tracks at a time as 2 GiB hold; none
+// (batch 0) where one track's do not fit or the axis is too short to gain.
+struct AdjFields {
+  uint32_t n_split;  // runs of directions whose gradients are summed apart
+  uint32_t batch;    // tracks at a time
+  uint32_t n_bands, nb, M;
+  size_t bytes;
+};
+
+inline AdjFields adj_fields_layout(int64_t total_steps, uint32_t n_omega, uint64_t n_dirs,
+                                   uint32_t n_tracks, uint32_t n_snaps, size_t cell,
+                                   int steps_per_item) {
+  AdjFields l{1, 0, 0, 0, 0, 0};
+  if (n_omega < 8 || n_omega >= 65536u || n_tracks == 0 || n_snaps == 0 || total_steps <= 0)
+    return l;
+  l.n_bands = (n_omega + kFastMaxBand - 1) / kFastMaxBand;
+  l.nb = (n_omega + l.n_bands - 1) / l.n_bands;
+  l.M = fast_cells(l.nb);
+  // A snapshot's transforms cost as much as walking the frequencies of about
+  // 60 M / nb steps; with several snapshots the steps between two must be more
+  // (400 frequencies, 45 steps a snapshot: far 11.3 / 9.3 ms, near 30.6 / 13.9 ms
+  // transforms / walking; 64 frequencies, 150 steps: 0.49 / 1.13, 0.56 / 1.81).
+  if (n_snaps > 1 && (uint64_t)total_steps * n_omega <
+                         60ull * l.M * l.n_bands * n_snaps * n_tracks)
+    return l;
+  const uint64_t per = (uint64_t)n_snaps * n_dirs * l.n_bands * (l.M + kTaps) * cell;
+  l.batch = (uint32_t)std::min<uint64_t>(n_tracks, (2ull << 30) / per);
+  if (l.batch == 0) return l;
+  l.bytes = (size_t)(l.batch * per);
+  // few items: runs of at least 16 directions apart, so that the SMs fill
+  const uint64_t slots = 2ull * device_sm_count();
+  const uint64_t items = l.batch * ((uint64_t)total_steps / n_tracks / steps_per_item + 1);
+  l.n_split = (uint32_t)std::max<uint64_t>(
+      1, std::min<uint64_t>({(2 * slots + items - 1) / items, n_dirs / 16, 16}));
+  return l;
 }
 
 }  // namespace

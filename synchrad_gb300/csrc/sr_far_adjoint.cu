@@ -64,6 +64,8 @@ struct AdjParams {
   uint32_t t_lo, t_hi;         // the batch
   double *grad[6];             // x, y, z, ux, uy, uz  [total_steps]
   double *grad_w;              // [n_tracks]
+  double *wpart;               // [n_tracks][w_chunks] partial weight gradients
+  uint32_t w_chunks;
 };
 
 // Point sensitivity of the loss to (A_theta, A_phi) for output gradients g_k
@@ -204,15 +206,6 @@ __global__ void adj_weight_partial_far_kernel(AdjParams a, uint64_t P, uint32_t 
 
 // quadratic comps: dL/dw = (A^H M A) / 2 (M holds 2 dt^2); linear comps:
 // dL/dw = Re(conj(V) . A) / (2 sqrt(w)).
-__global__ void adj_weight_final_far_kernel(const double *wpart, uint32_t n_tracks,
-                                            uint32_t n_chunks, int linear, const double *weight,
-                                            double *grad_w) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tracks) return;
-  double s = 0.0;
-  for (uint32_t b = 0; b < n_chunks; ++b) s += wpart[(uint64_t)t * n_chunks + b];
-  grad_w[t] = linear ? (weight[t] > 0.0 ? s / (2.0 * sqrt(weight[t])) : 0.0) : 0.5 * s;
-}
 
 // Per-step gradients: map dL/dbbar and dL/da of steps s-1 and s to dL/dbeta_s
 // and dL/du_s.
@@ -221,6 +214,7 @@ __global__ void adj_final_kernel(AdjParams a) {
   const FarMixedParams &p = a.f;
   const TT *UX = (const TT *)p.ux, *UY = (const TT *)p.uy, *UZ = (const TT *)p.uz;
   const double dtInv = 1.0 / p.dt;
+  adj_weight_final(p, a.wpart, a.w_chunks, a.linear, a.grad_w);
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < p.total_steps;
        g += (int64_t)gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = p.n_tracks;
@@ -573,7 +567,8 @@ __global__ void __launch_bounds__(W * 32, 2) adj_far_kernel(AdjParams a) {
 // frequencies.  E_c = Re H_c, F_c = Im K_c.
 //
 // adj_fields_kernel: a warp per (track, snapshot segment, direction, band)
-// writes the cells of the four fields, [cell][H_th, H_ph, K_th, K_ph].
+// writes the cells of the four fields, [cell][H_th, H_ph, K_th, K_ph], the
+// circle's first 8 cells again behind its last.
 // adj_interp_kernel: as below a CTA owns 256 steps of a track, a lane one step,
 // and loops over its directions; the records are turned into the plane of phi
 // once per phi.  Bound by the 16 cell loads of a (direction, step), 64 cycles
@@ -665,9 +660,13 @@ __global__ void __launch_bounds__(kFastWarps * 32, 3) adj_fields_kernel(
     if (d < n_dirs) {
       float2 *o = a.fields +
                   ((((uint64_t)(t - a.t_lo) * p.n_snaps + k0) * n_dirs + d) * f.n_bands + band) *
-                      (4ull * M) + (fq & 3);
+                      (4ull * (M + kTaps)) + (fq & 3);
 #pragma unroll
       for (int b = 0; b < 32; ++b) o[4 * (al + R1 * b)] = y[bitrev<32>(b)];
+      // the circle's first cells once more behind its last
+#pragma unroll
+      for (int b = 0; b * R1 < kTaps; ++b)
+        if (al + R1 * b < kTaps) o[4 * (M + al + R1 * b)] = y[bitrev<32>(b)];
     }
     __syncwarp();
   }
@@ -731,7 +730,7 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
     for (int c = 0; c < kAG; ++c) gF[c] = 0.f;
     const float2 *fld = a.fields +
                         (((uint64_t)(t - a.t_lo) * p.n_snaps + seg.k0) * n_dirs) * f.n_bands *
-                            (4ull * M);
+                            (4ull * (M + kTaps));
     uint32_t d = dA;
     while (d < dB) {
       const uint32_t iP = d / nT, dE = min(dB, (iP + 1) * nT);
@@ -775,36 +774,57 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
           const float adt = fabsf(dt0);
           if (valid)
             mode = G.wabs_max * adt < kPiLo ? 0 : (G.wabs_min * adt > kPiHi ? 1 : 2);
-          // cut steps, one after the other: the warp sums the included
-          // frequencies term by term
-          for (uint32_t cut = __ballot_sync(0xffffffffu, mode == 2); cut; cut &= cut - 1) {
-            const int b = __ffs(cut) - 1;
-            uint32_t r = 0;
-            if (lane == b)
-              r = cut_interval<false>(p, 0, (int)p.n_omega, G.w0f, G.dwf, d, base, s, it_start, adt);
-            r = __shfl_sync(0xffffffffu, r, b);
-            const float th = __shfl_sync(0xffffffffu, tau.hi, b);
-            const float tl = __shfl_sync(0xffffffffu, tau.lo, b);
-            const int jf = (int)(r & 0xffffu), jl = (int)(r >> 16);
-            float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-            for (int j = jf + lane; j <= jl; j += 32) {
-              const float4 u = point_u(a, t, seg.k0, seg.k1, P, (uint64_t)d * p.n_omega + j, wt, swt);
-              const float4 w = a.wtab[j];
-              float zs, zc;
-              phasor_rev(w.x, w.y, th, tl, zs, zc);
-              v0 += u.x * zc + u.y * zs;
-              v1 += u.z * zc + u.w * zs;
-              v2 += w.z * (u.x * zs - u.y * zc);
-              v3 += w.z * (u.z * zs - u.w * zc);
-            }
+          // cut steps: each lane finds its included frequencies, then the warp
+          // sums four steps' at a time term by term, lane + 32 k
+          const uint32_t mine =
+              mode == 2 ? cut_interval<false>(p, 0, (int)p.n_omega, G.w0f, G.dwf, d, base, s,
+                                              it_start, adt)
+                        : 1u;
+          for (uint32_t cut = __ballot_sync(0xffffffffu, mode == 2); cut;) {
+            float v[16];
+            uint32_t batch = 0u;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-              v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-              v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-              v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-              v3 += __shfl_xor_sync(0xffffffffu, v3, o);
+            for (int e = 0; e < 4; ++e) {
+              v[4 * e] = v[4 * e + 1] = v[4 * e + 2] = v[4 * e + 3] = 0.f;
+              if (cut) {
+                const int b = __ffs(cut) - 1;
+                cut &= cut - 1;
+                batch |= 1u << b;
+                const uint32_t r = __shfl_sync(0xffffffffu, mine, b);
+                const float th = __shfl_sync(0xffffffffu, tau.hi, b);
+                const float tl = __shfl_sync(0xffffffffu, tau.lo, b);
+                const int jl = (int)(r >> 16);
+                for (int j = (int)(r & 0xffffu) + lane; j <= jl; j += 32) {
+                  const float4 u =
+                      point_u(a, t, seg.k0, seg.k1, P, (uint64_t)d * p.n_omega + j, wt, swt);
+                  const float4 w = __ldg(a.wtab + j);
+                  float zs, zc;
+                  phasor_rev(w.x, w.y, th, tl, zs, zc);
+                  v[4 * e] += u.x * zc + u.y * zs;
+                  v[4 * e + 1] += u.z * zc + u.w * zs;
+                  v[4 * e + 2] += w.z * (u.x * zs - u.y * zc);
+                  v[4 * e + 3] += w.z * (u.z * zs - u.w * zc);
+                }
+              }
             }
-            if (lane == b) { et = v0; ep = v1; ft = v2; fp = v3; }
+            // lane i ends with the warp's sum of value i / 2
+#pragma unroll
+            for (int n = 8; n > 0; n >>= 1) {
+              const int o = 2 * n;
+              const bool up = (lane & o) != 0;
+#pragma unroll
+              for (int i = 0; i < n; ++i) {
+                const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+              }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            const int e = __popc(batch & ((1u << lane) - 1u)) & 3;
+            const float s0 = __shfl_sync(0xffffffffu, v[0], 8 * e);
+            const float s1 = __shfl_sync(0xffffffffu, v[0], 8 * e + 2);
+            const float s2 = __shfl_sync(0xffffffffu, v[0], 8 * e + 4);
+            const float s3 = __shfl_sync(0xffffffffu, v[0], 8 * e + 6);
+            if ((batch >> lane) & 1u) { et = s0; ep = s1; ft = s2; fp = s3; }
           }
         }
         if (mode == 0) {
@@ -816,15 +836,14 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
           const float rm = rintf((uh - 0.5f) + ul);
           float wk[kTaps];
           kb_taps(((uh - rm) - 0.5f) + ul, wk);
-          const int m = (int)rm - 3;
+          const int m = ((int)rm - 3) & (M - 1);
           for (uint32_t band = 0; band < f.n_bands; ++band) {
             const float4 *cell = reinterpret_cast<const float4 *>(
-                fld + ((uint64_t)d * f.n_bands + band) * (4ull * M));
+                fld + ((uint64_t)d * f.n_bands + band) * (4ull * (M + kTaps)) + 4 * m);
             float2 ht = make_float2(0.f, 0.f), hp = ht, kt = ht, kp = ht;
 #pragma unroll
             for (int l = 0; l < kTaps; ++l) {
-              const float4 *q = cell + 2 * ((m + l) & (M - 1));
-              const float4 h = __ldg(q), k = __ldg(q + 1);
+              const float4 h = __ldg(cell + 2 * l), k = __ldg(cell + 2 * l + 1);
               const float2 ww = make_float2(wk[l], wk[l]);
               ht = __ffma2_rn(ww, make_float2(h.x, h.y), ht);
               hp = __ffma2_rn(ww, make_float2(h.z, h.w), hp);
@@ -910,8 +929,7 @@ void launch_adj_fields(const AdjParams &a, uint64_t n_dirs, cudaStream_t s) {
 struct AdjLayout {
   size_t records, gcst, wtab, dirtab, glob, item_off, gstep, wpart, tables, bandtab, fields, total;
   uint32_t w_chunks;
-  uint32_t n_split, batch;  // runs of directions; tracks per batch of fields (0: term by term)
-  uint32_t n_bands, nb, M;
+  AdjFields fl;
 };
 
 AdjLayout adj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t n_dirs,
@@ -919,39 +937,19 @@ AdjLayout adj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   AdjLayout l;
   l.w_chunks = adj_weight_chunks(P, n_tracks, device_sm_count());
-  l.records = 256;
+  l.fl = adj_fields_layout(total_steps, n_omega, n_dirs, n_tracks, n_snaps, 32, kASteps);
+  l.gstep = 256;
+  l.records = l.gstep + up((size_t)total_steps * kAG * 8 * l.fl.n_split);
   l.gcst = l.records + up((size_t)total_steps * kRecBytes);
   l.wtab = l.gcst + up((size_t)P * 16 * (n_snaps ? n_snaps : 1));
   l.dirtab = l.wtab + up((size_t)n_omega * 16);
   l.glob = l.dirtab + up((size_t)n_dirs * 96);
-  // The transforms' cells: 32 bytes each for every (track, snapshot, direction),
-  // of as many tracks at a time as 2 GiB hold (at least what fills the SMs).
-  l.n_split = 1;
-  l.batch = 0;
-  l.n_bands = l.nb = l.M = 0;
-  if (n_omega >= 8 && n_omega < 65536u && n_tracks > 0 && n_snaps > 0 && total_steps > 0) {
-    l.n_bands = (n_omega + kFastMaxBand - 1) / kFastMaxBand;
-    l.nb = (n_omega + l.n_bands - 1) / l.n_bands;
-    l.M = fast_cells(l.nb);
-    const uint64_t per = (uint64_t)n_snaps * n_dirs * l.n_bands * l.M * 32;
-    const uint64_t fit = (2ull << 30) / per;
-    const uint64_t slots = 2ull * device_sm_count();
-    const uint64_t mean_items = (uint64_t)total_steps / n_tracks / kASteps + 1;
-    if (fit >= 1) {
-      l.batch = (uint32_t)std::min<uint64_t>(n_tracks, fit);
-      // few items: runs of at least 16 directions apart, so that the SMs fill
-      const uint64_t items = l.batch * mean_items;
-      l.n_split = (uint32_t)std::max<uint64_t>(
-          1, std::min<uint64_t>({(2 * slots + items - 1) / items, n_dirs / 16, 16}));
-    }
-  }
   l.item_off = l.glob + 256;
-  l.gstep = l.item_off + up(((size_t)n_tracks + 1) * 8);
-  l.wpart = l.gstep + up((size_t)total_steps * kAG * 8 * l.n_split);
+  l.wpart = l.item_off + up(((size_t)n_tracks + 1) * 8);
   l.tables = l.wpart + up((size_t)n_tracks * l.w_chunks * 8);
   l.bandtab = l.tables + up(kFastTables);
-  l.fields = l.bandtab + up((size_t)l.n_bands * 16);
-  l.total = l.fields + (size_t)l.batch * n_snaps * n_dirs * l.n_bands * l.M * 32;
+  l.fields = l.bandtab + up((size_t)l.fl.n_bands * 16);
+  l.total = l.fields + l.fl.bytes;
   return l;
 }
 
@@ -1080,34 +1078,29 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   a.gstep = (double *)(w + lay.gstep);
   for (int i = 0; i < 6; ++i) a.grad[i] = grad_track[i];
   a.grad_w = grad_weight;
-  a.n_split = lay.n_split;
+  a.n_split = lay.fl.n_split;
   a.bandtab = (float4 *)(w + lay.bandtab);
   a.fields = (float2 *)(w + lay.fields);
-  if (lay.batch) fast_tables_bind(a.f, lay.n_bands, lay.nb, lay.M, w + lay.tables, w);
+  if (lay.fl.batch) fast_tables_bind(a.f, lay.fl.n_bands, lay.fl.nb, lay.fl.M, w + lay.tables, w);
 
-  e = cudaMemsetAsync(w, 0, 256, s);
+  // the status block and, behind it, the per-step gradients: steps that enter
+  // no snapshot (after the last one written) are not visited
+  e = cudaMemsetAsync(w, 0, lay.records, s);
   if (e != cudaSuccess) return cuda_fail(e, "status reset");
-  // steps that enter no snapshot (after the last one written) are not visited
-  e = cudaMemsetAsync(a.gstep, 0, (size_t)t->total_steps * kAG * 8 * lay.n_split, s);
-  if (e != cudaSuccess) return cuda_fail(e, "gradient reset");
   const int n_sm = device_sm_count();
   const int64_t step_blocks = std::max<int64_t>(
       16, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
   if (t->total_steps > 0) launch_far_prepass(a.f, (int)step_blocks, s);
-  adj_globals_kernel<<<1, 256, 0, s>>>(a.f, a.wtab, a.glob);
+  adj_setup_kernel<<<2, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kASteps);
   {
     const uint64_t work = std::max<uint64_t>(P, n_dirs);
     const uint64_t nb = std::min<uint64_t>((work + 255) / 256, (uint64_t)n_sm * 64);
     adj_prep_kernel<<<(unsigned)nb, 256, 0, s>>>(a);
   }
-  adj_items_kernel<<<1, 1024, 0, s>>>(a.f, a.item_off, (uint32_t)kASteps);
-  {
-    double *wpart = (double *)(w + lay.wpart);
-    adj_weight_partial_far_kernel<<<t->n_tracks * lay.w_chunks, kWeightThreads, 0, s>>>(
-        a, P, lay.w_chunks, wpart);
-    adj_weight_final_far_kernel<<<(t->n_tracks + 255) / 256, 256, 0, s>>>(
-        wpart, t->n_tracks, lay.w_chunks, a.linear, t->weight, grad_weight);
-  }
+  a.wpart = (double *)(w + lay.wpart);
+  a.w_chunks = lay.w_chunks;
+  adj_weight_partial_far_kernel<<<t->n_tracks * lay.w_chunks, kWeightThreads, 0, s>>>(
+      a, P, lay.w_chunks, a.wpart);
   rc = cuda_fail(cudaGetLastError(), "adjoint prep launch");
   if (rc) return rc;
   const size_t smem = adj_smem_bytes();
@@ -1118,11 +1111,11 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items_max, 2 * (int64_t)n_sm));
   void *tok = nullptr;
   timing_record(s, true, &tok);
-  for (uint32_t lo = 0; lay.batch && lo < t->n_tracks; lo += lay.batch) {
+  for (uint32_t lo = 0; lay.fl.batch && lo < t->n_tracks; lo += lay.fl.batch) {
     a.t_lo = lo;
-    a.t_hi = std::min(t->n_tracks, lo + lay.batch);
+    a.t_hi = std::min(t->n_tracks, lo + lay.fl.batch);
     launch_adj_fields(a, n_dirs, s);
-    const int64_t most = items_max * lay.n_split;
+    const int64_t most = items_max * lay.fl.n_split;
     adj_interp_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm)),
                         kASteps, 0, s>>>(a);
   }
@@ -1130,11 +1123,9 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   timing_record(s, false, &tok);
   rc = cuda_fail(cudaGetLastError(), "adjoint kernel launch");
   if (rc) return rc;
-  if (t->total_steps > 0) {
-    if (a.f.track_f32)
-      adj_final_kernel<float><<<(int)step_blocks, 256, 0, s>>>(a);
-    else
-      adj_final_kernel<double><<<(int)step_blocks, 256, 0, s>>>(a);
-  }
+  if (a.f.track_f32)
+    adj_final_kernel<float><<<(int)step_blocks, 256, 0, s>>>(a);
+  else
+    adj_final_kernel<double><<<(int)step_blocks, 256, 0, s>>>(a);
   return cuda_fail(cudaGetLastError(), "adjoint final launch");
 }

@@ -71,13 +71,28 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
       l.n_segs = (uint32_t)((uint64_t)total_steps / seg + c.n_tracks);
     }
   }
-  // Several snapshots: a unit per interval between them; a snapshot's
-  // transform adds up the circles of the intervals before it.
-  if (n_snaps > 1 && n_snaps <= 16 && units <= resident &&
-      units * n_snaps * l.slice_bytes <= (4ull << 30)) {
-    l.split = true;
-    l.seg_steps = 0;
-    l.n_segs = c.n_tracks * n_snaps;
+  if (n_snaps > 1) {
+    // A snapshot costs transforms that grow with the circle and, of several
+    // units' circles, leave the L2: with few steps between two, the term-by-term
+    // kernel, which only reads its sums out, is ahead (ms, transforms / term by
+    // term, 40 tracks, 24 x 24 directions, steps x frequencies / cells in
+    // brackets: far 64 frequencies 4.6 / 5.4 [7], 256: 4.4 / 9.2 [22] and
+    // 26 / 24 [7], 400: 11.1 / 14.9 [22] and 76 / 46 [5]; near 400: 34.9 / 35.0
+    // [22], 298 / 120 [5]).
+    if (mean * c.n_omega * 128 < 3ull * l.M * l.M * l.n_bands * n_snaps) return FastLayout{};
+    // A unit per interval between them; a snapshot's transform adds up the
+    // circles of the intervals before it.  More than 16 or 4 GiB: whole tracks,
+    // which takes some hundred of them (32 directions, 900 steps, 20 snapshots,
+    // 256 frequencies: 40 tracks far 2.84 / 1.81 ms, near 10.5 / 2.3; 300 tracks
+    // 3.4 / 8.9 and 11.4 / 11.3).
+    if (n_snaps <= 16 && units <= resident &&
+        units * n_snaps * l.slice_bytes <= (4ull << 30)) {
+      l.split = true;
+      l.seg_steps = 0;
+      l.n_segs = c.n_tracks * n_snaps;
+    } else if (8 * units < resident) {
+      return FastLayout{};
+    }
   }
   uint64_t subs;
   if (l.split) {

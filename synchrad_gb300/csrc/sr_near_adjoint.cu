@@ -32,6 +32,7 @@
 
 #include "sr_common.cuh"
 #include "sr_internal.h"
+#include "sr_fast_sum.cuh"
 #include "sr_mixed_common.cuh"
 #include "sr_adjoint_common.cuh"
 
@@ -58,9 +59,15 @@ struct NearAdjParams {
   float4 *sctab;               // [n_screen] (X hi, lo, Y hi, lo) of the screen point
   AdjGlobals *glob;
   int64_t *item_off;           // [n_tracks + 1] first work item of each track
-  double *gstep;               // [total_steps][kNAG] per-step gradients (x, beta)
+  double *gstep;               // [n_split][total_steps][kNAG] per-step gradients (x, beta)
+  uint32_t n_split;            // runs of screen points summed apart
+  float4 *bandtab;             // [n_bands] centre frequency / 2 pi
+  float2 *fields;              // transforms' cells of a batch of tracks (see below)
+  uint32_t t_lo, t_hi;         // the batch
   double *grad[6];             // x, y, z, ux, uy, uz  [total_steps]
   double *grad_w;              // [n_tracks]
+  double *wpart;               // [n_tracks][w_chunks] partial weight gradients
+  uint32_t w_chunks;
 };
 
 // Point sensitivity (FP64) of the loss to (A_x, A_y, A_z) at point gi for the
@@ -118,16 +125,6 @@ __global__ void nadj_weight_partial_kernel(NearAdjParams a, uint64_t P, uint32_t
   if (threadIdx.x == 0) wpart[blockIdx.x] = red[0];
 }
 
-__global__ void nadj_weight_final_kernel(const double *wpart, uint32_t n_tracks,
-                                         uint32_t n_chunks, int linear, const double *weight,
-                                         double *grad_w) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tracks) return;
-  double s = 0.0;
-  for (uint32_t b = 0; b < n_chunks; ++b) s += wpart[(uint64_t)t * n_chunks + b];
-  grad_w[t] = linear ? (weight[t] > 0.0 ? s / (2.0 * sqrt(weight[t])) : 0.0) : 0.5 * s;
-}
-
 // Point sensitivities in FP32 and the screen table.
 __global__ void nadj_prep_kernel(NearAdjParams a) {
   const FarMixedParams &p = a.f;
@@ -148,6 +145,16 @@ __global__ void nadj_prep_kernel(NearAdjParams a) {
     const df Y = df_from_double(p.sin_theta[iR] * p.sin_phi[iP]);  // radius * sin(phi)
     a.sctab[d] = make_float4(X.hi, X.lo, Y.hi, Y.lo);
   }
+  if (p.fast.M != 0u) {
+    const double w0 = p.omega[0];
+    const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < p.fast.n_bands;
+         b += stride) {
+      const uint32_t j0 = (uint32_t)b * p.fast.nb, n = min(p.fast.nb, p.n_omega - j0);
+      const df c = df_from_double((w0 + (double)(j0 + n / 2) * dw) * 0.15915494309189533577);
+      a.bandtab[b] = make_float4(c.hi, c.lo, 0.f, 0.f);
+    }
+  }
 }
 
 // dL/du_s from dL/dbeta_s (beta = u / gamma at the same step).
@@ -155,6 +162,7 @@ template <typename TT>
 __global__ void nadj_final_kernel(NearAdjParams a) {
   const FarMixedParams &p = a.f;
   const TT *UX = (const TT *)p.ux, *UY = (const TT *)p.uy, *UZ = (const TT *)p.uz;
+  adj_weight_final(p, a.wpart, a.w_chunks, a.linear, a.grad_w);
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < p.total_steps;
        g += (int64_t)gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = p.n_tracks;
@@ -166,7 +174,8 @@ __global__ void nadj_final_kernel(NearAdjParams a) {
     const int64_t s = g - p.offsets[t];
     double v[kNAG] = {0, 0, 0, 0, 0, 0};
     if (s < (int64_t)track_body(p, t))
-      for (int c = 0; c < kNAG; ++c) v[c] = a.gstep[g * kNAG + c];
+      for (uint32_t k = 0; k < a.n_split; ++k)
+        for (int c = 0; c < kNAG; ++c) v[c] += a.gstep[((int64_t)k * p.total_steps + g) * kNAG + c];
     a.grad[0][g] = v[0];
     a.grad[1][g] = v[1];
     a.grad[2][g] = v[2];
@@ -247,6 +256,7 @@ __device__ __forceinline__ NearGeo near_geo(const float4 *rec, const float4 &sc,
 template <int W>
 __global__ void __launch_bounds__(W * 32, 2) nadj_kernel(NearAdjParams a) {
   const FarMixedParams &p = a.f;
+  if (by_transform(p)) return;  // nadj_interp_kernel's
   extern __shared__ __align__(128) unsigned char smem_raw[];
   NearAdjSmem &sm = *reinterpret_cast<NearAdjSmem *>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -512,11 +522,314 @@ __global__ void __launch_bounds__(W * 32, 2) nadj_kernel(NearAdjParams a) {
   }
 }
 
+// ------------------------------------------------------------------------
+// Even omega axes: the sums over omega by transforms, as in the far-field
+// adjoint (sr_far_adjoint.cu).  Nine fields per (track, screen point): conj(U_k),
+// omega conj(U_k) and omega^2 conj(U_k), k = x, y, z; a cell holds the nine
+// complex values and one of padding (80 bytes, five 16-byte loads), and a
+// (screen point, step) takes 8 cells: bound by the 40 loads, 160 cycles per
+// warp and SM.
+// ------------------------------------------------------------------------
+constexpr int kNAFields = 9, kNACell = 10;  // fields; float2 per cell
+
+__device__ __forceinline__ void near_point_u(const NearAdjParams &a, uint32_t t, uint32_t k0,
+                                             uint32_t k1, uint64_t P, uint64_t gi, float wt,
+                                             float swt, float (&ur)[3], float (&ui)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) ur[k] = ui[k] = 0.f;
+  for (uint32_t ks = k0; ks <= k1; ++ks) {
+    const uint64_t ic = 2 * ((uint64_t)ks * P + gi);
+    const float4 C0 = a.gcst[ic], C1 = a.gcst[ic + 1];
+    if (a.linear) {  // U_k = sqrt(w) V_k
+      ur[0] += swt * C0.x; ui[0] += swt * C0.y;
+      ur[1] += swt * C0.z; ui[1] += swt * C0.w;
+      ur[2] += swt * C1.x; ui[2] += swt * C1.y;
+    } else {         // U_k = w g'_k A_k
+      const uint64_t ia = 2 * (((uint64_t)t * a.f.n_snaps + ks) * P + gi);
+      const float4 A0 = a.save_A[ia], A1 = a.save_A[ia + 1];
+      ur[0] += wt * C0.x * A0.x; ui[0] += wt * C0.x * A0.y;
+      ur[1] += wt * C0.y * A0.z; ui[1] += wt * C0.y * A0.w;
+      ur[2] += wt * C0.z * A1.x; ui[2] += wt * C0.z * A1.y;
+    }
+  }
+}
+
+template <int R1>
+__global__ void __launch_bounds__(kFastWarps * 32, 3) nadj_fields_kernel(
+    const __grid_constant__ NearAdjParams a) {
+  const FarMixedParams &p = a.f;
+  if (!by_transform(p)) return;
+  constexpr int NF = 32 / R1, M = 32 * R1;
+  __shared__ float2 tr_all[kFastWarps][32 * 33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2 *tr = tr_all[warp];
+  const FastParams &f = p.fast;
+  const uint32_t n_scr = p.n_theta * p.n_phi;
+  const uint64_t P = (uint64_t)p.n_omega * n_scr;
+  uint64_t task = (uint64_t)blockIdx.x * kFastWarps + warp;
+  const uint32_t band = (uint32_t)(task % f.n_bands);
+  task /= f.n_bands;
+  const uint32_t d = (uint32_t)(task % n_scr);
+  task /= n_scr;
+  const uint32_t k0 = (uint32_t)(task % p.n_snaps), t = a.t_lo + (uint32_t)(task / p.n_snaps);
+  if (t >= a.t_hi) return;
+  const uint32_t k1 = last_fired(p, t);
+  if (k1 == 0xffffffffu || k0 > k1) return;
+  const uint32_t j0 = band * f.nb;
+  const int nb = (int)min(f.nb, p.n_omega - j0);
+  const float wt = (float)p.weight[t], swt = (float)sqrt(p.weight[t]);
+#pragma unroll 1
+  for (int f0 = 0; f0 < kNAFields; f0 += NF) {
+    float2 x[NF][R1], y[32];
+#pragma unroll
+    for (int i = 0; i < R1; ++i) {
+      const int n = 32 * i + lane;                        // frequency index mod M
+      const int j = (n < M / 2 ? n : n - M) + nb / 2;
+      float ur[3] = {0.f, 0.f, 0.f}, ui[3] = {0.f, 0.f, 0.f}, dv = 0.f, w = 0.f;
+      if (j >= 0 && j < nb) {
+        near_point_u(a, t, k0, k1, P, (uint64_t)d * p.n_omega + j0 + j, wt, swt, ur, ui);
+        dv = (float)f.deconv[j - nb / 2 + kFastMaxBand / 2];
+        w = a.wtab[j0 + j].z;
+      }
+#pragma unroll
+      for (int q = 0; q < NF; ++q) {
+        const int fq = f0 + q, c = fq % 3, e = fq / 3;    // component, power of omega
+        const float g = dv * (e == 0 ? 1.f : e == 1 ? w : w * w);
+        const float re = c == 0 ? ur[0] : c == 1 ? ur[1] : ur[2];
+        const float im = c == 0 ? ui[0] : c == 1 ? ui[1] : ui[2];
+        x[q][i] = make_float2(re * g, -im * g);
+      }
+    }
+    fft_fields<R1, NF>(x, y, tr, f.twiddle, lane);
+    const int q = lane / R1, al = lane % R1, fq = f0 + q;
+    if (fq < kNAFields) {
+      float2 *o = a.fields +
+                  ((((uint64_t)(t - a.t_lo) * p.n_snaps + k0) * n_scr + d) * f.n_bands + band) *
+                      ((uint64_t)kNACell * (M + kTaps)) + fq;
+#pragma unroll
+      for (int b = 0; b < 32; ++b) o[kNACell * (al + R1 * b)] = y[bitrev<32>(b)];
+      // the circle's first cells once more behind its last
+#pragma unroll
+      for (int b = 0; b * R1 < kTaps; ++b)
+        if (al + R1 * b < kTaps) o[kNACell * (M + al + R1 * b)] = y[bitrev<32>(b)];
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kNASteps, 2) nadj_interp_kernel(
+    const __grid_constant__ NearAdjParams a) {
+  const FarMixedParams &p = a.f;
+  if (!by_transform(p)) return;
+  const FastParams &f = p.fast;
+  const int lane = threadIdx.x & 31;
+  const uint32_t nR = p.n_theta, n_scr = nR * p.n_phi;
+  const uint64_t P = (uint64_t)p.n_omega * n_scr;
+  const AdjGlobals G = *a.glob;
+  const df dL = df_from_double(p.L_screen);
+  const int M = (int)f.M;
+  const float Mf = (float)M;
+  const double dw = (p.omega[p.n_omega - 1] - p.omega[0]) / (double)(p.n_omega - 1);
+  const df f_d = df_from_double(dw * 0.15915494309189533577);
+  const int64_t i_lo = a.item_off[a.t_lo], i_hi = a.item_off[a.t_hi];
+  const int64_t n_items = (i_hi - i_lo) * a.n_split;
+
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int64_t it = i_lo + item / a.n_split;
+    const uint32_t split = (uint32_t)(item % a.n_split);
+    const uint32_t dA = (uint32_t)((uint64_t)n_scr * split / a.n_split);
+    const uint32_t dB = (uint32_t)((uint64_t)n_scr * (split + 1) / a.n_split);
+    uint32_t lo = a.t_lo, hi = a.t_hi;  // last track with item_off[t] <= it
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (a.item_off[mid] <= it) lo = mid; else hi = mid;
+    }
+    const uint32_t t = lo;
+    const int64_t base = p.offsets[t];
+    SnapSegment seg{0, 0, 0, 0};
+    track_segments(p, t, (uint32_t)kNASteps, (uint32_t)(it - a.item_off[t]), &seg);
+    const uint32_t s = seg.r0 + threadIdx.x;
+    const bool valid = s < seg.r1;
+    if (!__any_sync(0xffffffffu, valid)) continue;  // whole warps
+    const uint32_t sc = valid ? s : seg.r1 - 1;
+    const uint32_t it_start = p.it_start[t];
+    const float wt = (float)p.weight[t], swt = (float)sqrt(p.weight[t]);
+    const float4 *rp = p.records + (base + sc) * kRecF4;
+    const float4 rec[3] = {__ldg(rp), __ldg(rp + 1), __ldg(rp + 2)};
+    // differences to the step before, for the quick test of the mask
+    float dq = 0.f, dz = 0.f, dx = 0.f, dy = 0.f, d2 = 0.f;
+    if (sc > 0) {
+      const float4 e0 = __ldg(rp - kRecF4), e1 = __ldg(rp - kRecF4 + 1);
+      dq = (rec[0].x - e0.x) + (rec[0].y - e0.y);
+      dx = (rec[0].z - e0.z) + (rec[0].w - e0.w);
+      dy = (rec[1].x - e1.x) + (rec[1].y - e1.y);
+      dz = (rec[1].z - e1.z) + (rec[1].w - e1.w);
+      d2 = dx * dx + dy * dy + dz * dz;
+    }
+    double gD[kNAG];
+    float gF[kNAG];
+#pragma unroll
+    for (int c = 0; c < kNAG; ++c) {
+      gD[c] = 0.0;
+      gF[c] = 0.f;
+    }
+    const float2 *fld = a.fields + (((uint64_t)(t - a.t_lo) * p.n_snaps + seg.k0) * n_scr) *
+                                       f.n_bands * ((uint64_t)kNACell * (M + kTaps));
+#pragma unroll 1
+    for (uint32_t d = dA; d < dB; ++d) {
+      const float4 scr = __ldg(a.sctab + d);
+      const NearGeo g = near_geo(rec, scr, dL);
+      const float ir = __frcp_rn(g.r);
+      int mode = valid ? 0 : 1;  // 0: every frequency enters, 1: none, 2: some
+      float R0[3] = {0.f, 0.f, 0.f}, I1[3] = {0.f, 0.f, 0.f}, R2[3] = {0.f, 0.f, 0.f};
+      // mask: certain where the FP32 difference (first order in the step, with
+      // the second as a bound) leaves a 1e-3 margin, else from the double-float
+      // times of both steps
+      const float quick =
+          sc > 0 ? fabsf(dq + g.omn * dz - g.nx * dx - g.ny * dy) + d2 * ir : INFINITY;
+      if (__any_sync(0xffffffffu, valid && !(G.wabs_max * quick < 0.999f * kPiLo))) {
+        // the track's first step compares the whole phase omega (t + r) with zero
+        float dt0 = (g.tau.hi + g.tau.lo) + (dL.hi + dL.lo);
+        if (sc > 0) {
+          const float4 prev[3] = {__ldg(rp - kRecF4), __ldg(rp - kRecF4 + 1),
+                                  __ldg(rp - kRecF4 + 2)};
+          const NearGeo gp = near_geo(prev, scr, dL);
+          dt0 = (g.tau.hi - gp.tau.hi) + (g.tau.lo - gp.tau.lo);
+        }
+        const float adt = fabsf(dt0);
+        if (valid) mode = G.wabs_max * adt < kPiLo ? 0 : (G.wabs_min * adt > kPiHi ? 1 : 2);
+        // cut steps, one after the other: the warp sums the included frequencies
+        // term by term
+        const uint32_t mine =
+            mode == 2 ? cut_interval<true>(p, 0, (int)p.n_omega, G.w0f, G.dwf, d, base, s,
+                                           it_start, adt)
+                      : 1u;
+        for (uint32_t cut = __ballot_sync(0xffffffffu, mode == 2); cut; cut &= cut - 1) {
+          const int b = __ffs(cut) - 1;
+          const uint32_t r = __shfl_sync(0xffffffffu, mine, b);
+          const float th = __shfl_sync(0xffffffffu, g.tau.hi, b);
+          const float tl = __shfl_sync(0xffffffffu, g.tau.lo, b);
+          const int jf = (int)(r & 0xffffu), jl = (int)(r >> 16);
+          float v[9];
+#pragma unroll
+          for (int k = 0; k < 9; ++k) v[k] = 0.f;
+          for (int j = jf + lane; j <= jl; j += 32) {
+            float ur[3], ui[3];
+            near_point_u(a, t, seg.k0, seg.k1, P, (uint64_t)d * p.n_omega + j, wt, swt, ur, ui);
+            const float4 w = a.wtab[j];
+            float zs, zc;
+            phasor_rev(w.x, w.y, th, tl, zs, zc);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const float re = ur[k] * zc + ui[k] * zs;
+              v[k] += re;
+              v[3 + k] += w.z * (ur[k] * zs - ui[k] * zc);
+              v[6 + k] += w.z * w.z * re;
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 9; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+          }
+          if (lane == b) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              R0[k] = v[k];
+              I1[k] = v[3 + k];
+              R2[k] = v[6 + k];
+            }
+          }
+        }
+      }
+      if (mode == 0) {
+        const float pr = f_d.hi * g.tau.hi;
+        float e = __fmaf_rn(f_d.hi, g.tau.hi, -pr);
+        e = __fmaf_rn(f_d.hi, g.tau.lo, e);
+        e = __fmaf_rn(f_d.lo, g.tau.hi, e);
+        const float uh = (pr - rintf(pr)) * Mf, ul = e * Mf;
+        const float rm = rintf((uh - 0.5f) + ul);
+        float wk[kTaps];
+        kb_taps(((uh - rm) - 0.5f) + ul, wk);
+        const int m = ((int)rm - 3) & (M - 1);
+        for (uint32_t band = 0; band < f.n_bands; ++band) {
+          const float4 *cell = reinterpret_cast<const float4 *>(
+              fld + ((uint64_t)d * f.n_bands + band) * ((uint64_t)kNACell * (M + kTaps)) +
+              kNACell * m);
+          float2 h[kNACell];
+#pragma unroll
+          for (int k = 0; k < kNACell; ++k) h[k] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int l = 0; l < kTaps; ++l) {
+            const float2 ww = make_float2(wk[l], wk[l]);
+#pragma unroll
+            for (int k = 0; k < kNACell / 2; ++k) {
+              const float4 v = __ldg(cell + (kNACell / 2) * l + k);
+              h[2 * k] = __ffma2_rn(ww, make_float2(v.x, v.y), h[2 * k]);
+              if (2 * k + 1 < kNAFields)
+                h[2 * k + 1] = __ffma2_rn(ww, make_float2(v.z, v.w), h[2 * k + 1]);
+            }
+          }
+          const float4 fc = __ldg(a.bandtab + band);  // its centre frequency / 2 pi
+          float zs, zc;
+          phasor_exact(fc.x, fc.y, g.tau.hi, g.tau.lo, zs, zc);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            R0[k] += h[k].x * zc - h[k].y * zs;
+            I1[k] += h[3 + k].x * zs + h[3 + k].y * zc;
+            R2[k] += h[6 + k].x * zc - h[6 + k].y * zs;
+          }
+        }
+      }
+      if (mode != 1) {  // the chain rule
+        const float n[3] = {g.nx, g.ny, g.nz};
+        const float bmn[3] = {rec[2].x - g.nx, rec[2].y - g.ny, g.omn - rec[2].w};  // beta - n
+        const float ir2 = ir * ir, ir3 = ir2 * ir;
+        const float nR0 = n[0] * R0[0] + n[1] * R0[1] + n[2] * R0[2];
+        const float nI1 = n[0] * I1[0] + n[1] * I1[1] + n[2] * I1[2];
+        const float bI1 = bmn[0] * I1[0] + bmn[1] * I1[1] + bmn[2] * I1[2];
+        const float bR2 = bmn[0] * R2[0] + bmn[1] * R2[1] + bmn[2] * R2[2];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          gF[k] += (3.f * n[k] * nR0 - R0[k]) * ir3 -
+                   (I1[k] + n[k] * bI1 - 2.f * n[k] * nI1) * ir2 + n[k] * bR2 * ir;
+          gF[3 + k] -= I1[k] * ir;
+        }
+      }
+      if (((d - dA) & 31u) == 31u || d + 1 == dB) {  // FP32 over 32 points, then FP64
+#pragma unroll
+        for (int c = 0; c < kNAG; ++c) {
+          gD[c] += (double)gF[c];
+          gF[c] = 0.f;
+        }
+      }
+    }
+    if (valid) {
+#pragma unroll
+      for (int c = 0; c < kNAG; ++c)
+        a.gstep[((uint64_t)split * p.total_steps + base + s) * kNAG + c] = gD[c];
+    }
+  }
+}
+
+void launch_nadj_fields(const NearAdjParams &a, uint64_t n_scr, cudaStream_t s) {
+  const uint64_t warps =
+      (uint64_t)(a.t_hi - a.t_lo) * a.f.n_snaps * n_scr * a.f.fast.n_bands;
+  const unsigned blocks = (unsigned)((warps + kFastWarps - 1) / kFastWarps);
+  switch (a.f.fast.M) {
+    case 128: nadj_fields_kernel<4><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    case 256: nadj_fields_kernel<8><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    case 512: nadj_fields_kernel<16><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+    default: nadj_fields_kernel<32><<<blocks, kFastWarps * 32, 0, s>>>(a); break;
+  }
+}
+
 size_t nadj_smem_bytes() { return sizeof(NearAdjSmem); }
 
 struct NearAdjLayout {
-  size_t records, gcst, wtab, sctab, glob, item_off, gstep, wpart, total;
+  size_t records, gcst, wtab, sctab, glob, item_off, gstep, wpart, tables, bandtab, fields, total;
   uint32_t w_chunks;
+  AdjFields fl;
 };
 
 NearAdjLayout nadj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t n_scr,
@@ -524,15 +837,19 @@ NearAdjLayout nadj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uin
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   NearAdjLayout l;
   l.w_chunks = adj_weight_chunks(P, n_tracks, device_sm_count());
-  l.records = 256;
+  l.fl = adj_fields_layout(total_steps, n_omega, n_scr, n_tracks, n_snaps, kNACell * 8, kNASteps);
+  l.gstep = 256;
+  l.records = l.gstep + up((size_t)total_steps * kNAG * 8 * l.fl.n_split);
   l.gcst = l.records + up((size_t)total_steps * kRecBytes);
   l.wtab = l.gcst + up((size_t)P * 32 * (n_snaps ? n_snaps : 1));
   l.sctab = l.wtab + up((size_t)n_omega * 16);
   l.glob = l.sctab + up((size_t)n_scr * 16);
   l.item_off = l.glob + 256;
-  l.gstep = l.item_off + up(((size_t)n_tracks + 1) * 8);
-  l.wpart = l.gstep + up((size_t)total_steps * kNAG * 8);
-  l.total = l.wpart + up((size_t)n_tracks * l.w_chunks * 8);
+  l.wpart = l.item_off + up(((size_t)n_tracks + 1) * 8);
+  l.tables = l.wpart + up((size_t)n_tracks * l.w_chunks * 8);
+  l.bandtab = l.tables + up(kFastTables);
+  l.fields = l.bandtab + up((size_t)l.fl.n_bands * 16);
+  l.total = l.fields + l.fl.bytes;
   return l;
 }
 
@@ -647,49 +964,54 @@ extern "C" int sr_near_backward(const sr_tracks *t, const sr_grid *g, int comp,
   a.gstep = (double *)(w + lay.gstep);
   for (int i = 0; i < 6; ++i) a.grad[i] = grad_track[i];
   a.grad_w = grad_weight;
+  a.n_split = lay.fl.n_split;
+  a.bandtab = (float4 *)(w + lay.bandtab);
+  a.fields = (float2 *)(w + lay.fields);
+  if (lay.fl.batch)
+    fast_tables_bind(a.f, lay.fl.n_bands, lay.fl.nb, lay.fl.M, w + lay.tables, w);
 
-  e = cudaMemsetAsync(w, 0, 256, s);
+  // the status block and, behind it, the per-step gradients: steps that enter
+  // no snapshot (after the last one written) are not visited
+  e = cudaMemsetAsync(w, 0, lay.records, s);
   if (e != cudaSuccess) return cuda_fail(e, "status reset");
-  // steps that enter no snapshot (after the last one written) are not visited
-  e = cudaMemsetAsync(a.gstep, 0, (size_t)t->total_steps * kNAG * 8, s);
-  if (e != cudaSuccess) return cuda_fail(e, "gradient reset");
   const int n_sm = device_sm_count();
   const int64_t step_blocks = std::max<int64_t>(
-      1, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
+      16, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
   if (t->total_steps > 0) launch_near_prepass(a.f, (int)step_blocks, s);
-  adj_globals_kernel<<<1, 256, 0, s>>>(a.f, a.wtab, a.glob);
+  adj_setup_kernel<<<2, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kNASteps);
   {
     const uint64_t work = std::max<uint64_t>(P, n_scr);
     const uint64_t nb = std::min<uint64_t>((work + 255) / 256, (uint64_t)n_sm * 64);
     nadj_prep_kernel<<<(unsigned)nb, 256, 0, s>>>(a);
   }
-  adj_items_kernel<<<1, 1024, 0, s>>>(a.f, a.item_off, (uint32_t)kNASteps);
-  {
-    double *wpart = (double *)(w + lay.wpart);
-    nadj_weight_partial_kernel<<<t->n_tracks * lay.w_chunks, kWeightThreads, 0, s>>>(
-        a, P, lay.w_chunks, wpart);
-    nadj_weight_final_kernel<<<(t->n_tracks + 255) / 256, 256, 0, s>>>(
-        wpart, t->n_tracks, lay.w_chunks, a.linear, t->weight, grad_weight);
-  }
+  a.wpart = (double *)(w + lay.wpart);
+  a.w_chunks = lay.w_chunks;
+  nadj_weight_partial_kernel<<<t->n_tracks * lay.w_chunks, kWeightThreads, 0, s>>>(
+      a, P, lay.w_chunks, a.wpart);
   rc = cuda_fail(cudaGetLastError(), "near adjoint prep launch");
   if (rc) return rc;
   const size_t smem = nadj_smem_bytes();
-  e = cudaFuncSetAttribute(nadj_kernel<kNAW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
+  e = allow_smem((const void *)nadj_kernel<kNAW>, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "near adjoint smem attribute");
-  const int64_t items_max = t->total_steps / kNASteps + (int64_t)t->n_tracks;
+  const int64_t items_max = t->total_steps / kNASteps + (int64_t)t->n_tracks * t->n_snaps;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items_max, 2 * (int64_t)n_sm));
   void *tok = nullptr;
   timing_record(s, true, &tok);
+  for (uint32_t lo = 0; lay.fl.batch && lo < t->n_tracks; lo += lay.fl.batch) {
+    a.t_lo = lo;
+    a.t_hi = std::min(t->n_tracks, lo + lay.fl.batch);
+    launch_nadj_fields(a, n_scr, s);
+    const int64_t most = items_max * lay.fl.n_split;
+    nadj_interp_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm)),
+                         kNASteps, 0, s>>>(a);
+  }
   nadj_kernel<kNAW><<<grid, kNAW * 32, smem, s>>>(a);
   timing_record(s, false, &tok);
   rc = cuda_fail(cudaGetLastError(), "near adjoint kernel launch");
   if (rc) return rc;
-  if (t->total_steps > 0) {
-    if (a.f.track_f32)
-      nadj_final_kernel<float><<<(int)step_blocks, 256, 0, s>>>(a);
-    else
-      nadj_final_kernel<double><<<(int)step_blocks, 256, 0, s>>>(a);
-  }
+  if (a.f.track_f32)
+    nadj_final_kernel<float><<<(int)step_blocks, 256, 0, s>>>(a);
+  else
+    nadj_final_kernel<double><<<(int)step_blocks, 256, 0, s>>>(a);
   return cuda_fail(cudaGetLastError(), "near adjoint final launch");
 }
