@@ -33,12 +33,20 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
   l.nb = (c.n_omega + l.n_bands - 1) / l.n_bands;
   l.M = fast_cells(l.nb);
   l.n_dwb = (c.n_dirs + 31) / 32 * l.n_bands;
-  l.slice_bytes = up256((size_t)32 * (np * (size_t)(l.M + 2 * l.nb) * 16 +
-                                      kFastList * (16 + 8 * (size_t)np)));
+  // A list holds what a segment of a block can add and a chunk more (it is
+  // summed when a further chunk might not fit), longer walks get longer ones:
+  // each emptying reads and writes the warp's direct sums (half of the steps
+  // listed, 256 frequencies: 48.9 ms with 96 entries, 38.5 with 512).
+  auto use_list = [&](uint32_t entries) {
+    l.list = entries;
+    l.slice_bytes = up256((size_t)32 * (np * (size_t)(l.M + 2 * l.nb) * 16 +
+                                        entries * (16 + 8 * (size_t)np)));
+  };
   // Steps between two writes of the whole window: 128, fewer where they could
   // lap the circle (a step moves by up to M / (2 nb) cells).
   l.block = 128;
   while (l.block > 32 && (uint64_t)l.block * l.M + 16ull * l.nb > 2ull * l.nb * l.M) l.block /= 2;
+  use_list(l.block + 32);
   const uint64_t resident = (uint64_t)c.n_sm * (near ? 2 : 3) * kFastWarps;
   const uint64_t units = (uint64_t)c.n_tracks * l.n_dwb;
   l.dirs_per_warp = std::max(1u, 512u / l.M);
@@ -53,8 +61,9 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
   // the few long tracks that would not fill the SMs, else tracks stay whole.
   if (n_snaps == 1 && units <= resident) {
     const uint64_t all = (uint64_t)total_steps * l.n_dwb;
-    const uint64_t room = (4ull << 30) / l.slice_bytes;
     uint64_t seg = l.block;
+    if (l.M >= 512) use_list(kFastList);
+    const uint64_t room = (4ull << 30) / l.slice_bytes;
     if (l.M >= 512)
       seg = std::max<uint64_t>(
           seg, (uint64_t)(std::sqrt((double)all * (2.0 * np * l.M * 512.0) / 1.6e6) / 128.0) * 128);
@@ -64,6 +73,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
       const uint64_t most =
           std::max<uint64_t>(2 * resident, std::min<uint64_t>(4 * resident, room));
       seg = std::max<uint64_t>(seg, (all / (most - units) / 128 + 1) * 128);
+      use_list(kFastList);
     }
     if (split && (uint64_t)total_steps > seg) {
       l.split = true;
@@ -85,6 +95,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
     // which takes some hundred of them (32 directions, 900 steps, 20 snapshots,
     // 256 frequencies: 40 tracks far 2.84 / 1.81 ms, near 10.5 / 2.3; 300 tracks
     // 3.4 / 8.9 and 11.4 / 11.3).
+    use_list(kFastList);
     if (n_snaps <= 16 && units <= resident &&
         units * n_snaps * l.slice_bytes <= (4ull << 30)) {
       l.split = true;
@@ -94,6 +105,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
       return FastLayout{};
     }
   }
+  if (!l.split) use_list(kFastList);
   uint64_t subs;
   if (l.split) {
     const uint64_t groups = (uint64_t)l.n_dwb * (32u / l.dirs_per_warp) * n_snaps;
@@ -133,6 +145,7 @@ void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char 
   f.n_segs = l.n_segs;
   f.seg_steps = l.seg_steps;
   f.block = l.block;
+  f.list = l.list;
   f.dirs_per_warp = l.dirs_per_warp;
   // phi nodes spanned by 32 consecutive directions, and the steps whose turned
   // records of all of them fit the staging buffer (128 records)

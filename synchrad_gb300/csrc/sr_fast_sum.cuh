@@ -35,7 +35,7 @@ namespace sr {
 namespace {
 
 constexpr int kTaps = 8;
-constexpr int kFastList = 96;     // list entries per lane (a chunk adds at most 32)
+constexpr int kFastList = 512;    // list entries per lane, fewer for short segments
 constexpr int kFastWarps = 4;     // warps per CTA
 // Per-warp shared memory: step records of the current chunk while spreading,
 // the transpose buffer of the FFT otherwise; the first field's outputs; the
@@ -247,13 +247,13 @@ struct FastSlice {
   __device__ float4 *grid() const { return (float4 *)base; }
   // [NP][32][2][nb] direct sums of the listed steps: sums, then low parts
   __device__ float4 *part(const FastParams &f) const { return grid() + (size_t)NP * 32 * f.M; }
-  // [32][kFastList] tau.hi, tau.lo, first | last << 16
+  // [32][list] tau.hi, tau.lo, first | last << 16
   __device__ float4 *lhead(const FastParams &f) const {
     return grid() + (size_t)NP * 32 * (f.M + 2 * f.nb);
   }
-  // [NP][32][kFastList] amplitudes X, Y
+  // [NP][32][list] amplitudes X, Y
   __device__ float2 *lamp(const FastParams &f) const {
-    return (float2 *)(lhead(f) + kFastList * 32);
+    return (float2 *)(lhead(f) + f.list * 32);
   }
 };
 
@@ -483,13 +483,16 @@ __device__ __forceinline__ uint32_t cut_interval(const FarMixedParams &p, uint32
 
 // Direct sums of the listed steps of every lane, by the whole warp: point
 // j = lane + 32 k, seeded by sin/cos and rotated by exp(32 i d_omega tau).
-// Two entries at a time share the packed FP32 operations (their chains are
-// independent; one at a time the sums waited for the rotations).  At most 8
-// blocks of 32 points per pass, so that the pair sums stay in registers.
+// Pairs of entries share the packed FP32 operations, and two pairs run side by
+// side: bound by the instructions of short dependent chains at 12 warps an SM
+// (16 betatron tracks, half of their steps listed, 256 frequencies: one pair
+// 35.8 ms, two 33.6, four 46.4, out of registers; the entries' values handed
+// round by shuffles 38.5 where shared memory takes 35.8).  At most 8 blocks of
+// 32 points per pass, so that the pair sums stay in registers.
 template <bool NEAR, int NK>
 __device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<NEAR> sl, uint32_t slot0,
                                          uint32_t j0, int nb, int64_t base, uint32_t it_start,
-                                         int n_list, bool dirty, int lane) {
+                                         int n_list, bool dirty, FastSmem &sm, int lane) {
   constexpr int NP = NEAR ? 3 : 1;
   constexpr int KB = NK < 8 ? NK : 8;
   __syncwarp();
@@ -502,12 +505,15 @@ __device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<N
   const float w0f = (float)(w0 + (double)j0 * dw), dwf = (float)dw;
   float4 *lhead = sl.lhead(p.fast), *part = sl.part(p.fast);
   const float2 *lamp = sl.lamp(p.fast);
+  constexpr int kPairF = 20;  // floats a staged pair takes (14, padded)
+  constexpr int kPairs = 2;
+  float *pairs = reinterpret_cast<float *>(sm.rec);
   // the included frequencies of each entry, in place of its |dtau|
   for (uint32_t m = has; m; m &= m - 1) {
     const int d = __ffs(m) - 1;
     const int n = __shfl_sync(0xffffffffu, n_list, d);
     for (int e = lane; e < n; e += 32) {
-      float4 *h = lhead + d * kFastList + e;
+      float4 *h = lhead + d * p.fast.list + e;
       const float adt = __ldcg(&h->z);
       const uint32_t s = __float_as_uint(__ldcg(&h->w));
       const uint32_t r =
@@ -533,44 +539,64 @@ __device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<N
           // a lane loads one entry and its rotation; the warp then takes the
           // entries in order
           const int ne = min(32, n - e0), el = e0 + min(lane, ne - 1);
-          const float4 h = __ldcg(lhead + d * kFastList + el);
-          float2 am = __ldcg(lamp + ((size_t)c * 32 + d) * kFastList + el);
-          if (lane >= ne) am = make_float2(0.f, 0.f);
+          const float4 h = __ldcg(lhead + d * p.fast.list + el);
+          float2 am = __ldcg(lamp + ((size_t)c * 32 + d) * p.fast.list + el);
+          const bool own = lane < ne;
+          if (!own) am = make_float2(0.f, 0.f);
           float hs, hc;
           phasor_rev(f32.hi, f32.lo, h.x, h.y, hs, hc);
-          for (int e = 0; e < ne; e += 2) {
-            auto two = [&](float v) {
-              return make_float2(__shfl_sync(0xffffffffu, v, e), __shfl_sync(0xffffffffu, v, e + 1));
-            };
-            const float2 th = two(h.x), tl = two(h.y), r = two(h.z);
-            const float2 vx = two(am.x), vy = two(am.y), rc = two(hc), rs = two(hs);
-            const float2 nrs = make_float2(-rs.x, -rs.y);
-            const uint32_t ra = __float_as_uint(r.x), rb = __float_as_uint(r.y);
-            const int fa = (int)(ra & 0xffffu) - 32 * h0, la = (int)(ra >> 16) - 32 * h0;
-            const int fb = (int)(rb & 0xffffu) - 32 * h0, lb = (int)(rb >> 16) - 32 * h0;
-            // an entry without frequencies (fa > la) adds nothing below: its
-            // block range is empty or masked
-            const int last = max(la, lb);
-            if (last < 0) continue;
-            // blocks below kw are included whole by both
-            const int kw = max(fa, fb) <= 0 ? (min(la, lb) + 1) >> 5 : 0;
-            float2 zc, zs;
-            phasor_rev(fl.hi, fl.lo, th.x, tl.x, zs.x, zc.x);
-            phasor_rev(fl.hi, fl.lo, th.y, tl.y, zs.y, zc.y);
+          __syncwarp();
+          {
+            float *q = pairs + (lane >> 1) * kPairF + (lane & 1);
+            q[0] = h.x; q[2] = h.y; q[4] = own ? h.z : __uint_as_float(1u); q[6] = am.x;
+            q[8] = am.y; q[10] = hc; q[12] = hs;
+          }
+          __syncwarp();
+          for (int e = 0; e < ne; e += 2 * kPairs) {
+            // kPairs chains of rotations side by side; entries past the last of
+            // the list have no amplitude and end at block 0
+            float2 vx[kPairs], vy[kPairs], rc[kPairs], rs[kPairs], zc[kPairs], zs[kPairs];
+            int fa[kPairs], la[kPairs], fb[kPairs], lb[kPairs];
+            int last = -1, whole = 0x7fff;
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) {
+              const float4 *q =
+                  reinterpret_cast<const float4 *>(pairs + ((e >> 1) + i) * kPairF);
+              const float4 q0 = q[0], q1 = q[1], q2 = q[2];
+              rs[i] = *reinterpret_cast<const float2 *>(q + 3);
+              vx[i] = make_float2(q1.z, q1.w);
+              vy[i] = make_float2(q2.x, q2.y);
+              rc[i] = make_float2(q2.z, q2.w);
+              const uint32_t ra = __float_as_uint(q1.x), rb = __float_as_uint(q1.y);
+              fa[i] = (int)(ra & 0xffffu) - 32 * h0;
+              la[i] = (int)(ra >> 16) - 32 * h0;
+              fb[i] = (int)(rb & 0xffffu) - 32 * h0;
+              lb[i] = (int)(rb >> 16) - 32 * h0;
+              // an entry without frequencies (fa > la) adds nothing below: its
+              // block range is empty or masked
+              last = max(last, max(la[i], lb[i]));
+              whole = min(whole, max(fa[i], fb[i]) <= 0 ? min(la[i], lb[i]) + 1 : 0);
+              phasor_rev(fl.hi, fl.lo, q0.x, q0.z, zs[i].x, zc[i].x);
+              phasor_rev(fl.hi, fl.lo, q0.y, q0.w, zs[i].y, zc[i].y);
+            }
+            const int kw = whole >> 5;  // blocks below are included whole by all
 #pragma unroll
             for (int k = 0; k < KB; ++k) {
               if (32 * k > last) break;
-              float2 px = vx, py = vy;
-              if (k >= kw) {
-                const int j = lane + 32 * k;
-                if (j < fa || j > la) px.x = py.x = 0.f;
-                if (j < fb || j > lb) px.y = py.y = 0.f;
+#pragma unroll
+              for (int i = 0; i < kPairs; ++i) {
+                float2 px = vx[i], py = vy[i];
+                if (k >= kw) {
+                  const int j = lane + 32 * k;
+                  if (j < fa[i] || j > la[i]) px.x = py.x = 0.f;
+                  if (j < fb[i] || j > lb[i]) px.y = py.y = 0.f;
+                }
+                xr[k] = __ffma2_rn(px, zc[i], xr[k]);
+                xi[k] = __ffma2_rn(px, zs[i], xi[k]);
+                yr[k] = __ffma2_rn(py, zc[i], yr[k]);
+                yi[k] = __ffma2_rn(py, zs[i], yi[k]);
+                rot2p(zc[i], zs[i], rc[i], rs[i], make_float2(-rs[i].x, -rs[i].y), zc[i], zs[i]);
               }
-              xr[k] = __ffma2_rn(px, zc, xr[k]);
-              xi[k] = __ffma2_rn(px, zs, xi[k]);
-              yr[k] = __ffma2_rn(py, zc, yr[k]);
-              yi[k] = __ffma2_rn(py, zs, yi[k]);
-              rot2p(zc, zs, rc, rs, nrs, zc, zs);
             }
           }
         }
@@ -722,20 +748,20 @@ __device__ __forceinline__ void spread_steps(const FarMixedParams &p, const Fast
         }
       } else if (mine && !(u.wmin * adt > kPiHi)) {
         const int k = w.n_list++;
-        sl.lhead(p.fast)[lane * kFastList + k] =
+        sl.lhead(p.fast)[lane * p.fast.list + k] =
             make_float4(tau.hi, tau.lo, adt, __uint_as_float(s));
 #pragma unroll
         for (int c = 0; c < NP; ++c)
-          sl.lamp(p.fast)[((size_t)c * 32 + lane) * kFastList + k] = make_float2(X[c], Y[c]);
+          sl.lamp(p.fast)[((size_t)c * 32 + lane) * p.fast.list + k] = make_float2(X[c], Y[c]);
       }
     }
     // cells that stay in the window for long would gather hundreds of terms:
     // started afresh every 128 steps (fewer where a sweep would lap the circle), their FP32 sums round a fifth as much
-    const bool drain = __any_sync(0xffffffffu, w.n_list > kFastList - 32);
+    const bool drain = __any_sync(0xffffffffu, w.n_list > (int)p.fast.list - 32);
     if (drain || ((s0 + cnt - from) & (p.fast.block - 1u)) == 0u) {
       if (w.live) window_flush(w, cells, M);
       if (drain) {
-        drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, lane);
+        drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, sm, lane);
         w.dirty = w.dirty || w.n_list > 0;
         w.n_list = 0;
         window_clear(w);
@@ -764,7 +790,7 @@ __device__ __forceinline__ bool spread_range(const FarMixedParams &p, const Fast
   spread_steps<NEAR, NK>(p, u, sl, sm, w, base, it_start, a ? a - 1 : 0u, b, a, lane);
   if (w.live) window_flush(w, sl.grid() + (size_t)lane * p.fast.M, (int)p.fast.M);
   if (__any_sync(0xffffffffu, w.n_list > 0)) {
-    drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, lane);
+    drain_lists<NEAR, NK>(p, sl, u.slot0, u.j0, u.nb, base, it_start, w.n_list, w.dirty, sm, lane);
     w.dirty = w.dirty || w.n_list > 0;
   }
   __threadfence();

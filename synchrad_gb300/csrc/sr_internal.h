@@ -50,6 +50,7 @@ struct FastParams {
   uint32_t n_sub;        // track subsets
   uint32_t n_segs;       // few tracks: segments of seg_steps steps, of all tracks
   uint32_t seg_steps;
+  uint32_t list;         // entries of a lane's list of steps that are summed directly
   uint32_t block;        // steps after which the window is written out (a power of two)
   uint32_t n_phik;       // phi nodes a warp's 32 directions span at most (far field)
   uint32_t chunk;        // steps staged at a time
@@ -116,7 +117,7 @@ struct FarMixedConfig {
 struct FastLayout {
   bool on;     // worth it for these sizes
   bool split;  // steps and transforms in two kernels (few tracks, one snapshot)
-  uint32_t n_bands, nb, M, n_dwb, n_sub, n_segs, seg_steps, block, slices, dirs_per_warp;
+  uint32_t n_bands, nb, M, n_dwb, n_sub, n_segs, seg_steps, block, slices, dirs_per_warp, list;
   size_t slice_bytes;
 };
 FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
