@@ -4,8 +4,8 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <set>
-#include <tuple>
+#include <map>
+#include <utility>
 
 #include "sr_common.cuh"
 #include "sr_internal.h"
@@ -131,15 +131,15 @@ int device_sm_count() { return n_sm_of_current_device(); }
 
 cudaError_t allow_smem(const void *kernel, int bytes) {
   static std::mutex mu;
-  static std::set<std::tuple<int, const void *, int>> done;
+  static std::map<std::pair<int, const void *>, int> most;  // the attribute as last set
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, kernel, bytes);
-  if (done.count(key)) return cudaSuccess;
+  int &have = most[std::make_pair(dev, kernel)];
+  if (bytes <= have) return cudaSuccess;  // never lowered: a later call may need it
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) done.insert(key);
+  if (e == cudaSuccess) have = bytes;
   return e;
 }
 
