@@ -677,6 +677,7 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
   const FarMixedParams &p = a.f;
   if (!by_transform(p)) return;
   const FastParams &f = p.fast;
+  __shared__ float sum[kAG][2][kASteps];
   const int lane = threadIdx.x & 31;
   const uint32_t nT = p.n_theta, n_dirs = nT * p.n_phi;
   const uint64_t P = (uint64_t)p.n_omega * n_dirs;
@@ -722,12 +723,10 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
       dy = (r1.x - e1.x) + (r1.y - e1.y);
       dz = (r1.z - e1.z) + (r1.w - e1.w);
     }
-    double gD[kAG];
+    // x, bbar, a: FP32 over up to 8 directions of a phi (rho, phi, z of each),
+    // turned back and added as double-floats
 #pragma unroll
-    for (int c = 0; c < kAG; ++c) gD[c] = 0.0;
-    float gF[kAG];   // x, bbar, a; within a phi: rho, phi, z of each
-#pragma unroll
-    for (int c = 0; c < kAG; ++c) gF[c] = 0.f;
+    for (int c = 0; c < kAG; ++c) sum[c][0][threadIdx.x] = sum[c][1][threadIdx.x] = 0.f;
     const float2 *fld = a.fields +
                         (((uint64_t)(t - a.t_lo) * p.n_snaps + seg.k0) * n_dirs) * f.n_bands *
                             (4ull * (M + kTaps));
@@ -884,29 +883,31 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
           g_ap -= c2 * ep;
           g_az += ka * ct - c2 * ez;
         }
-      }
-      gF[0] += ph.x * g_xr;
-      gF[1] += ph.z * g_xr;
-      gF[2] += g_xz;
-      gF[3] += ph.x * g_br - ph.z * g_bp;
-      gF[4] += ph.z * g_br + ph.x * g_bp;
-      gF[5] += g_bz;
-      gF[6] += ph.x * g_ar - ph.z * g_ap;
-      gF[7] += ph.z * g_ar + ph.x * g_ap;
-      gF[8] += g_az;
-      // FP32 over at least 32 directions, then FP64
-      if (nT >= 32 || d == dB || (iP & 7u) == 7u) {
+        if (((d - dA) & 7u) == 7u || d + 1u == dE) {
+          const float gF[kAG] = {ph.x * g_xr,
+                                 ph.z * g_xr,
+                                 g_xz,
+                                 ph.x * g_br - ph.z * g_bp,
+                                 ph.z * g_br + ph.x * g_bp,
+                                 g_bz,
+                                 ph.x * g_ar - ph.z * g_ap,
+                                 ph.z * g_ar + ph.x * g_ap,
+                                 g_az};
 #pragma unroll
-        for (int c = 0; c < kAG; ++c) {
-          gD[c] += (double)gF[c];
-          gF[c] = 0.f;
+          for (int c = 0; c < kAG; ++c) {
+            const df v = two_sum(sum[c][0][threadIdx.x], gF[c]);
+            sum[c][0][threadIdx.x] = v.hi;
+            sum[c][1][threadIdx.x] += v.lo;
+          }
+          g_xr = g_xz = g_br = g_bp = g_bz = g_ar = g_ap = g_az = 0.f;
         }
       }
     }
     if (valid) {
 #pragma unroll
       for (int c = 0; c < kAG; ++c)
-        a.gstep[((uint64_t)split * p.total_steps + base + s) * kAG + c] = gD[c];
+        a.gstep[((uint64_t)split * p.total_steps + base + s) * kAG + c] =
+            (double)sum[c][0][threadIdx.x] + (double)sum[c][1][threadIdx.x];
     }
   }
 }
