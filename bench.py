@@ -41,8 +41,6 @@ sys.path.insert(0, str(ROOT))
 METRIC = "Gpt·steps/s (spectral pts × track steps), mixed vs FP64 at ≤1e-5 rel err"
 UNIT = "Gpt·steps/s"
 FLOPS_PER_UNIT = 14      # far field, mixed: 2 FMUL + 6 FFMA per point-step
-ADJ_FLOPS_PER_UNIT = 22  # far adjoint: 8 FFMA (E and F sums) + 1 FMUL + 2 FFMA (rotation)
-NEAR_ADJ_FLOPS_PER_UNIT = 42  # near adjoint: 18 FFMA (R0, I1, R2 x 3) + rotation
 CANONICAL_FLOPS = 18     # the 3-component formulation's count
 
 
@@ -184,8 +182,26 @@ def executed_flops_per_unit(w):
     return 30 if w.args.get("mode", "far") == "near" else FLOPS_PER_UNIT
 
 
-# DRAM bytes of one launch of the dominant kernel on the full default
-# workloads, from single-pass ncu captures (dram__bytes_read.sum,
+def transform_flops(mode, n_omega, mean_steps, adjoint=False):
+    """Algorithmic FP32 flops per point-step where the sum is taken by
+    transforms (even frequency axes, no pinned shape): per (direction, step) 8
+    taps from degree-8 polynomials (72), 8 cells x 4 (far) or 12 (near) real
+    sums forward, x 8 or 18 in the adjoints, 2 flops each, and the step's
+    phase, amplitudes or chain rule (60, near 120; adjoints 150); per
+    (direction, band) one FFT of 5 M log2 M flops per complex field."""
+    far = mode == "far"
+    fields = (4 if far else 9) if adjoint else (2 if far else 6)
+    values = 150 if adjoint else (60 if far else 120)
+    bands = -(-n_omega // 512)
+    m = 128
+    while m < 2 * -(-n_omega // bands):
+        m *= 2
+    fft = fields * 5 * m * np.log2(m) * bands / max(1.0, mean_steps)
+    return float((bands * (72 + 32 * fields) + values + fft) / n_omega)
+
+
+# DRAM bytes of one launch of the term-by-term kernel on the full default
+# workloads (a pinned shape), from single-pass ncu captures (dram__bytes_read.sum,
 # dram__bytes_write.sum) of
 #   bench.py --workload W --steps 1 --warmup 1 --no-e2e --no-cpu --no-fp64 --no-graph --shape K L S N
 # with the shape the autotuner picks for that workload.  Most of it is the
@@ -489,8 +505,8 @@ def adjoint_main(args):
                                     ctypes.c_void_p(stream.cuda_stream)))
     peak = max(tf_s.value, tf_p.value)
     kern_avg = kern_ms.value / max(kern_n.value, 1)
-    fpu = ADJ_FLOPS_PER_UNIT if mode == "far" else NEAR_ADJ_FLOPS_PER_UNIT
-    kname = "adj_far_kernel" if mode == "far" else "nadj_kernel"
+    fpu = transform_flops(mode, nO, float(np.mean(lengths)), adjoint=True)
+    kname = "adj_interp_kernel" if mode == "far" else "nadj_interp_kernel"
     achieved = pt_steps * fpu / (kern_avg * 1e-3) / 1e12
     if rank == 0:
         line = {"metric": ("Gpt·steps/s through forward + backward of a spectrum misfit loss "
@@ -516,7 +532,9 @@ def adjoint_main(args):
                 "adjoint": {"forward_ms": fwd_ms, "backward_ms": bwd_ms,
                             "backward_over_forward": bwd_ms / fwd_ms,
                             "adjoint_kernel_ms": kern_avg, "forward_autotune": tune},
-                "e2e": None, "gpu_launches": 10 * args.steps,
+                # forward: records, sums, uneven axes, reduction; backward: records, two
+                # preparations, weights, fields, gradients, uneven axes, final
+                "e2e": None, "gpu_launches": 12 * args.steps,
                 "clocks": clocks.summary(),
                 "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
                              "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
@@ -642,23 +660,32 @@ def main():
     _lib.check(L.sr_probe_fp32_peak(ctypes.byref(tf_s), ctypes.byref(tf_p),
                                     ctypes.c_void_p(stream.cuda_stream)))
     kern_avg_ms = kern_ms.value / max(kern_n.value, 1)
-    fpu = flops_per_unit(w)
-    fpu_exec = executed_flops_per_unit(w)
+    pinned = args.shape is not None
+    fpu = (flops_per_unit(w) if pinned else
+           transform_flops(mode, w.args["grid"][-1][0], batch.total_steps / len(w.tracks)))
+    fpu_exec = executed_flops_per_unit(w) if pinned else fpu
     achieved = pt_steps * fpu / (kern_avg_ms * 1e-3) / 1e12
     achieved_exec = pt_steps * fpu_exec / (kern_avg_ms * 1e-3) / 1e12
     peak = max(tf_s.value, tf_p.value)
     clk = clocks.summary()
     kname = "near_mixed_kernel" if mode == "near" else "far_mixed_kernel"
-    traffic, traffic_src = launch_traffic(args.workload, args, len(w.tracks), shape)
+    traffic, traffic_src = None, "not captured at this size"
+    if pinned:
+        traffic, traffic_src = launch_traffic(args.workload, args, len(w.tracks), shape)
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak if peak else None,
                 "traffic": traffic, "traffic_unit": "bytes per launch",
                 "traffic_source": traffic_src,
                 "kernel": (f"{kname} ({shape['points_per_lane']} omega points per lane, "
-                           f"{shape['lanes_per_direction']} lanes per direction, 8 warps per CTA)"),
+                           f"{shape['lanes_per_direction']} lanes per direction, 8 warps per CTA)"
+                           if pinned else "fast_tracks_kernel (spreading and transforms, a lane "
+                           "per direction, 4 warps per CTA)"),
                 "kernel_ms_avg": kern_avg_ms,
                 "flops_per_unit": fpu,
-                "flops_per_unit_source": ("algorithmic work per point-step of the "
+                "flops_per_unit_source": (("per (direction, step) taps, cells and amplitudes, per "
+                                           "direction and track the FFTs, over the frequencies")
+                                          if not pinned else
+                                          "algorithmic work per point-step of the "
                                           "three-component formulation (rotation 2 FMUL + "
                                           "2 FFMA, accumulation 6 FFMA)"
                                           if mode == "far" else
@@ -766,7 +793,9 @@ def main():
                                  + ("exceed L2" if batch.total_steps * 64 > 129e6
                                     else "fit in L2"),
                            "parallelism": f"replicas x{ws} (tracks independent)"},
-                "e2e": e2e, "gpu_launches": 3 * args.steps,
+                "e2e": e2e,
+                # record pass, sums (one kernel or two), uneven axes, reduction
+                "gpu_launches": (graph.nodes()[0] if graph is not None else 4) * args.steps,
                 "launch": {"cuda_graph": graph is not None,
                            "graph_nodes": (dict(zip(("kernels", "nodes"), graph.nodes()))
                                            if graph is not None else None),

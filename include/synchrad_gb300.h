@@ -115,7 +115,8 @@ typedef struct sr_grid {
  *   out:  n_out device arrays (1, 3 or 6 by comp), element type double for
  *         SR_PREC_DOUBLE / SR_PREC_MIXED and float for SR_PREC_FLOAT*.
  *   workspace: device scratch of at least sr_workspace_bytes(...) bytes,
- *         256-byte aligned (NULL allowed when that size is 0).
+ *         256-byte aligned (NULL allowed when that size is 0); up to some GiB
+ *         where an even omega axis is summed by transforms.
  * Track and grid element types: SR_PREC_DOUBLE needs F64 tracks and grid,
  * SR_PREC_FLOAT* need F32 tracks and grid, SR_PREC_MIXED takes F64 or F32
  * tracks with an F64 grid.
@@ -203,7 +204,9 @@ int sr_config_get(const sr_tracks *tracks, const sr_grid *grid, int comp, int pr
  * lanes_per_direction (8/16/32), steps_per_stage (far: multiple of 32 in
  * [32, 512]) and track_subsets (0: default, at most 64) are used, the rest is
  * derived.  A shape whose shared memory would exceed a CTA's 227 KB is
- * refused with SR_ERR_INVALID. */
+ * refused with SR_ERR_INVALID.  The shape is that of the term-by-term kernels:
+ * a pinned problem is summed term by term, without the transforms that even
+ * omega axes are summed by otherwise. */
 int sr_config_set(const sr_tracks *tracks, const sr_grid *grid, int comp, int precision,
                   const sr_config *config);
 

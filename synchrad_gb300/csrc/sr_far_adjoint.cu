@@ -29,6 +29,10 @@
 // every direction, so each step's gradient is summed in registers and written
 // once: no atomics, no cross-lane reductions, a deterministic result.
 // Phases are recomputed, not stored.
+//
+// On even omega axes the sums over omega come from transforms instead
+// (adj_fields_kernel, adj_interp_kernel below); the walk keeps uneven axes,
+// fewer than 8 frequencies and snapshots a few steps apart.
 #include <algorithm>
 #include <cmath>
 
@@ -571,8 +575,10 @@ __global__ void __launch_bounds__(W * 32, 2) adj_far_kernel(AdjParams a) {
 // circle's first 8 cells again behind its last.
 // adj_interp_kernel: as below a CTA owns 256 steps of a track, a lane one step,
 // and loops over its directions; the records are turned into the plane of phi
-// once per phi.  Bound by the 16 cell loads of a (direction, step), 64 cycles
-// per warp and SM, and about as many for the arithmetic.
+// once per phi.  Bound by instructions (57 % of the issue slots at 16 warps an
+// SM, 128 registers) with the 16 cell loads of a (direction, step), 64 cycles
+// per warp and SM, beside them.  128 tracks of 2000 steps, 128 x 32 x 32 points:
+// 33.9 ms walking, 5.2 with the transforms (0.4 for the fields).
 // ------------------------------------------------------------------------
 
 // U of one point: summed over the snapshots k0..k1 that the steps enter.

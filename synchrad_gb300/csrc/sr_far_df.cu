@@ -30,6 +30,10 @@
 // step records of its subset directly (one record per lane per 32-step chunk,
 // coalesced) and broadcasts its per-(direction, step) setup through shared
 // memory.  Nothing waits on another CTA or on an asynchronous copy.
+//
+// On even omega axes the steps that include a whole band are summed by
+// transforms (df_spread_kernel, df_transform_kernel) and far_df_kernel adds the
+// others.
 #include <algorithm>
 #include <cmath>
 

@@ -36,6 +36,11 @@
 // shared memory.  Each (task group, track subset) item writes its own partial
 // spectrum; a final kernel adds the subsets in fixed order, so results are
 // deterministic.
+//
+// Even omega axes with steps enough are summed by transforms instead
+// (sr_fast_sum.cuh, rules and both sides' times in sr_fast_far.cu), uneven axes
+// by uneven_axis_kernel there; this kernel keeps short tracks on few directions,
+// snapshots a few steps apart, and pinned work shapes.
 #include <algorithm>
 #include <cmath>
 

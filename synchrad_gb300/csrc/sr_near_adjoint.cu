@@ -26,7 +26,9 @@
 // every 8 points, pairs of points in packed FP32), the U/W/Y constants of a
 // block of (screen point, omega) slots are built in shared memory from the
 // saved amplitudes, and a CTA owns 256 steps of one track and loops over
-// every screen point, so each step's gradient is written once.
+// every screen point, so each step's gradient is written once.  On even omega
+// axes the sums over omega come from transforms (nadj_fields_kernel,
+// nadj_interp_kernel below).
 #include <algorithm>
 #include <cmath>
 
@@ -528,7 +530,8 @@ __global__ void __launch_bounds__(W * 32, 2) nadj_kernel(NearAdjParams a) {
 // omega conj(U_k) and omega^2 conj(U_k), k = x, y, z; a cell holds the nine
 // complex values and one of padding (80 bytes, five 16-byte loads), and a
 // (screen point, step) takes 8 cells: bound by the 40 loads, 160 cycles per
-// warp and SM.
+// warp and SM.  24 tracks of 2500 to 3000 steps, 128 x 24 x 24 points, forward and
+// backward: 10.6 ms walking, 3.3 with the transforms.
 // ------------------------------------------------------------------------
 constexpr int kNAFields = 9, kNACell = 10;  // fields; float2 per cell
 

@@ -18,6 +18,8 @@
 //  * phasors, mask, compensated sums and FP64 results as in the far field
 //    (sr_far_mixed.cu), with K = 8 or 16 points per lane (six complex sums per
 //    point: 48 or 96 packed accumulator registers per lane).
+// As in the far field, even omega axes with steps enough are summed by
+// transforms and uneven ones by uneven_axis_kernel (sr_fast_sum.cuh).
 #include <algorithm>
 #include <cmath>
 
