@@ -180,6 +180,11 @@ __device__ __forceinline__ void adj_weight_final(const FarMixedParams &p, const 
   }
 }
 
+// Rounding of a step's retarded time difference formed in FP32, as a fraction of
+// the sum of its terms' sizes (which cancel by (gamma theta)^2 along the
+// motion): constants, differences, products and sums, 8 x 2^-24 at most, doubled.
+constexpr float kQuickErr = 1e-6f;
+
 // The transforms' cells (`cell` bytes each) of every (track, snapshot,
 // direction, omega band), of as many tracks at a time as 2 GiB hold; none
 // (batch 0) where one track's do not fit or the axis is too short to gain.

@@ -729,6 +729,7 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
       dy = (r1.x - e1.x) + (r1.y - e1.y);
       dz = (r1.z - e1.z) + (r1.w - e1.w);
     }
+    const float aq = kQuickErr * fabsf(dq), az = kQuickErr * fabsf(dz);
     // x, bbar, a: FP32 over up to 8 directions of a phi (rho, phi, z of each),
     // turned back and added as double-floats
 #pragma unroll
@@ -746,6 +747,7 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
       const float b_r = ph.x * r2.x + ph.z * r2.y, b_p = ph.x * r2.y - ph.z * r2.x;
       const float a_r = ph.x * r3.x + ph.z * r3.y, a_p = ph.x * r3.y - ph.z * r3.x;
       const float drho = ph.x * dx + ph.z * dy;
+      const float arho = kQuickErr * (fabsf(ph.x * dx) + fabsf(ph.z * dy));
       float g_xr = 0.f, g_xz = 0.f, g_br = 0.f, g_bp = 0.f, g_bz = 0.f, g_ar = 0.f, g_ap = 0.f,
             g_az = 0.f;
 #pragma unroll 1
@@ -758,11 +760,12 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
         const df s1 = two_sum(r0.x, p1.hi);
         const df s2 = two_sum(s1.hi, -p2.hi);
         const df tau = fast_two_sum(s2.hi, ((r0.y + p1.lo) - p2.lo) + (s1.lo + s2.lo));
-        // mask: certain where the FP32 difference leaves a 1e-3 margin, else from
-        // the double-float tau of both steps
+        // mask: certain where the FP32 difference with its error leaves a 1e-3
+        // margin, else from the double-float tau of both steps
         int mode = valid ? 0 : 1;  // 0: every frequency enters, 1: none, 2: some
         float et = 0.f, ep = 0.f, ft = 0.f, fp = 0.f;
-        const float quick = fabsf(dq + c1v.x * dz - c1v.y * drho);
+        const float quick = fabsf(dq + c1v.x * dz - c1v.y * drho) +
+                            (aq + (c1v.x * az + fabsf(c1v.y) * arho));
         if (__any_sync(0xffffffffu, valid && !(G.wabs_max * quick < 0.999f * kPiLo))) {
           float dt0 = tau.hi + tau.lo;
           if (sc > 0) {
