@@ -37,6 +37,13 @@ namespace {
 constexpr int kTaps = 8;
 constexpr int kFastList = 512;    // list entries per lane, fewer for short segments
 constexpr int kFastWarps = 4;     // warps per CTA
+// Steps that one circle of M FP32 cells takes.  A track laps its circle every M
+// steps or fewer and every lap adds to the same cells, so that their rounding
+// would grow with the track: the circle of a longer track is transformed and added
+// to compensated sums every 64 M steps, for one more transform each time.  On
+// resonance, 1e6 steps, 4 frequencies: 2.6e-5 of the spectrum (whole tracks
+// 4.8e-5) without, 3e-8 with.
+__host__ __device__ constexpr uint32_t fold_steps(uint32_t M) { return 64u * M; }
 // Per-warp shared memory: step records of the current chunk while spreading,
 // the transpose buffer of the FFT otherwise; the first field's outputs; the
 // cos/sin phi of the warp's directions.
@@ -879,19 +886,55 @@ __device__ __forceinline__ void emit_point(const FarMixedParams &p, uint32_t dir
   }
 }
 
+// The band sums xs, ys (undivided) of one pair of fields added to the
+// compensated sums `part` beside its circle, which they open where `add` is
+// false.
+template <bool NEAR>
+__device__ __forceinline__ void fold_pair(const FarMixedParams &p, const FastUnit<NEAR> &u,
+                                          const float2 *xs, const float2 *ys, float4 *part,
+                                          bool add, int lane) {
+  for (int m = lane; m < u.nb; m += 32) {
+    const df dv = df_from_double(p.fast.deconv[m - u.nb / 2 + kFastMaxBand / 2]);
+    const float2 x = xs[m], y = ys[m];
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f), l = o;
+    if (add) {
+      o = part[m];
+      l = part[p.fast.nb + m];
+    }
+    auto put = [&](float v, float &hi, float &lo) {
+      const float h = v * dv.hi;
+      const df s = two_sum(hi, h);
+      hi = s.hi;
+      lo += s.lo + (__fmaf_rn(v, dv.hi, -h) + v * dv.lo);
+    };
+    put(x.x, o.x, l.x);
+    put(x.y, o.y, l.y);
+    put(y.x, o.z, l.z);
+    put(y.y, o.w, l.w);
+    part[m] = o;
+    part[p.fast.nb + m] = l;
+  }
+}
+
 // The spectrum of one pair of fields, X and Y (band sums xs, ys, undivided),
-// added to the partial spectrum of track subset `sub`.
+// with the compensated sums of n_seg slices beside them (`held`: directions for
+// which the first slice's hold something, `dirty`: the others'), added to the
+// partial spectrum of track subset `sub`.
 template <bool NEAR>
 __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUnit<NEAR> &u,
                                           uint32_t dir, int d, int c, const float2 *xs,
                                           const float2 *ys, const float4 *part, int n_seg,
-                                          const uint32_t *dirty, uint32_t t, uint32_t ksnap, uint32_t sub, int lane) {
+                                          uint32_t held, const uint32_t *dirty, uint32_t t,
+                                          uint32_t ksnap, uint32_t sub, int lane) {
   const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
   const double wp = p.weight[t];
   const double wpdt2 = wp * p.dt * p.dt, wpdt = sqrt(wp) * p.dt;
   double *out = p.partial + (uint64_t)sub * p.n_out * p.n_snaps * P;
+  auto holds = [&](int i) {
+    return (((i ? dirty[(size_t)i * p.fast.n_dwb] : held) >> d) & 1u) != 0u;
+  };
   bool listed = p.save_A != nullptr;
-  for (int i = 0; i < n_seg; ++i) listed = listed || ((dirty[(size_t)i * p.fast.n_dwb] >> d) & 1u);
+  for (int i = 0; i < n_seg; ++i) listed = listed || holds(i);
   const uint64_t g0 = (uint64_t)u.j0 + (uint64_t)p.n_omega * dir;
   if (!listed && p.comp == SR_COMP_TOTAL) {
     // |A|^2 from the FP32 sums in double-float (exact products), scaled and
@@ -919,7 +962,7 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
     double Ar = (double)x.x * dv, Ai = (double)x.y * dv;
     double Br = (double)y.x * dv, Bi = (double)y.y * dv;
     for (int i = 0; i < n_seg; ++i)
-      if ((dirty[(size_t)i * p.fast.n_dwb] >> d) & 1u) {  // direct sums of the listed steps
+      if (holds(i)) {  // direct sums of the listed steps, circles folded before
         const float4 *q = part + (size_t)i * (p.fast.slice_bytes * p.fast.n_dwb / 16) + m;
         const float4 v = q[0], l = q[p.fast.nb];
         Ar += (double)v.x + (double)l.x;
@@ -931,24 +974,31 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
   }
 }
 
-// Transforms and emits the pairs [pr0, pr1) (pair = local direction x NP + c)
-// of one track, summing the circles of n_seg slices (slice stride in bytes).
+// Transforms the pairs [pr0, pr1) (pair = local direction x NP + c) of one
+// track, the circles of n_circ slices from `circles` on added up, and folds them
+// into the first slice's sums (`fold`) or emits them with the sums of n_seg
+// slices from `slice0` on.
 template <bool NEAR, int R1>
 __device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const FastUnit<NEAR> &u,
-                                                const unsigned char *slice0, int n_seg,
-                                                const uint32_t *dirty, FastSmem &sm, int pr0,
-                                                int pr1, uint32_t t, uint32_t ksnap,
+                                                const unsigned char *circles, int n_circ,
+                                                unsigned char *slice0, int n_seg, uint32_t held,
+                                                const uint32_t *dirty, bool fold, FastSmem &sm,
+                                                int pr0, int pr1, uint32_t t, uint32_t ksnap,
                                                 uint32_t sub, int lane) {
   constexpr int NP = NEAR ? 3 : 1;
   constexpr int NF = 32 / R1, M = 32 * R1;
   const uint32_t n_dirs = p.n_theta * p.n_phi;
   const size_t stride = p.fast.slice_bytes * p.fast.n_dwb;  // between a track's segments
-  const float4 *grid = (const float4 *)slice0;
-  const float4 *parts = grid + (size_t)NP * 32 * M;
+  const float4 *grid = (const float4 *)circles;
+  float4 *parts = (float4 *)slice0 + (size_t)NP * 32 * M;
   auto emit = [&](int pr, const float2 *xs, const float2 *ys) {
     const int d = pr / NP, c = pr % NP;
-    emit_pair<NEAR>(p, u, u.slot0 + d, d, c, xs, ys, parts + ((size_t)c * 32 + d) * 2 * p.fast.nb,
-                    n_seg, dirty, t, ksnap, sub, lane);
+    float4 *part = parts + ((size_t)c * 32 + d) * 2 * p.fast.nb;
+    if (fold)
+      fold_pair<NEAR>(p, u, xs, ys, part, (held >> d) & 1u, lane);
+    else
+      emit_pair<NEAR>(p, u, u.slot0 + d, d, c, xs, ys, part, n_seg, held, dirty, t, ksnap, sub,
+                      lane);
   };
   if constexpr (R1 == 32) {
     for (int pr = pr0; pr < pr1; ++pr) {
@@ -960,7 +1010,7 @@ __device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const F
         const float2 *g = (const float2 *)(grid + ((size_t)c * 32 + d) * M) + h;
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[0][i] = __ldcg(g + 2 * (32 * i + lane));
-        for (int sg = 1; sg < n_seg; ++sg) {
+        for (int sg = 1; sg < n_circ; ++sg) {
           const float2 *gs = g + (size_t)sg * (stride / 8);
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -988,7 +1038,7 @@ __device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const F
           x[2 * k][i] = make_float2(v.x, v.y);
           x[2 * k + 1][i] = make_float2(v.z, v.w);
         }
-        for (int sg = 1; sg < n_seg; ++sg) {
+        for (int sg = 1; sg < n_circ; ++sg) {
           const float4 *gs = g + (size_t)sg * (stride / 16);
 #pragma unroll
           for (int i = 0; i < R1; ++i) {
@@ -1021,6 +1071,14 @@ __device__ __forceinline__ void fast_tracks_of(const FarMixedParams &p, uint32_t
   } else {
     subset_range(p, sub, p.fast.n_sub, t0, t1);
   }
+}
+
+template <bool NEAR>
+__device__ __forceinline__ void clear_circles(const FastSlice<NEAR> &sl, uint32_t M, int lane) {
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t i = lane; i < FastSlice<NEAR>::NP * 32u * M; i += 32u) __stcg(sl.grid() + i, zero);
+  __threadfence();
+  __syncwarp();
 }
 
 // Whole tracks: a warp takes (32 directions x band, track subset) items from
@@ -1064,25 +1122,30 @@ fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
       SnapState snap;
       snap.init(it_start, it_end, snaps, p.n_snaps);
       if (snap.fire_it == SnapState::NEVER) continue;  // nothing of the track is written
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (uint32_t i = lane; i < (uint32_t)(NP * 32 * 32 * R1); i += 32u) __stcg(sl.grid() + i, zero);
-      __threadfence();
-      __syncwarp();
+      clear_circles<NEAR>(sl, 32 * R1, lane);
       bool dirty_l = false;
       const int64_t base = p.offsets[t];
-      uint32_t s = 0;
+      uint32_t s = 0, s_circle = 0;  // next step, first step of the circles
       // steps up to each snapshot's write; those due after the last body step
       // repeat the same amplitudes; steps after the last write enter nothing
       while (snap.fire_it != SnapState::NEVER) {
-        const uint32_t e = (uint32_t)min((int64_t)n_body, snap.fire_it + 1);
+        const uint32_t due = (uint32_t)min((int64_t)n_body, snap.fire_it + 1);
+        const bool fold = due > s && due - s_circle > fold_steps(32 * R1);
+        const uint32_t e = fold ? s_circle + fold_steps(32 * R1) : due;
         if (e > s) {
           dirty_l = spread_range<NEAR, R1 / 2>(p, u, sl, sm, base, it_start, s, e, dirty_l, lane);
           s = e;
         }
-        const uint32_t dirty = __ballot_sync(0xffffffffu, dirty_l);
-        transform_pairs<NEAR, R1>(p, u, sl.base, 1, &dirty, sm, 0, 32 * NP,
-                                  t, snap.k, sub, lane);
-        snap.advance(it_start, it_end, snaps, p.n_snaps);
+        const uint32_t held = __ballot_sync(0xffffffffu, dirty_l);
+        transform_pairs<NEAR, R1>(p, u, sl.base, 1, sl.base, 1, held, nullptr, fold, sm, 0,
+                                  32 * NP, t, snap.k, sub, lane);
+        if (fold) {
+          clear_circles<NEAR>(sl, 32 * R1, lane);
+          dirty_l = true;
+          s_circle = s;
+        } else {
+          snap.advance(it_start, it_end, snaps, p.n_snaps);
+        }
       }
     }
   }
@@ -1109,7 +1172,8 @@ __device__ __forceinline__ bool nth_snapshot(const FarMixedParams &p, uint32_t t
   return snap.fire_it != SnapState::NEVER;
 }
 
-template <bool NEAR, int R1>
+// FOLD: units of more than fold_steps(M).
+template <bool NEAR, int R1, bool FOLD>
 __global__ void __launch_bounds__(kFastWarps * 32, NEAR ? 2 : 3)
 fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
   if (*p.fast.uneven) return;
@@ -1147,14 +1211,21 @@ fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
   const FastSlice<NEAR> sl(f, unit);
   FastUnit<NEAR> u;
   unit_init<NEAR>(p, dwb, lane, sm, u);
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (uint32_t i = lane; i < NP * 32u * f.M; i += 32u) __stcg(sl.grid() + i, zero);
-  __threadfence();
-  __syncwarp();
+  clear_circles<NEAR>(sl, f.M, lane);
   bool dirty_l = false;
-  if (b > a)
+  while (b > a) {
+    const uint64_t e = FOLD ? min(b, a + fold_steps(32 * R1)) : b;
     dirty_l = spread_range<NEAR, R1 / 2>(p, u, sl, sm, p.offsets[t], p.it_start[t], (uint32_t)a,
-                                         (uint32_t)b, false, lane);
+                                         (uint32_t)e, dirty_l, lane);
+    a = e;
+    if (FOLD && a < b) {
+      const uint32_t held = __ballot_sync(0xffffffffu, dirty_l);
+      transform_pairs<NEAR, R1>(p, u, sl.base, 1, sl.base, 1, held, nullptr, true, sm, 0, 32 * NP,
+                                t, 0u, 0u, lane);
+      clear_circles<NEAR>(sl, f.M, lane);
+      dirty_l = true;
+    }
+  }
   const uint32_t dirty = __ballot_sync(0xffffffffu, dirty_l);
   if (lane == 0) f.dirty[unit] = dirty;
 }
@@ -1197,8 +1268,20 @@ fast_transform_kernel(const __grid_constant__ FarMixedParams p) {
       n_seg = n ? (int)((n + f.seg_steps - 1) / f.seg_steps) : 1;
     }
     unit0 = unit0 * f.n_dwb + dwb;
-    transform_pairs<NEAR, R1>(p, u, f.scratch + unit0 * f.slice_bytes, n_seg, f.dirty + unit0, sm,
-                              (int)(g * per) * NP, (int)((g + 1) * per) * NP, t, snap.k, sub, lane);
+    // circles of segments: plain sums of up to fold_steps(M) steps, as one
+    // circle would hold them
+    const int many =
+        f.seg_steps == 0 ? n_seg : (int)max(1u, fold_steps(32 * R1) / f.seg_steps);
+    unsigned char *slice0 = f.scratch + unit0 * f.slice_bytes;
+    uint32_t held = f.dirty[unit0];
+    for (int c0 = 0; c0 < n_seg; c0 += many) {
+      const bool fold = c0 + many < n_seg;
+      transform_pairs<NEAR, R1>(p, u, slice0 + (size_t)c0 * f.n_dwb * f.slice_bytes,
+                                min(many, n_seg - c0), slice0, n_seg, held, f.dirty + unit0, fold,
+                                sm, (int)(g * per) * NP, (int)((g + 1) * per) * NP, t, snap.k, sub,
+                                lane);
+      held = 0xffffffffu;
+    }
   }
 }
 
@@ -1394,10 +1477,13 @@ int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) 
     fast_tracks_kernel<NEAR, R1><<<l.slices / kFastWarps, threads, smem, s>>>(p);
     return cuda_fail(cudaGetLastError(), "fast sum launch");
   }
-  e = allow_smem((const void *)fast_spread_kernel<NEAR, R1>, smem);
+  const bool fold = l.seg_steps == 0 ? p.total_steps > (int64_t)fold_steps(l.M)
+                                     : l.seg_steps > fold_steps(l.M);
+  auto *spread = fold ? fast_spread_kernel<NEAR, R1, true> : fast_spread_kernel<NEAR, R1, false>;
+  e = allow_smem((const void *)spread, smem);
   if (e == cudaSuccess) e = allow_smem((const void *)fast_transform_kernel<NEAR, R1>, smem);
   if (e != cudaSuccess) return cuda_fail(e, "fast sum smem attribute");
-  fast_spread_kernel<NEAR, R1><<<l.slices / kFastWarps, threads, smem, s>>>(p);
+  spread<<<l.slices / kFastWarps, threads, smem, s>>>(p);
   const uint32_t items = l.n_dwb * (32u / l.dirs_per_warp) * l.n_sub * p.n_snaps;
   fast_transform_kernel<NEAR, R1><<<(items + kFastWarps - 1) / kFastWarps, threads, smem, s>>>(p);
   return cuda_fail(cudaGetLastError(), "fast sum launch");
