@@ -115,8 +115,10 @@ typedef struct sr_grid {
  *   out:  n_out device arrays (1, 3 or 6 by comp), element type double for
  *         SR_PREC_DOUBLE / SR_PREC_MIXED and float for SR_PREC_FLOAT*.
  *   workspace: device scratch of at least sr_workspace_bytes(...) bytes,
- *         256-byte aligned (NULL allowed when that size is 0); up to some GiB
- *         where an even omega axis is summed by transforms.
+ *         256-byte aligned (NULL allowed when that size is 0); up to 10 GiB
+ *         (SR_PREC_DF: 4 GiB and 4 bytes per 32 steps x 32 directions) where an
+ *         even omega axis is summed by transforms.  With less, down to
+ *         sr_workspace_bytes_min(...), the sum is taken term by term.
  * Track and grid element types: SR_PREC_DOUBLE needs F64 tracks and grid,
  * SR_PREC_FLOAT* need F32 tracks and grid, SR_PREC_MIXED takes F64 or F32
  * tracks with an F64 grid.
@@ -154,6 +156,14 @@ int sr_noalloc_status(void *stream);
  * precision, or a spheric comp on a near-field grid. */
 int64_t sr_workspace_bytes(const sr_tracks *tracks, const sr_grid *grid,
                            int comp, int precision);
+
+/* The least scratch sr_spectrum runs with: without the circles of the sums by
+ * transforms (up to 10 GiB, see sr_workspace_bytes).  Given less than
+ * sr_workspace_bytes but at least this, sr_spectrum sums term by term: the same
+ * results to the precision's tolerance, slower on even omega axes and the same on
+ * others, which the transforms do not serve. */
+int64_t sr_workspace_bytes_min(const sr_tracks *tracks, const sr_grid *grid,
+                               int comp, int precision);
 
 /* Synchronises `stream` and reads the kernels' status word from a workspace
  * used by sr_spectrum: SR_OK, or SR_ERR_TIMEOUT if a bounded wait expired. */
@@ -275,6 +285,9 @@ int sr_far_forward_saved(const sr_tracks *tracks, const sr_grid *grid, int comp,
                          void *const *out, float *saved_A, void *workspace,
                          size_t workspace_bytes, void *stream);
 int64_t sr_far_backward_workspace_bytes(const sr_tracks *tracks, const sr_grid *grid);
+/* The least scratch sr_far_backward runs with (without the cells of the sums by
+ * transforms, up to 2 GiB): it then walks the frequencies of every step. */
+int64_t sr_far_backward_workspace_bytes_min(const sr_tracks *tracks, const sr_grid *grid);
 int sr_far_backward(const sr_tracks *tracks, const sr_grid *grid, int comp,
                     const double *const *grad_out, const float *saved_A,
                     double *const *grad_track, double *grad_weight, void *workspace,
@@ -305,6 +318,8 @@ int sr_near_forward_saved(const sr_tracks *tracks, const sr_grid *grid, int comp
                           void *const *out, float *saved_A, void *workspace,
                           size_t workspace_bytes, void *stream);
 int64_t sr_near_backward_workspace_bytes(const sr_tracks *tracks, const sr_grid *grid);
+/* As sr_far_backward_workspace_bytes_min. */
+int64_t sr_near_backward_workspace_bytes_min(const sr_tracks *tracks, const sr_grid *grid);
 int sr_near_backward(const sr_tracks *tracks, const sr_grid *grid, int comp,
                      const double *const *grad_out, const float *saved_A,
                      double *const *grad_track, double *grad_weight, void *workspace,

@@ -102,7 +102,7 @@ class SrConfig(ctypes.Structure):
 
 
 EXPORTS = (
-    "sr_spectrum", "sr_workspace_bytes", "sr_workspace_status", "sr_last_error",
+    "sr_spectrum", "sr_workspace_bytes", "sr_workspace_bytes_min", "sr_workspace_status", "sr_last_error",
     "sr_version", "sr_far_total", "sr_far_cartesian_comps",
     "sr_far_cartesian_comps_complex", "sr_far_spheric_comps",
     "sr_far_spheric_comps_complex", "sr_near_total", "sr_near_cartesian_comps",
@@ -115,7 +115,8 @@ EXPORTS = (
     "sr_graph_nodes", "sr_graph_destroy", "sr_near_total_forward_saved",
     "sr_near_total_backward_workspace_bytes", "sr_near_total_backward",
     "sr_selftest_wait_timeout", "sr_near_forward_saved", "sr_near_backward_workspace_bytes",
-    "sr_near_backward",
+    "sr_near_backward", "sr_far_backward_workspace_bytes_min",
+    "sr_near_backward_workspace_bytes_min",
 )
 
 _lock = threading.Lock()
@@ -197,8 +198,14 @@ def _declare(L: ctypes.CDLL) -> None:
                        ctypes.POINTER(vp), vp, vp, ctypes.c_size_t, vp]
     L.sr_selftest_wait_timeout.restype = i32
     L.sr_selftest_wait_timeout.argtypes = [ctypes.c_int64, vp, vp]
-    L.sr_workspace_bytes.restype = ctypes.c_int64
-    L.sr_workspace_bytes.argtypes = [ctypes.POINTER(SrTracks), ctypes.POINTER(SrGrid), i32, i32]
+    for name in ("sr_workspace_bytes", "sr_workspace_bytes_min"):
+        f = getattr(L, name)
+        f.restype = ctypes.c_int64
+        f.argtypes = [ctypes.POINTER(SrTracks), ctypes.POINTER(SrGrid), i32, i32]
+    for kind in ("far", "near"):
+        f = getattr(L, f"sr_{kind}_backward_workspace_bytes_min")
+        f.restype = ctypes.c_int64
+        f.argtypes = [ctypes.POINTER(SrTracks), ctypes.POINTER(SrGrid)]
     L.sr_workspace_status.restype = i32
     L.sr_workspace_status.argtypes = [vp, vp]
     L.sr_last_error.restype = ctypes.c_char_p

@@ -103,6 +103,14 @@ def _spectrum_shape(layout: SpectrumLayout) -> tuple:
     return (nP, nT, nO) if layout.n_snaps == 1 else (layout.n_snaps, nP, nT, nO)
 
 
+def _backward_scratch(L, ts, gs, layout: SpectrumLayout) -> tuple:
+    args = (ctypes.byref(ts), ctypes.byref(gs))
+    need = getattr(L, f"sr_{layout.mode}_backward_workspace_bytes")
+    need_min = getattr(L, f"sr_{layout.mode}_backward_workspace_bytes_min")
+    return layout.workspace.get_for(lambda: need(*args), lambda: need_min(*args),
+                                    layout.grid.even)
+
+
 _SAVED_FLOATS = {"far": 4, "near": 8}  # per point and track
 
 
@@ -123,14 +131,14 @@ class TotalSpectrum(torch.autograd.Function):
                             dtype=torch.float32, device=x.device)
         df_fwd = layout.precision == "double-float"
         prec = _lib.SR_PREC_DF if df_fwd else _lib.SR_PREC_MIXED
-        need = L.sr_workspace_bytes(ctypes.byref(ts), ctypes.byref(gs), 0, prec)
-        if need < 0:
-            _lib.check(_lib.SR_ERR_INVALID if need == -1 else int(need))
-        ws = layout.workspace.get(max(int(need), 256))
+        args = (ctypes.byref(ts), ctypes.byref(gs), 0, prec)
+        ws, ws_bytes = layout.workspace.get_for(lambda: L.sr_workspace_bytes(*args),
+                                                lambda: L.sr_workspace_bytes_min(*args),
+                                                layout.grid.even)
         stream = ctypes.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
         fwd = getattr(L, f"sr_{layout.mode}_total_forward_saved" + ("_df" if df_fwd else ""))
         _lib.check(fwd(ctypes.byref(ts), ctypes.byref(gs), spec.data_ptr(), saved.data_ptr(),
-                       ws.data_ptr(), ctypes.c_size_t(int(need)), stream))
+                       ws.data_ptr(), ctypes.c_size_t(ws_bytes), stream))
         ctx.save_for_backward(*coords, wd, saved)
         ctx.layout = layout
         return spec
@@ -145,16 +153,12 @@ class TotalSpectrum(torch.autograd.Function):
         g = grad_spec.detach().contiguous().to(torch.float64)
         grads = [torch.empty_like(c) for c in coords]
         gw = torch.empty(layout.n_tracks, dtype=torch.float64, device=g.device)
-        need = getattr(L, f"sr_{layout.mode}_total_backward_workspace_bytes")(
-            ctypes.byref(ts), ctypes.byref(gs))
-        if need < 0:
-            _lib.check(_lib.SR_ERR_INVALID)
-        ws = layout.workspace.get(max(int(need), 256))
+        ws, ws_bytes = _backward_scratch(L, ts, gs, layout)
         ptrs = (ctypes.c_void_p * 6)(*[t.data_ptr() for t in grads])
         stream = ctypes.c_void_p(torch.cuda.current_stream(g.device).cuda_stream)
         bwd = getattr(L, f"sr_{layout.mode}_total_backward")
         _lib.check(bwd(ctypes.byref(ts), ctypes.byref(gs), g.data_ptr(), saved.data_ptr(), ptrs,
-                       gw.data_ptr(), ws.data_ptr(), ctypes.c_size_t(int(need)), stream))
+                       gw.data_ptr(), ws.data_ptr(), ctypes.c_size_t(ws_bytes), stream))
         return (*grads, gw, None)
 
 
@@ -184,20 +188,20 @@ class SpectrumComps(torch.autograd.Function):
         saved = torch.empty(layout.n_tracks * layout.n_snaps * P * _SAVED_FLOATS[layout.mode],
                             dtype=torch.float32, device=x.device)
         prec = _lib.SR_PREC_DF if layout.precision == "double-float" else _lib.SR_PREC_MIXED
-        need = L.sr_workspace_bytes(ctypes.byref(ts), ctypes.byref(gs), cid, prec)
-        if need < 0:
-            _lib.check(_lib.SR_ERR_INVALID if need == -1 else int(need))
-        ws = layout.workspace.get(max(int(need), 256))
+        args = (ctypes.byref(ts), ctypes.byref(gs), cid, prec)
+        ws, ws_bytes = layout.workspace.get_for(lambda: L.sr_workspace_bytes(*args),
+                                                lambda: L.sr_workspace_bytes_min(*args),
+                                                layout.grid.even)
         ptrs = (ctypes.c_void_p * 6)(*([o.data_ptr() for o in outs] + [None] * (6 - len(outs))))
         stream = ctypes.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
         if layout.mode == "far":
             rc = L.sr_far_forward_saved(ctypes.byref(ts), ctypes.byref(gs), cid, prec, ptrs,
                                         saved.data_ptr(), ws.data_ptr(),
-                                        ctypes.c_size_t(int(need)), stream)
+                                        ctypes.c_size_t(ws_bytes), stream)
         else:
             rc = L.sr_near_forward_saved(ctypes.byref(ts), ctypes.byref(gs), cid, ptrs,
                                          saved.data_ptr(), ws.data_ptr(),
-                                         ctypes.c_size_t(int(need)), stream)
+                                         ctypes.c_size_t(ws_bytes), stream)
         _lib.check(rc)
         ctx.save_for_backward(*coords, wd, saved)
         ctx.layout = layout
@@ -218,17 +222,13 @@ class SpectrumComps(torch.autograd.Function):
              for gr in grad_outs]
         grads = [torch.empty_like(c) for c in coords]
         gw = torch.empty(layout.n_tracks, dtype=torch.float64, device=dev)
-        need = getattr(L, f"sr_{layout.mode}_backward_workspace_bytes")(ctypes.byref(ts),
-                                                                         ctypes.byref(gs))
-        if need < 0:
-            _lib.check(_lib.SR_ERR_INVALID)
-        ws = layout.workspace.get(max(int(need), 256))
+        ws, ws_bytes = _backward_scratch(L, ts, gs, layout)
         gptrs = (ctypes.c_void_p * 6)(*([t.data_ptr() for t in g] + [None] * (6 - len(g))))
         tptrs = (ctypes.c_void_p * 6)(*[t.data_ptr() for t in grads])
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         bwd = getattr(L, f"sr_{layout.mode}_backward")
         _lib.check(bwd(ctypes.byref(ts), ctypes.byref(gs), cid, gptrs, saved.data_ptr(), tptrs,
-                       gw.data_ptr(), ws.data_ptr(), ctypes.c_size_t(int(need)), stream))
+                       gw.data_ptr(), ws.data_ptr(), ctypes.c_size_t(ws_bytes), stream))
         return (*grads, gw, None, None)
 
 

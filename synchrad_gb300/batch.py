@@ -273,6 +273,7 @@ class GridDevice:
     cos_phi: torch.Tensor
     form_factor: torch.Tensor | None = None
     L_screen: float = 0.0
+    even: bool = True           # False: the omega axis is known to be uneven
 
     def c_struct(self) -> _lib.SrGrid:
         g = _lib.SrGrid()
@@ -289,17 +290,32 @@ class GridDevice:
         return g
 
 
-def make_grid(mode, host_axes, n, dtype, device, form_factor=None, L_screen=0.0) -> GridDevice:
-    """host_axes: far (omega2pi, sinT, cosT, sinP, cosP), near (omega2pi, R, sinP, cosP)."""
+def even_axis(omega) -> bool:
+    """Whether the frequencies are evenly spaced to 1e-12, the test that the
+    kernels make on the device before they sum by transforms."""
+    w = np.asarray(omega, dtype=np.float64)
+    if w.size < 2:
+        return True
+    dw = (w[-1] - w[0]) / (w.size - 1)
+    if not np.isfinite(dw) or dw == 0.0:
+        return False
+    return bool(np.all(np.abs(w - (w[0] + dw * np.arange(w.size))) <= 1e-12 * np.abs(w) + 1e-300))
+
+
+def make_grid(mode, host_axes, n, dtype, device, form_factor=None, L_screen=0.0,
+              even=None) -> GridDevice:
+    """host_axes: far (omega2pi, sinT, cosT, sinP, cosP), near (omega2pi, R, sinP, cosP);
+    even: ``even_axis(omega2pi)`` where the caller knows it."""
+    even = even_axis(host_axes[0]) if even is None else even
     tdev = [torch.from_numpy(np.ascontiguousarray(a)).to(device) for a in host_axes]
     ff = (torch.from_numpy(np.ascontiguousarray(form_factor)).to(device)
           if form_factor is not None else None)
     tdt = torch.float32 if np.asarray(host_axes[0]).dtype == np.float32 else torch.float64
     if mode == "far":
         return GridDevice("far", tdt, tuple(n), tdev[0], tdev[1], tdev[2], tdev[3], tdev[4],
-                          ff, 0.0)
+                          ff, 0.0, even)
     return GridDevice("near", tdt, tuple(n), tdev[0], tdev[1], None, tdev[2], tdev[3], ff,
-                      float(L_screen))
+                      float(L_screen), even)
 
 
 def precision_id(dtype_name: str, native: bool) -> int:
@@ -329,6 +345,23 @@ class Workspace:
             self.buf = torch.empty(int(nbytes), dtype=torch.uint8, device=self.device)
         return self.buf
 
+    def get_for(self, need, need_min, even: bool = True) -> tuple:
+        """(buffer, its usable bytes) for a call that takes ``need()`` bytes and
+        runs, term by term, with ``need_min()`` of them: where the memory is not
+        there, and on an axis that is known to be uneven, which the transforms
+        do not serve."""
+        nbytes = int(need() if even else need_min())
+        if nbytes < 0:
+            _lib.check(nbytes)
+        try:
+            buf = self.get(nbytes)
+        except torch.OutOfMemoryError:
+            least = int(need_min())
+            if least >= nbytes:
+                raise
+            buf, nbytes = self.get(least), least
+        return buf, nbytes if buf is not None else 0
+
 
 def run_spectrum(batch: TrackBatch, grid: GridDevice, comp: str, precision: int,
                  outputs: list, workspace: Workspace | None = None, stream=None,
@@ -339,17 +372,16 @@ def run_spectrum(batch: TrackBatch, grid: GridDevice, comp: str, precision: int,
     if len(outputs) != _lib.N_OUT[cid]:
         raise ValueError(f"comp {comp!r} needs {_lib.N_OUT[cid]} output arrays")
     ts, gs = batch.c_struct(), grid.c_struct()
-    need = L.sr_workspace_bytes(ctypes.byref(ts), ctypes.byref(gs), cid, precision)
-    if need < 0:
-        _lib.check(_lib.SR_ERR_INVALID if need == -1 else int(need))
-    ws = (workspace or Workspace(outputs[0].device)).get(int(need))
+    args = (ctypes.byref(ts), ctypes.byref(gs), cid, precision)
+    ws, ws_bytes = (workspace or Workspace(outputs[0].device)).get_for(
+        lambda: L.sr_workspace_bytes(*args), lambda: L.sr_workspace_bytes_min(*args), grid.even)
     outs = (ctypes.c_void_p * 6)(*([o.data_ptr() for o in outputs] + [None] * (6 - len(outputs))))
     if stream is None:
         stream = torch.cuda.current_stream(outputs[0].device)
     sptr = ctypes.c_void_p(stream.cuda_stream)
     rc = L.sr_spectrum(ctypes.byref(ts), ctypes.byref(gs), cid, precision, outs,
                        ws.data_ptr() if ws is not None else None,
-                       ctypes.c_size_t(int(need) if ws is not None else 0), sptr)
+                       ctypes.c_size_t(ws_bytes), sptr)
     _lib.check(rc)
     if check_status and ws is not None:
         _lib.check(L.sr_workspace_status(ctypes.c_void_p(ws.data_ptr()), sptr))
@@ -408,17 +440,16 @@ class SpectrumGraph:
         if len(outputs) != _lib.N_OUT[cid]:
             raise ValueError(f"comp {comp!r} needs {_lib.N_OUT[cid]} output arrays")
         ts, gs = batch.c_struct(), grid.c_struct()
-        need = L.sr_workspace_bytes(ctypes.byref(ts), ctypes.byref(gs), cid, precision)
-        if need < 0:
-            _lib.check(_lib.SR_ERR_INVALID)
+        args = (ctypes.byref(ts), ctypes.byref(gs), cid, precision)
         self.workspace = workspace or Workspace(outputs[0].device)
-        ws = self.workspace.get(int(need))
+        ws, ws_bytes = self.workspace.get_for(lambda: L.sr_workspace_bytes(*args),
+                                              lambda: L.sr_workspace_bytes_min(*args), grid.even)
         outs = (ctypes.c_void_p * 6)(*([o.data_ptr() for o in outputs]
                                        + [None] * (6 - len(outputs))))
         h = ctypes.c_void_p()
         _lib.check(L.sr_graph_create(ctypes.byref(ts), ctypes.byref(gs), cid, precision, outs,
                                      ws.data_ptr() if ws is not None else None,
-                                     ctypes.c_size_t(int(need) if ws is not None else 0),
+                                     ctypes.c_size_t(ws_bytes),
                                      ctypes.byref(h)))
         self._keep = (batch, grid, outputs, ws)
         self.handle = h

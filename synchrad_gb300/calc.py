@@ -28,7 +28,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .batch import (TrackStream, Workspace, autotune, make_grid, pack_tracks, plan_chunks,
+from .batch import (TrackStream, Workspace, autotune, even_axis, make_grid, pack_tracks, plan_chunks,
                     precision_id, run_spectrum, snap_iterations)
 from .utils import Utilities
 
@@ -371,6 +371,7 @@ class SynchRad(Utilities):
         else:
             axes = (om, self.Args["radius"], np.sin(self.Args["phi"]), np.cos(self.Args["phi"]))
         self._host_axes = [np.ascontiguousarray(a) for a in axes]
+        self._even = even_axis(om)
 
     def _compile_kernels(self):
         """Loads the CUDA library (the OpenCL JIT of synchrad/calc.py:605-624)."""
@@ -399,7 +400,8 @@ class SynchRad(Utilities):
         L = self.Args.get("L_screen", 0.0) if self.Args["mode"] == "near" else 0.0
         self._grid_dev = make_grid(self.Args["mode"], self._host_axes, n, tdt, self.device,
                                    form_factor=np.ascontiguousarray(form_factor),
-                                   L_screen=self.dtype(L) if L is not None else 0.0)
+                                   L_screen=self.dtype(L) if L is not None else 0.0,
+                                   even=self._even)
 
     def _spectr_from_device(self, nSnaps):
         """synchrad/calc.py:573-577: to host, (nSnaps, nOmega, nTheta, nPhi)

@@ -187,7 +187,8 @@ constexpr float kQuickErr = 1e-6f;
 
 // The transforms' cells (`cell` bytes each) of every (track, snapshot,
 // direction, omega band), of as many tracks at a time as 2 GiB hold; none
-// (batch 0) where one track's do not fit or the axis is too short to gain.
+// (batch 0) where one track's do not fit, the axis is too short to gain or the
+// least scratch is asked for.
 struct AdjFields {
   uint32_t n_split;  // runs of directions whose gradients are summed apart
   uint32_t batch;    // tracks at a time
@@ -197,9 +198,9 @@ struct AdjFields {
 
 inline AdjFields adj_fields_layout(int64_t total_steps, uint32_t n_omega, uint64_t n_dirs,
                                    uint32_t n_tracks, uint32_t n_snaps, size_t cell,
-                                   int steps_per_item) {
+                                   int steps_per_item, bool least) {
   AdjFields l{1, 0, 0, 0, 0, 0};
-  if (n_omega < 8 || n_omega >= 65536u || n_tracks == 0 || n_snaps == 0 || total_steps <= 0)
+  if (least || n_omega < 8 || n_omega >= 65536u || n_tracks == 0 || n_snaps == 0 || total_steps <= 0)
     return l;
   l.n_bands = (n_omega + kFastMaxBand - 1) / kFastMaxBand;
   l.nb = (n_omega + l.n_bands - 1) / l.n_bands;

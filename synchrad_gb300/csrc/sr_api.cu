@@ -151,8 +151,9 @@ extern "C" const char *sr_last_error(void) { return g_err; }
 
 extern "C" int sr_version(void) { return 100; }
 
-extern "C" int64_t sr_workspace_bytes(const sr_tracks *t, const sr_grid *g, int comp,
-                                      int precision) {
+namespace {
+int64_t workspace_bytes_of(const sr_tracks *t, const sr_grid *g, int comp, int precision,
+                           bool least) {
   clear_error();
   if (!t || !g) return fail(SR_ERR_INVALID, "tracks and grid must not be NULL");
   if (g->mode != SR_MODE_FAR && g->mode != SR_MODE_NEAR)
@@ -167,15 +168,28 @@ extern "C" int64_t sr_workspace_bytes(const sr_tracks *t, const sr_grid *g, int 
   if (precision == SR_PREC_DF) {
     if (g->mode != SR_MODE_FAR)
       return fail(SR_ERR_UNSUPPORTED, "SR_PREC_DF evaluates the far field only");
-    const FarMixedConfig cfg =
+    FarMixedConfig cfg =
         far_df_choose(g->n_omega, g->n_theta * g->n_phi, t->n_tracks, device_sm_count());
+    cfg.direct = cfg.direct || least;
     return (int64_t)far_df_workspace(t->total_steps, P, nout, t->n_snaps ? t->n_snaps : 1, cfg);
   }
   if (precision != SR_PREC_MIXED) return 0;
-  const FarMixedConfig cfg = mixed_config(t, g, comp);
+  FarMixedConfig cfg = mixed_config(t, g, comp);
+  cfg.direct = cfg.direct || least;
   if (g->mode == SR_MODE_FAR)
     return (int64_t)far_mixed_workspace(t->total_steps, P, nout, t->n_snaps ? t->n_snaps : 1, cfg);
   return (int64_t)near_mixed_workspace(t->total_steps, P, nout, t->n_snaps ? t->n_snaps : 1, cfg);
+}
+}  // namespace
+
+extern "C" int64_t sr_workspace_bytes(const sr_tracks *t, const sr_grid *g, int comp,
+                                      int precision) {
+  return workspace_bytes_of(t, g, comp, precision, false);
+}
+
+extern "C" int64_t sr_workspace_bytes_min(const sr_tracks *t, const sr_grid *g, int comp,
+                                          int precision) {
+  return workspace_bytes_of(t, g, comp, precision, true);
 }
 
 extern "C" int sr_workspace_status(const void *workspace, void *stream) {

@@ -943,11 +943,11 @@ struct AdjLayout {
 };
 
 AdjLayout adj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t n_dirs,
-                     uint32_t n_tracks, uint32_t n_snaps) {
+                     uint32_t n_tracks, uint32_t n_snaps, bool least) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   AdjLayout l;
   l.w_chunks = adj_weight_chunks(P, n_tracks, device_sm_count());
-  l.fl = adj_fields_layout(total_steps, n_omega, n_dirs, n_tracks, n_snaps, 32, kASteps);
+  l.fl = adj_fields_layout(total_steps, n_omega, n_dirs, n_tracks, n_snaps, 32, kASteps, least);
   l.gstep = 256;
   l.records = l.gstep + up((size_t)total_steps * kAG * 8 * l.fl.n_split);
   l.gcst = l.records + up((size_t)total_steps * kRecBytes);
@@ -1018,12 +1018,22 @@ extern "C" int sr_far_total_forward_saved_df(const sr_tracks *t, const sr_grid *
                               workspace_bytes, stream);
 }
 
-extern "C" int64_t sr_far_backward_workspace_bytes(const sr_tracks *t, const sr_grid *g) {
+namespace {
+int64_t backward_bytes(const sr_tracks *t, const sr_grid *g, bool least) {
   if (!t || !g) return -1;
   const uint64_t n_dirs = (uint64_t)g->n_theta * g->n_phi;
   return (int64_t)adj_layout(t->total_steps, n_dirs * g->n_omega, g->n_omega, n_dirs,
-                             t->n_tracks, t->n_snaps)
+                             t->n_tracks, t->n_snaps, least)
       .total;
+}
+}  // namespace
+
+extern "C" int64_t sr_far_backward_workspace_bytes(const sr_tracks *t, const sr_grid *g) {
+  return backward_bytes(t, g, false);
+}
+
+extern "C" int64_t sr_far_backward_workspace_bytes_min(const sr_tracks *t, const sr_grid *g) {
+  return backward_bytes(t, g, true);
 }
 
 extern "C" int64_t sr_far_total_backward_workspace_bytes(const sr_tracks *t, const sr_grid *g) {
@@ -1064,7 +1074,10 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
     e = cudaMemsetAsync(grad_weight, 0, (size_t)t->n_tracks * 8, s);
     return e == cudaSuccess ? SR_OK : cuda_fail(e, "gradient reset");
   }
-  const AdjLayout lay = adj_layout(t->total_steps, P, g->n_omega, n_dirs, t->n_tracks, t->n_snaps);
+  // the walk along the frequencies where the scratch does not hold the cells
+  AdjLayout lay = adj_layout(t->total_steps, P, g->n_omega, n_dirs, t->n_tracks, t->n_snaps, false);
+  if (workspace_bytes < lay.total)
+    lay = adj_layout(t->total_steps, P, g->n_omega, n_dirs, t->n_tracks, t->n_snaps, true);
   if (!workspace || workspace_bytes < lay.total)
     return fail(SR_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", lay.total,
                 workspace_bytes);

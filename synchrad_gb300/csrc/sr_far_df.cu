@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(kDW * 32, 1)
 // 749 / 407.
 DfFast df_fast_layout(const FarMixedConfig &c, int64_t total_steps, uint32_t n_snaps) {
   DfFast f{};
-  if (n_snaps != 1 || c.n_omega < 16 || c.n_dirs == 0 || c.n_tracks == 0 || total_steps <= 0)
+  if (c.direct || n_snaps != 1 || c.n_omega < 16 || c.n_dirs == 0 || c.n_tracks == 0 || total_steps <= 0)
     return f;
   const uint64_t mean = (uint64_t)total_steps / c.n_tracks;
   if (mean < 160 || (mean < 256 && (uint64_t)c.n_omega * c.n_dirs * c.n_tracks < 200000)) return f;
@@ -1157,11 +1157,17 @@ size_t far_df_workspace(int64_t total_steps, uint64_t n_points, int n_out, uint3
   return df_layout(total_steps, n_points, n_out, n_snaps, cfg).total;
 }
 
-int launch_far_df(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size_t ws_bytes,
+int launch_far_df(FarMixedParams p, const FarMixedConfig &shape, void *ws, size_t ws_bytes,
                   cudaStream_t stream) {
   const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
   if (P == 0 || p.n_tracks == 0 || p.n_snaps == 0) return SR_OK;
-  const DfLayout lay = df_layout(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  // term by term where the scratch does not hold the transforms' circles
+  FarMixedConfig cfg = shape;
+  DfLayout lay = df_layout(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  if (ws_bytes < lay.total) {
+    cfg.direct = true;
+    lay = df_layout(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  }
   if (ws == nullptr || ws_bytes < lay.total)
     return fail(SR_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", lay.total, ws_bytes);
   if (((uintptr_t)ws & 255u) != 0) return fail(SR_ERR_WORKSPACE, "workspace not 256-byte aligned");

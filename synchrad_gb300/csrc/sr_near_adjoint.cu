@@ -836,11 +836,12 @@ struct NearAdjLayout {
 };
 
 NearAdjLayout nadj_layout(int64_t total_steps, uint64_t P, uint32_t n_omega, uint64_t n_scr,
-                          uint32_t n_tracks, uint32_t n_snaps) {
+                          uint32_t n_tracks, uint32_t n_snaps, bool least) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   NearAdjLayout l;
   l.w_chunks = adj_weight_chunks(P, n_tracks, device_sm_count());
-  l.fl = adj_fields_layout(total_steps, n_omega, n_scr, n_tracks, n_snaps, kNACell * 8, kNASteps);
+  l.fl = adj_fields_layout(total_steps, n_omega, n_scr, n_tracks, n_snaps, kNACell * 8, kNASteps,
+                           least);
   l.gstep = 256;
   l.records = l.gstep + up((size_t)total_steps * kNAG * 8 * l.fl.n_split);
   l.gcst = l.records + up((size_t)total_steps * kRecBytes);
@@ -900,12 +901,22 @@ extern "C" int64_t sr_near_total_backward_workspace_bytes(const sr_tracks *t, co
   return sr_near_backward_workspace_bytes(t, g);
 }
 
-extern "C" int64_t sr_near_backward_workspace_bytes(const sr_tracks *t, const sr_grid *g) {
+namespace {
+int64_t backward_bytes(const sr_tracks *t, const sr_grid *g, bool least) {
   if (!t || !g) return -1;
   const uint64_t n_scr = (uint64_t)g->n_theta * g->n_phi;
   return (int64_t)nadj_layout(t->total_steps, n_scr * g->n_omega, g->n_omega, n_scr,
-                              t->n_tracks, t->n_snaps)
+                              t->n_tracks, t->n_snaps, least)
       .total;
+}
+}  // namespace
+
+extern "C" int64_t sr_near_backward_workspace_bytes(const sr_tracks *t, const sr_grid *g) {
+  return backward_bytes(t, g, false);
+}
+
+extern "C" int64_t sr_near_backward_workspace_bytes_min(const sr_tracks *t, const sr_grid *g) {
+  return backward_bytes(t, g, true);
 }
 
 extern "C" int sr_near_total_backward(const sr_tracks *t, const sr_grid *g,
@@ -942,8 +953,10 @@ extern "C" int sr_near_backward(const sr_tracks *t, const sr_grid *g, int comp,
     e = cudaMemsetAsync(grad_weight, 0, (size_t)t->n_tracks * 8, s);
     return e == cudaSuccess ? SR_OK : cuda_fail(e, "gradient reset");
   }
-  const NearAdjLayout lay =
-      nadj_layout(t->total_steps, P, g->n_omega, n_scr, t->n_tracks, t->n_snaps);
+  // the walk along the frequencies where the scratch does not hold the cells
+  NearAdjLayout lay = nadj_layout(t->total_steps, P, g->n_omega, n_scr, t->n_tracks, t->n_snaps, false);
+  if (workspace_bytes < lay.total)
+    lay = nadj_layout(t->total_steps, P, g->n_omega, n_scr, t->n_tracks, t->n_snaps, true);
   if (!workspace || workspace_bytes < lay.total)
     return fail(SR_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", lay.total,
                 workspace_bytes);

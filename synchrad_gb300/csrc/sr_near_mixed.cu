@@ -624,11 +624,17 @@ size_t near_mixed_workspace(int64_t total_steps, uint64_t n_points, int n_out, u
   return (b + 255) / 256 * 256 + fast_workspace(l);
 }
 
-int launch_near_mixed(FarMixedParams p, const FarMixedConfig &cfg, void *ws, size_t ws_bytes,
+int launch_near_mixed(FarMixedParams p, const FarMixedConfig &shape, void *ws, size_t ws_bytes,
                       cudaStream_t stream) {
   const uint64_t P = (uint64_t)p.n_omega * p.n_theta * p.n_phi;
   if (P == 0 || p.n_tracks == 0 || p.n_snaps == 0) return SR_OK;
-  const size_t need = near_mixed_workspace(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  // term by term where the scratch does not hold the transforms' circles
+  FarMixedConfig cfg = shape;
+  size_t need = near_mixed_workspace(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  if (ws_bytes < need) {
+    cfg.direct = true;
+    need = near_mixed_workspace(p.total_steps, P, p.n_out, p.n_snaps, cfg);
+  }
   if (ws == nullptr || ws_bytes < need)
     return fail(SR_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, ws_bytes);
   if (((uintptr_t)ws & 255u) != 0) return fail(SR_ERR_WORKSPACE, "workspace not 256-byte aligned");
