@@ -185,6 +185,26 @@ __device__ __forceinline__ void adj_weight_final(const FarMixedParams &p, const 
 // motion): constants, differences, products and sums, 8 x 2^-24 at most, doubled.
 constexpr float kQuickErr = 1e-6f;
 
+// Cut steps of a warp (steps of which the phase limit takes a part of the axis):
+// a few are summed one after the other, 32 frequencies at a time over the lanes
+// (`each` instructions per step and 32 frequencies, 35 for the sums over the
+// lanes); many are walked side by side, a lane its own step (`walk` instructions
+// per frequency).  The counts are the loops' instructions; the measured times
+// cross where they do.
+__device__ __forceinline__ bool walk_cut(uint32_t cut, uint32_t n_omega, uint32_t each,
+                                         uint32_t walk) {
+  return (uint32_t)__popc(cut) * (35u + each * ((n_omega + 31u) / 32u)) > 60u + walk * n_omega;
+}
+
+// First and last frequency that any of the warp's cut steps includes (of none:
+// first > last).
+__device__ __forceinline__ void cut_span(bool is_cut, uint32_t range, int &first, int &last) {
+  const int jf = (int)(range & 0xffffu), jl = (int)(range >> 16);
+  const bool some = is_cut && jf <= jl;
+  first = __reduce_min_sync(0xffffffffu, some ? jf : 0x7fffffff);
+  last = __reduce_max_sync(0xffffffffu, some ? jl : -1);
+}
+
 // The transforms' cells (`cell` bytes each) of every (track, snapshot,
 // direction, omega band), of as many tracks at a time as 2 GiB hold; none
 // (batch 0) where one track's do not fit, the axis is too short to gain or the
