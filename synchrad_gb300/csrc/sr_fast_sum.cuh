@@ -37,13 +37,6 @@ namespace {
 constexpr int kTaps = 8;
 constexpr int kFastList = 512;    // list entries per lane, fewer for short segments
 constexpr int kFastWarps = 4;     // warps per CTA
-// Steps that one circle of M FP32 cells takes.  A track laps its circle every M
-// steps or fewer and every lap adds to the same cells, so that their rounding
-// would grow with the track: the circle of a longer track is transformed and added
-// to compensated sums every 64 M steps, for one more transform each time.  On
-// resonance, 1e6 steps, 4 frequencies: 2.6e-5 of the spectrum (whole tracks
-// 4.8e-5) without, 3e-8 with.
-__host__ __device__ constexpr uint32_t fold_steps(uint32_t M) { return 64u * M; }
 // Per-warp shared memory: step records of the current chunk while spreading,
 // the transpose buffer of the FFT otherwise; the first field's outputs; the
 // cos/sin phi of the warp's directions.
@@ -917,10 +910,10 @@ __device__ __forceinline__ void fold_pair(const FarMixedParams &p, const FastUni
 }
 
 // The spectrum of one pair of fields, X and Y (band sums xs, ys, undivided),
-// with the compensated sums of n_seg slices beside them (`held`: directions for
-// which the first slice's hold something, `dirty`: the others'), added to the
-// partial spectrum of track subset `sub`.
-template <bool NEAR>
+// with the compensated sums of n_seg slices beside them (`dirty`: the directions
+// for which they hold something, with FOLD `held` for the first slice), added to
+// the partial spectrum of track subset `sub`.
+template <bool NEAR, bool FOLD>
 __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUnit<NEAR> &u,
                                           uint32_t dir, int d, int c, const float2 *xs,
                                           const float2 *ys, const float4 *part, int n_seg,
@@ -931,7 +924,7 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
   const double wpdt2 = wp * p.dt * p.dt, wpdt = sqrt(wp) * p.dt;
   double *out = p.partial + (uint64_t)sub * p.n_out * p.n_snaps * P;
   auto holds = [&](int i) {
-    return (((i ? dirty[(size_t)i * p.fast.n_dwb] : held) >> d) & 1u) != 0u;
+    return (((FOLD && i == 0 ? held : dirty[(size_t)i * p.fast.n_dwb]) >> d) & 1u) != 0u;
   };
   bool listed = p.save_A != nullptr;
   for (int i = 0; i < n_seg; ++i) listed = listed || holds(i);
@@ -976,9 +969,9 @@ __device__ __forceinline__ void emit_pair(const FarMixedParams &p, const FastUni
 
 // Transforms the pairs [pr0, pr1) (pair = local direction x NP + c) of one
 // track, the circles of n_circ slices from `circles` on added up, and folds them
-// into the first slice's sums (`fold`) or emits them with the sums of n_seg
-// slices from `slice0` on.
-template <bool NEAR, int R1>
+// into the first slice's sums (FOLD and `fold`) or emits them with the sums of
+// n_seg slices from `slice0` on.
+template <bool NEAR, int R1, bool FOLD>
 __device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const FastUnit<NEAR> &u,
                                                 const unsigned char *circles, int n_circ,
                                                 unsigned char *slice0, int n_seg, uint32_t held,
@@ -994,10 +987,10 @@ __device__ __forceinline__ void transform_pairs(const FarMixedParams &p, const F
   auto emit = [&](int pr, const float2 *xs, const float2 *ys) {
     const int d = pr / NP, c = pr % NP;
     float4 *part = parts + ((size_t)c * 32 + d) * 2 * p.fast.nb;
-    if (fold)
+    if (FOLD && fold)
       fold_pair<NEAR>(p, u, xs, ys, part, (held >> d) & 1u, lane);
     else
-      emit_pair<NEAR>(p, u, u.slot0 + d, d, c, xs, ys, part, n_seg, held, dirty, t, ksnap, sub,
+      emit_pair<NEAR, FOLD>(p, u, u.slot0 + d, d, c, xs, ys, part, n_seg, held, dirty, t, ksnap, sub,
                       lane);
   };
   if constexpr (R1 == 32) {
@@ -1092,10 +1085,13 @@ __device__ __forceinline__ void clear_circles(const FastSlice<NEAR> &sl, uint32_
 // tracks of 4000 steps, 512 x 64 x 64 points: 85.8 ms term by term, 6.6 here;
 // near, 16 tracks of 8000 steps, 256 x 64 x 64: 83.8 and 13.7 ms.  1024 tracks,
 // 512 x 64 x 64: 2.71 s and 183 ms.
-template <bool NEAR, int R1>
+// FOLD: the tracks of more than fold_steps(M) steps (a launch of their own, only
+// where there can be any: with the fold in one kernel the spreading loop of all
+// tracks lost 1.5 % to the registers it takes).
+template <bool NEAR, int R1, bool FOLD>
 __global__ void __launch_bounds__(kFastWarps * 32, NEAR ? 2 : 3)
 fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
-  if (*p.fast.uneven) return;
+  if (*p.fast.uneven || (FOLD && !p.fast.uneven[1])) return;
   constexpr int NP = NEAR ? 3 : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1106,7 +1102,7 @@ fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
   const uint32_t n_items = f.n_dwb * f.n_sub;
   for (;;) {
     uint32_t item = 0;
-    if (lane == 0) item = atomicAdd(f.queue, 1u);
+    if (lane == 0) item = atomicAdd(f.queue + FOLD, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= n_items) return;
     const uint32_t sub = item / f.n_dwb;
@@ -1117,6 +1113,7 @@ fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
     fast_tracks_of(p, sub, t0, t1);
     for (uint32_t t = t0; t < t1; ++t) {
       const uint32_t n_body = track_body(p, t);
+      if (FOLD != (n_body > fold_steps(32 * R1))) continue;
       const uint32_t it_start = p.it_start[t], it_end = p.it_end[t];
       const uint32_t *snaps = p.snap_its + (size_t)t * p.snap_stride;
       SnapState snap;
@@ -1125,24 +1122,24 @@ fast_tracks_kernel(const __grid_constant__ FarMixedParams p) {
       clear_circles<NEAR>(sl, 32 * R1, lane);
       bool dirty_l = false;
       const int64_t base = p.offsets[t];
-      uint32_t s = 0, s_circle = 0;  // next step, first step of the circles
+      uint32_t s = 0;
       // steps up to each snapshot's write; those due after the last body step
       // repeat the same amplitudes; steps after the last write enter nothing
       while (snap.fire_it != SnapState::NEVER) {
         const uint32_t due = (uint32_t)min((int64_t)n_body, snap.fire_it + 1);
-        const bool fold = due > s && due - s_circle > fold_steps(32 * R1);
-        const uint32_t e = fold ? s_circle + fold_steps(32 * R1) : due;
+        const uint32_t full = (s & ~(fold_steps(32 * R1) - 1u)) + fold_steps(32 * R1);
+        const bool fold = FOLD && due > full;
+        const uint32_t e = fold ? full : due;
         if (e > s) {
           dirty_l = spread_range<NEAR, R1 / 2>(p, u, sl, sm, base, it_start, s, e, dirty_l, lane);
           s = e;
         }
         const uint32_t held = __ballot_sync(0xffffffffu, dirty_l);
-        transform_pairs<NEAR, R1>(p, u, sl.base, 1, sl.base, 1, held, nullptr, fold, sm, 0,
-                                  32 * NP, t, snap.k, sub, lane);
+        transform_pairs<NEAR, R1, FOLD>(p, u, sl.base, 1, sl.base, 1, held, &held, fold, sm, 0,
+                                        32 * NP, t, snap.k, sub, lane);
         if (fold) {
           clear_circles<NEAR>(sl, 32 * R1, lane);
           dirty_l = true;
-          s_circle = s;
         } else {
           snap.advance(it_start, it_end, snaps, p.n_snaps);
         }
@@ -1172,11 +1169,11 @@ __device__ __forceinline__ bool nth_snapshot(const FarMixedParams &p, uint32_t t
   return snap.fire_it != SnapState::NEVER;
 }
 
-// FOLD: units of more than fold_steps(M).
+// FOLD: the units of more than fold_steps(M).
 template <bool NEAR, int R1, bool FOLD>
 __global__ void __launch_bounds__(kFastWarps * 32, NEAR ? 2 : 3)
 fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
-  if (*p.fast.uneven) return;
+  if (*p.fast.uneven || (FOLD && !p.fast.uneven[1])) return;
   constexpr int NP = NEAR ? 3 : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1208,6 +1205,7 @@ fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
     if (a >= n && a > 0) return;  // no segment of the track
     b = min(n, a + f.seg_steps);
   }
+  if (FOLD != (b > a && b - a > fold_steps(32 * R1))) return;
   const FastSlice<NEAR> sl(f, unit);
   FastUnit<NEAR> u;
   unit_init<NEAR>(p, dwb, lane, sm, u);
@@ -1220,8 +1218,8 @@ fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
     a = e;
     if (FOLD && a < b) {
       const uint32_t held = __ballot_sync(0xffffffffu, dirty_l);
-      transform_pairs<NEAR, R1>(p, u, sl.base, 1, sl.base, 1, held, nullptr, true, sm, 0, 32 * NP,
-                                t, 0u, 0u, lane);
+      transform_pairs<NEAR, R1, true>(p, u, sl.base, 1, sl.base, 1, held, nullptr, true, sm, 0,
+                                      32 * NP, t, 0u, 0u, lane);
       clear_circles<NEAR>(sl, f.M, lane);
       dirty_l = true;
     }
@@ -1231,11 +1229,12 @@ fast_spread_kernel(const __grid_constant__ FarMixedParams p) {
 }
 
 // ... then, a few directions per warp and its track subset, the transforms of
-// the summed circles.
-template <bool NEAR, int R1>
+// the summed circles.  FOLD: of the tracks whose segments are more than one circle
+// may sum.
+template <bool NEAR, int R1, bool FOLD>
 __global__ void __launch_bounds__(kFastWarps * 32, 4)
 fast_transform_kernel(const __grid_constant__ FarMixedParams p) {
-  if (*p.fast.uneven) return;
+  if (*p.fast.uneven || (FOLD && !p.fast.uneven[1])) return;
   constexpr int NP = NEAR ? 3 : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1268,18 +1267,19 @@ fast_transform_kernel(const __grid_constant__ FarMixedParams p) {
       n_seg = n ? (int)((n + f.seg_steps - 1) / f.seg_steps) : 1;
     }
     unit0 = unit0 * f.n_dwb + dwb;
+    unsigned char *slice0 = f.scratch + unit0 * f.slice_bytes;
+    uint32_t held = FOLD ? f.dirty[unit0] : 0u;
     // circles of segments: plain sums of up to fold_steps(M) steps, as one
     // circle would hold them
     const int many =
         f.seg_steps == 0 ? n_seg : (int)max(1u, fold_steps(32 * R1) / f.seg_steps);
-    unsigned char *slice0 = f.scratch + unit0 * f.slice_bytes;
-    uint32_t held = f.dirty[unit0];
-    for (int c0 = 0; c0 < n_seg; c0 += many) {
-      const bool fold = c0 + many < n_seg;
-      transform_pairs<NEAR, R1>(p, u, slice0 + (size_t)c0 * f.n_dwb * f.slice_bytes,
-                                min(many, n_seg - c0), slice0, n_seg, held, f.dirty + unit0, fold,
-                                sm, (int)(g * per) * NP, (int)((g + 1) * per) * NP, t, snap.k, sub,
-                                lane);
+    if (FOLD != (n_seg > many)) continue;
+    for (int c0 = 0; c0 < (FOLD ? n_seg : 1); c0 += many) {
+      const bool fold = FOLD && c0 + many < n_seg;
+      transform_pairs<NEAR, R1, FOLD>(p, u, slice0 + (size_t)c0 * f.n_dwb * f.slice_bytes,
+                                      FOLD ? min(many, n_seg - c0) : n_seg, slice0, n_seg, held,
+                                      f.dirty + unit0, fold, sm, (int)(g * per) * NP,
+                                      (int)((g + 1) * per) * NP, t, snap.k, sub, lane);
       held = 0xffffffffu;
     }
   }
@@ -1470,22 +1470,26 @@ template <bool NEAR, int R1>
 int launch_fast_r(const FarMixedParams &p, const FastLayout &l, cudaStream_t s) {
   constexpr int smem = (int)sizeof(FastSmem) * kFastWarps;
   const unsigned threads = kFastWarps * 32;
-  cudaError_t e;
+  cudaError_t e = cudaSuccess;
+  auto launch = [&](auto *kernel, uint32_t blocks) {
+    if (e == cudaSuccess) e = allow_smem((const void *)kernel, smem);
+    if (e == cudaSuccess) kernel<<<blocks, threads, smem, s>>>(p);
+  };
+  // whether a track can have more steps than a circle takes
+  const bool longer = p.total_steps > (int64_t)fold_steps(l.M);
   if (!l.split) {
-    e = allow_smem((const void *)fast_tracks_kernel<NEAR, R1>, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "fast sum smem attribute");
-    fast_tracks_kernel<NEAR, R1><<<l.slices / kFastWarps, threads, smem, s>>>(p);
-    return cuda_fail(cudaGetLastError(), "fast sum launch");
+    launch(fast_tracks_kernel<NEAR, R1, false>, l.slices / kFastWarps);
+    if (longer) launch(fast_tracks_kernel<NEAR, R1, true>, l.slices / kFastWarps);
+  } else {
+    launch(fast_spread_kernel<NEAR, R1, false>, l.slices / kFastWarps);
+    if (longer && (l.seg_steps == 0 || l.seg_steps > fold_steps(l.M)))
+      launch(fast_spread_kernel<NEAR, R1, true>, l.slices / kFastWarps);
+    const uint32_t items = l.n_dwb * (32u / l.dirs_per_warp) * l.n_sub * p.n_snaps;
+    const uint32_t blocks = (items + kFastWarps - 1) / kFastWarps;
+    launch(fast_transform_kernel<NEAR, R1, false>, blocks);
+    if (longer && l.seg_steps) launch(fast_transform_kernel<NEAR, R1, true>, blocks);
   }
-  const bool fold = l.seg_steps == 0 ? p.total_steps > (int64_t)fold_steps(l.M)
-                                     : l.seg_steps > fold_steps(l.M);
-  auto *spread = fold ? fast_spread_kernel<NEAR, R1, true> : fast_spread_kernel<NEAR, R1, false>;
-  e = allow_smem((const void *)spread, smem);
-  if (e == cudaSuccess) e = allow_smem((const void *)fast_transform_kernel<NEAR, R1>, smem);
   if (e != cudaSuccess) return cuda_fail(e, "fast sum smem attribute");
-  spread<<<l.slices / kFastWarps, threads, smem, s>>>(p);
-  const uint32_t items = l.n_dwb * (32u / l.dirs_per_warp) * l.n_sub * p.n_snaps;
-  fast_transform_kernel<NEAR, R1><<<(items + kFastWarps - 1) / kFastWarps, threads, smem, s>>>(p);
   return cuda_fail(cudaGetLastError(), "fast sum launch");
 }
 

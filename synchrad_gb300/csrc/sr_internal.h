@@ -37,7 +37,9 @@ int launch_port(const PortParams &p, int mode, int comp, int dtype, bool native,
 // Arguments of the summation by transforms (sr_fast_sum.cuh), for evenly
 // spaced omega axes, and the test of the axis.
 struct FastParams {
-  unsigned int *uneven;  // set by the record pass when the axis is not evenly spaced
+  // [0] set by the record pass when the axis is not evenly spaced, [1] when a track
+  // has more steps than one circle takes
+  unsigned int *uneven;
   unsigned int *queue;   // next work item (zeroed per launch)
   double *deconv;        // 1 / transform of the spreading kernel, per frequency index
   float4 *twiddle;       // [M/32][32] exp(2 pi i a l / M): cos, sin, and their low parts
