@@ -16,7 +16,7 @@ struct AdjGlobals {
   float w0f, dwf;          // first omega and spacing in FP32
   float wabs_min, wabs_max;
   int uniform;             // omega axis uniform to 1e-12
-  int pad_;
+  float sin_max, omc_max;  // far field: largest |sin(theta)|, 1 - cos(theta)
 };
 
 // Omega table, axis uniformity and |omega| range (one block).
@@ -37,9 +37,16 @@ __device__ __forceinline__ void adj_globals(const FarMixedParams &p, float4 *wta
     amax = fmaxf(amax, aw);
   }
   __shared__ float smin[1024], smax[1024];
+  __shared__ unsigned int angle[2];
+  if (threadIdx.x < 2u) angle[threadIdx.x] = 0u;
   smin[threadIdx.x] = amin;
   smax[threadIdx.x] = amax;
   const int all_uni = __syncthreads_and(uni ? 1 : 0);
+  if (p.cos_theta != nullptr)  // not negative: ordered as integers, a NaN largest
+    for (uint32_t i = threadIdx.x; i < p.n_theta; i += blockDim.x) {
+      atomicMax(&angle[0], __float_as_uint(fabsf((float)p.sin_theta[i])));
+      atomicMax(&angle[1], __float_as_uint(fabsf((float)(1.0 - p.cos_theta[i]))));
+    }
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) {
       smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + o]);
@@ -57,7 +64,8 @@ __device__ __forceinline__ void adj_globals(const FarMixedParams &p, float4 *wta
     g.wabs_min = smin[0];
     g.wabs_max = smax[0];
     g.uniform = all_uni;
-    g.pad_ = 0;
+    g.sin_max = __uint_as_float(angle[0]);
+    g.omc_max = __uint_as_float(angle[1]);
     *glob = g;
   }
 }
@@ -146,13 +154,55 @@ __device__ __forceinline__ void adj_items(const FarMixedParams &p, int64_t *item
   if (threadIdx.x == blockDim.x - 1) item_off[n] = sums[blockDim.x - 1];
 }
 
-// The two one-block preparations in one launch (two blocks of 1024 threads).
+// Sets *many where the phase limit cuts more than 1/32 of 128 sampled
+// (direction, step) pairs (to FP32, for the choice of a kernel only).
+template <bool NEAR>
+__device__ __forceinline__ void adj_cut_share(const FarMixedParams &p, unsigned int *many) {
+  const uint32_t i = threadIdx.x, nT = p.n_theta;
+  constexpr uint32_t kSamples = 128;
+  const uint32_t t = (uint32_t)((uint64_t)(i % kSamples) * p.n_tracks / kSamples);
+  const uint32_t n = track_body(p, t);
+  bool cut = false;
+  if (i < kSamples && n > 1u) {
+    const uint32_t s = 1u + (i * 2654435761u >> 8) % (n - 1u), d = (i * 40503u) % (nT * p.n_phi);
+    const uint32_t iT = d % nT, iP = d / nT;
+    const float c0 = (float)(p.sin_theta[iT] * p.cos_phi[iP]);
+    const float c1 = (float)(p.sin_theta[iT] * p.sin_phi[iP]);
+    const int64_t g = p.offsets[t] + s;
+    auto ld = [&](const void *a, int64_t k) {
+      return p.track_f32 ? (double)((const float *)a)[k] : ((const double *)a)[k];
+    };
+    const double z = ld(p.z, g), dzd = z - ld(p.z, g - 1);
+    const float x = (float)ld(p.x, g), y = (float)ld(p.y, g), dz = (float)dzd;
+    const float dx = x - (float)ld(p.x, g - 1), dy = y - (float)ld(p.y, g - 1);
+    float nx = c0, ny = c1, omn;  // direction to the observer, 1 - n_z
+    if (NEAR) {
+      const float rx = c0 - x, ry = c1 - y, D = (float)(p.L_screen - z);
+      const float rho2 = rx * rx + ry * ry, r = sqrtf(rho2 + D * D);
+      nx = rx / r;
+      ny = ry / r;
+      omn = rho2 / (r * (r + D));
+    } else {
+      omn = (float)(1.0 - p.cos_theta[iT]);
+    }
+    const float adt = fabsf((float)(p.dt - dzd) + omn * dz - nx * dx - ny * dy);
+    const double wa = p.omega[0], wb = p.omega[p.n_omega - 1u];
+    const float wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
+    cut = !((float)fmax(fabs(wa), fabs(wb)) * adt < kPiLo) && !(wmin * adt > kPiHi);
+  }
+  if (__syncthreads_count(cut) > (int)kSamples / 32 && i == 0) *many = 1u;
+}
+
+// The one-block preparations in one launch (three blocks of 1024 threads).
+template <bool NEAR>
 __global__ void adj_setup_kernel(FarMixedParams p, float4 *wtab, AdjGlobals *glob,
-                                 int64_t *item_off, uint32_t steps_per_item) {
+                                 int64_t *item_off, uint32_t steps_per_item, unsigned int *many) {
   if (blockIdx.x == 0)
     adj_globals(p, wtab, glob);
-  else
+  else if (blockIdx.x == 1)
     adj_items(p, item_off, steps_per_item);
+  else if (p.fast.M != 0u)
+    adj_cut_share<NEAR>(p, many);
 }
 
 // Weight gradients are summed in two fixed-order stages: block (t, b) sums

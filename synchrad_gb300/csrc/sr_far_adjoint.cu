@@ -66,6 +66,7 @@ struct AdjParams {
   float4 *bandtab;             // [n_bands] centre frequency / 2 pi
   float2 *fields;              // transforms' cells of a batch of tracks (see below)
   uint32_t t_lo, t_hi;         // the batch
+  unsigned int *many_cut;      // whether the phase limit cuts many steps
   double *grad[6];             // x, y, z, ux, uy, uz  [total_steps]
   double *grad_w;              // [n_tracks]
   double *wpart;               // [n_tracks][w_chunks] partial weight gradients
@@ -678,13 +679,17 @@ __global__ void __launch_bounds__(kFastWarps * 32, 3) adj_fields_kernel(
   }
 }
 
+// WALK: with the walk of warps with many cut steps, taken where a sample of steps
+// says that there are some (beside it the loop of other steps loses 5 % to the
+// registers and the L1 cache that it takes).
+template <bool WALK>
 __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
     const __grid_constant__ AdjParams a) {
   const FarMixedParams &p = a.f;
-  if (!by_transform(p)) return;
+  if (!by_transform(p) || (*a.many_cut != 0u) != WALK) return;
   const FastParams &f = p.fast;
   __shared__ float sum[kAG][2][kASteps];
-  __shared__ float4 cut_u[kAW][32][2];  // U, omega U of 32 frequencies, for cut steps
+  __shared__ float4 cut_u[WALK ? kAW : 1][32][2];  // U, omega U of 32 frequencies, for cut steps
   const int lane = threadIdx.x & 31;
   const uint32_t nT = p.n_theta, n_dirs = nT * p.n_phi;
   const uint64_t P = (uint64_t)p.n_omega * n_dirs;
@@ -730,7 +735,11 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
       dy = (r1.x - e1.x) + (r1.y - e1.y);
       dz = (r1.z - e1.z) + (r1.w - e1.w);
     }
-    const float aq = kQuickErr * fabsf(dq), az = kQuickErr * fabsf(dz);
+    // below it the FP32 difference is certainly inside the limit for every
+    // frequency, with a 1e-3 margin, whatever its rounding
+    const float sure = 0.999f * kPiLo / G.wabs_max -
+                       kQuickErr * (fabsf(dq) + G.omc_max * fabsf(dz) +
+                                    G.sin_max * (fabsf(dx) + fabsf(dy)));
     // x, bbar, a: FP32 over up to 8 directions of a phi (rho, phi, z of each),
     // turned back and added as double-floats
 #pragma unroll
@@ -748,7 +757,6 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
       const float b_r = ph.x * r2.x + ph.z * r2.y, b_p = ph.x * r2.y - ph.z * r2.x;
       const float a_r = ph.x * r3.x + ph.z * r3.y, a_p = ph.x * r3.y - ph.z * r3.x;
       const float drho = ph.x * dx + ph.z * dy;
-      const float arho = kQuickErr * (fabsf(ph.x * dx) + fabsf(ph.z * dy));
       float g_xr = 0.f, g_xz = 0.f, g_br = 0.f, g_bp = 0.f, g_bz = 0.f, g_ar = 0.f, g_ap = 0.f,
             g_az = 0.f;
 #pragma unroll 1
@@ -761,13 +769,12 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
         const df s1 = two_sum(r0.x, p1.hi);
         const df s2 = two_sum(s1.hi, -p2.hi);
         const df tau = fast_two_sum(s2.hi, ((r0.y + p1.lo) - p2.lo) + (s1.lo + s2.lo));
-        // mask: certain where the FP32 difference with its error leaves a 1e-3
-        // margin, else from the double-float tau of both steps
+        // mask: certain where the FP32 difference is small enough, else from the
+        // double-float tau of both steps
         int mode = valid ? 0 : 1;  // 0: every frequency enters, 1: none, 2: some
         float et = 0.f, ep = 0.f, ft = 0.f, fp = 0.f;
-        const float quick = fabsf(dq + c1v.x * dz - c1v.y * drho) +
-                            (aq + (c1v.x * az + fabsf(c1v.y) * arho));
-        if (__any_sync(0xffffffffu, valid && !(G.wabs_max * quick < 0.999f * kPiLo))) {
+        const float quick = fabsf(dq + c1v.x * dz - c1v.y * drho);
+        if (__any_sync(0xffffffffu, valid && !(quick < sure))) {
           float dt0 = tau.hi + tau.lo;
           if (sc > 0) {
             const float4 e0 = __ldg(rp - kRecF4), e1 = __ldg(rp - kRecF4 + 1);
@@ -794,7 +801,7 @@ __global__ void __launch_bounds__(kASteps, 2) adj_interp_kernel(
                                               it_start, adt)
                         : 1u;
           uint32_t cut = __ballot_sync(0xffffffffu, mode == 2);
-          if (walk_cut(cut, p.n_omega, 45u, 23u)) {
+          if (WALK && walk_cut(cut, p.n_omega, 45u, 23u)) {
             cut = 0u;
             const int jf = (int)(mine & 0xffffu), jl = (int)(mine >> 16);
             int first, last;
@@ -1150,6 +1157,7 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   for (int i = 0; i < 6; ++i) a.grad[i] = grad_track[i];
   a.grad_w = grad_weight;
   a.n_split = lay.fl.n_split;
+  a.many_cut = (unsigned int *)(w + 96);  // in the zeroed status block
   a.bandtab = (float4 *)(w + lay.bandtab);
   a.fields = (float2 *)(w + lay.fields);
   if (lay.fl.batch) fast_tables_bind(a.f, lay.fl.n_bands, lay.fl.nb, lay.fl.M, w + lay.tables, w);
@@ -1162,7 +1170,8 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
   const int64_t step_blocks = std::max<int64_t>(
       16, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
   if (t->total_steps > 0) launch_far_prepass(a.f, (int)step_blocks, s);
-  adj_setup_kernel<<<2, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kASteps);
+  adj_setup_kernel<false><<<3, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kASteps,
+                                       a.many_cut);
   {
     const uint64_t work = std::max<uint64_t>(P, n_dirs);
     const uint64_t nb = std::min<uint64_t>((work + 255) / 256, (uint64_t)n_sm * 64);
@@ -1187,8 +1196,9 @@ extern "C" int sr_far_backward(const sr_tracks *t, const sr_grid *g, int comp,
     a.t_hi = std::min(t->n_tracks, lo + lay.fl.batch);
     launch_adj_fields(a, n_dirs, s);
     const int64_t most = items_max * lay.fl.n_split;
-    adj_interp_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm)),
-                        kASteps, 0, s>>>(a);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm));
+    adj_interp_kernel<false><<<blocks, kASteps, 0, s>>>(a);
+    adj_interp_kernel<true><<<blocks, kASteps, 0, s>>>(a);
   }
   adj_far_kernel<kAW><<<grid, kAW * 32, smem, s>>>(a);
   timing_record(s, false, &tok);

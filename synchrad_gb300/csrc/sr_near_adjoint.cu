@@ -66,6 +66,7 @@ struct NearAdjParams {
   float4 *bandtab;             // [n_bands] centre frequency / 2 pi
   float2 *fields;              // transforms' cells of a batch of tracks (see below)
   uint32_t t_lo, t_hi;         // the batch
+  unsigned int *many_cut;      // whether the phase limit cuts many steps
   double *grad[6];             // x, y, z, ux, uy, uz  [total_steps]
   double *grad_w;              // [n_tracks]
   double *wpart;               // [n_tracks][w_chunks] partial weight gradients
@@ -620,12 +621,14 @@ __global__ void __launch_bounds__(kFastWarps * 32, 3) nadj_fields_kernel(
   }
 }
 
+// WALK: as in the far field.
+template <bool WALK>
 __global__ void __launch_bounds__(kNASteps, 2) nadj_interp_kernel(
     const __grid_constant__ NearAdjParams a) {
   const FarMixedParams &p = a.f;
-  if (!by_transform(p)) return;
+  if (!by_transform(p) || (*a.many_cut != 0u) != WALK) return;
   const FastParams &f = p.fast;
-  __shared__ float4 cut_u[kNAW][32][2];  // U and omega of 32 frequencies, for cut steps
+  __shared__ float4 cut_u[WALK ? kNAW : 1][32][2];  // U and omega of 32 frequencies, for cut steps
   const int lane = threadIdx.x & 31;
   const uint32_t nR = p.n_theta, n_scr = nR * p.n_phi;
   const uint64_t P = (uint64_t)p.n_omega * n_scr;
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(kNASteps, 2) nadj_interp_kernel(
                                            it_start, adt)
                       : 1u;
         uint32_t cut = __ballot_sync(0xffffffffu, mode == 2);
-        if (walk_cut(cut, p.n_omega, 70u, 38u)) {
+        if (WALK && walk_cut(cut, p.n_omega, 70u, 38u)) {
           cut = 0u;
           const int jf = (int)(mine & 0xffffu), jl = (int)(mine >> 16);
           int first, last;
@@ -1041,6 +1044,7 @@ extern "C" int sr_near_backward(const sr_tracks *t, const sr_grid *g, int comp,
   for (int i = 0; i < 6; ++i) a.grad[i] = grad_track[i];
   a.grad_w = grad_weight;
   a.n_split = lay.fl.n_split;
+  a.many_cut = (unsigned int *)(w + 96);  // in the zeroed status block
   a.bandtab = (float4 *)(w + lay.bandtab);
   a.fields = (float2 *)(w + lay.fields);
   if (lay.fl.batch)
@@ -1054,7 +1058,8 @@ extern "C" int sr_near_backward(const sr_tracks *t, const sr_grid *g, int comp,
   const int64_t step_blocks = std::max<int64_t>(
       16, std::min<int64_t>((t->total_steps + 255) / 256, (int64_t)n_sm * 128));
   if (t->total_steps > 0) launch_near_prepass(a.f, (int)step_blocks, s);
-  adj_setup_kernel<<<2, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kNASteps);
+  adj_setup_kernel<true><<<3, 1024, 0, s>>>(a.f, a.wtab, a.glob, a.item_off, (uint32_t)kNASteps,
+                                       a.many_cut);
   {
     const uint64_t work = std::max<uint64_t>(P, n_scr);
     const uint64_t nb = std::min<uint64_t>((work + 255) / 256, (uint64_t)n_sm * 64);
@@ -1078,8 +1083,9 @@ extern "C" int sr_near_backward(const sr_tracks *t, const sr_grid *g, int comp,
     a.t_hi = std::min(t->n_tracks, lo + lay.fl.batch);
     launch_nadj_fields(a, n_scr, s);
     const int64_t most = items_max * lay.fl.n_split;
-    nadj_interp_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm)),
-                         kNASteps, 0, s>>>(a);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(most, 2 * (int64_t)n_sm));
+    nadj_interp_kernel<false><<<blocks, kNASteps, 0, s>>>(a);
+    nadj_interp_kernel<true><<<blocks, kNASteps, 0, s>>>(a);
   }
   nadj_kernel<kNAW><<<grid, kNAW * 32, smem, s>>>(a);
   timing_record(s, false, &tok);
