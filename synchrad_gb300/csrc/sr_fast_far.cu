@@ -8,6 +8,46 @@ namespace sr {
 
 namespace {
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+// Mean steps of a track from which the transforms are ahead of the term-by-term
+// kernel.  That one walks a track's steps one after the other at a cost that
+// falls with the number of (track, 32 directions) units once they fill the SMs;
+// the transforms pay for circles of M cells per unit, whatever its steps, and for
+// whole warps where there are fewer than 32 directions (`part`).  Term by term /
+// transforms, times of undulator batches of 20 to 1280 steps (each line: sizes,
+// ratio below and above its entry):
+//   far, 512 frequencies, 1024 directions, 64 tracks: 40 steps 0.72, 80 1.4
+//     64 directions, 500 tracks: 0.70 at 40, 1.03 at 80, 1000 units
+//     256 directions, 64 tracks: 0.80 at 80, 1.28 at 160, 512 units
+//     64 directions, 64 tracks: 0.91 at 160, 1.28 at 320, 128 units
+//     8 directions, 64 tracks: 0.69 at 320, 1.1 at 640
+//   far, 64 frequencies, same: 0.89 / 1.58 at 40 / 80, 0.97 / 1.54 at 80 / 160,
+//     0.93 / 1.34 at 80 / 160, 0.90 / 1.07 at 160 / 320, 0.87 / 1.08 at 160 / 320
+//   near, 16 frequencies: 1.37 at 40, 1.19 at 80, 0.86 / 1.06 at 80 / 160,
+//     0.64 at 320 and 0.99 at 1280, 0.71 / 1.24 at 640 / 1280
+//   near, 300 frequencies: 0.98 / 1.6 at 20 / 40, 0.72 / 1.29 at 20 / 40, 0.62 / 1.03
+//     at 20 / 40, 0.93 / 1.02 at 40 / 80, 0.68 / 0.90 at 640 / 1280
+uint64_t least_steps(bool near, uint32_t M, uint64_t units, bool part) {
+  if (!near) {
+    if (units >= 1824) return 64;
+    if (units >= 768) return M <= 512 ? 96 : 128;
+    if (units >= 140) {
+      if (part) return M > 512 ? 320 : units >= 400 ? 24 : 80;
+      return M <= 512 ? 112 : 128;
+    }
+    if (units >= 56) return M <= 512 ? 320 : part ? 800 : 256;
+    if (M <= 512) return M <= 256 ? 320 : part ? 200 : 160;
+    return part ? 640 : units >= 24 ? 400 : 320;
+  }
+  if (units >= 1216) return 32;
+  if (units >= 768) return M == 128 ? 128 : 64;
+  if (units >= 140) {
+    if (part) return M <= 256 ? 40 : M == 512 ? 200 : 400;
+    return M == 128 ? 280 : M <= 512 ? 64 : 96;
+  }
+  if (units >= 56) return M == 128 ? 1280 : M == 256 ? 400 : part ? 2 * (uint64_t)M : 200;
+  return M <= 512 ? 512 : 800;
+}
 }  // namespace
 
 FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
@@ -17,16 +57,6 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
       total_steps <= 0)
     return l;
   const uint64_t mean = (uint64_t)total_steps / c.n_tracks;
-  // The term-by-term kernel walks a track's steps one after the other, this
-  // sum splits them; below some hundred steps its extra launches and circles
-  // cost more than that.  Measured on one undulator track, 16 directions, 64
-  // frequencies (us, transforms / term by term): far 87 / 76 at 200 steps,
-  // 109 / 353 at 2000; near 128 / 92 and 263 / 440.  From 64 tracks on the
-  // transforms win at 200 steps too (147 / 243, 232 / 293 with 200 tracks),
-  // and in the far field with 129 to 256 frequencies (118 / 143), where the
-  // term-by-term work has doubled and the circles are still small.
-  const uint64_t least = near ? 512 : c.n_omega > 128 && c.n_omega <= 256 ? 160 : 320;
-  if (c.n_tracks < 64 && mean < least) return l;
   l.on = true;
   const int np = near ? 3 : 1;
   l.n_bands = (c.n_omega + kFastMaxBand - 1) / kFastMaxBand;
@@ -49,22 +79,29 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
   use_list(l.block + 32);
   const uint64_t resident = (uint64_t)c.n_sm * (near ? 2 : 3) * kFastWarps;
   const uint64_t units = (uint64_t)c.n_tracks * l.n_dwb;
+  const uint64_t least = least_steps(near, l.M, units, c.n_dirs < 32);
+  // few tracks: the rule of before the measurements by units, no lower
+  const uint64_t few = near ? 512 : c.n_omega > 128 && c.n_omega <= 256 ? 160 : 320;
+  if (mean < (c.n_tracks < 64 ? std::max(least, few) : least)) return FastLayout{};
   l.dirs_per_warp = std::max(1u, 512u / l.M);
   const uint64_t P = (uint64_t)c.n_omega * c.n_dirs;
   // Few (track, 32 directions) units: their steps are split in segments of a
   // block, after which a whole track's window is written out too, so that the
   // sums come out the same either way (a batch streamed in chunks
-  // gives what one call gives).  Larger circles take longer segments: each one
-  // is cleared and read once per segment (~4 TB/s) while a step takes ~0.4 us,
-  // shortest together at sqrt(steps x bytes / (4e12 x 0.4e-6)).  Where that
+  // gives what one call gives).  Larger circles and the near field's three take
+  // longer segments: each one is cleared and read once per segment (~4 TB/s) while a
+  // step takes ~0.4 us, shortest together at sqrt(steps x bytes / (4e12 x 0.4e-6))
+  // (near, 8 tracks of 1280 steps, 1024 directions, 16 frequencies: 0.63 of the
+  // term-by-term kernel's speed with segments of a block, 1.5 times it now).  Where that
   // leaves more than four units per resident warp or 4 GiB, segments grow for
   // the few long tracks that would not fill the SMs, else tracks stay whole.
   if (n_snaps == 1 && units <= resident) {
     const uint64_t all = (uint64_t)total_steps * l.n_dwb;
     uint64_t seg = l.block;
-    if (l.M >= 512) use_list(kFastList);
+    const bool larger = near || l.M >= 512;
+    if (larger) use_list(kFastList);
     const uint64_t room = (4ull << 30) / l.slice_bytes;
-    if (l.M >= 512)
+    if (larger)
       seg = std::max<uint64_t>(
           seg, (uint64_t)(std::sqrt((double)all * (2.0 * np * l.M * 512.0) / 1.6e6) / 128.0) * 128);
     bool split = true;
