@@ -154,43 +154,49 @@ __device__ __forceinline__ void adj_items(const FarMixedParams &p, int64_t *item
   if (threadIdx.x == blockDim.x - 1) item_off[n] = sums[blockDim.x - 1];
 }
 
+// Whether the phase limit cuts the axis inside at the i-th of kCutSamples
+// (direction, step) pairs, spread over the tracks (to FP32: for the choice of a
+// kernel only).
+constexpr uint32_t kCutSamples = 128;
+template <bool NEAR>
+__device__ __forceinline__ bool sampled_cut(const FarMixedParams &p, uint32_t i) {
+  if (i >= kCutSamples) return false;
+  const uint32_t t = (uint32_t)((uint64_t)i * p.n_tracks / kCutSamples), nT = p.n_theta;
+  const uint32_t n = track_body(p, t);
+  if (n < 2u) return false;
+  const uint32_t s = 1u + (i * 2654435761u >> 8) % (n - 1u), d = (i * 40503u) % (nT * p.n_phi);
+  const uint32_t iT = d % nT, iP = d / nT;
+  const float c0 = (float)(p.sin_theta[iT] * p.cos_phi[iP]);
+  const float c1 = (float)(p.sin_theta[iT] * p.sin_phi[iP]);
+  const int64_t g = p.offsets[t] + s;
+  auto ld = [&](const void *a, int64_t k) {
+    return p.track_f32 ? (double)((const float *)a)[k] : ((const double *)a)[k];
+  };
+  const double z = ld(p.z, g), dzd = z - ld(p.z, g - 1);
+  const float x = (float)ld(p.x, g), y = (float)ld(p.y, g), dz = (float)dzd;
+  const float dx = x - (float)ld(p.x, g - 1), dy = y - (float)ld(p.y, g - 1);
+  float nx = c0, ny = c1, omn;  // direction to the observer, 1 - n_z
+  if (NEAR) {
+    const float rx = c0 - x, ry = c1 - y, D = (float)(p.L_screen - z);
+    const float rho2 = rx * rx + ry * ry, r = sqrtf(rho2 + D * D);
+    nx = rx / r;
+    ny = ry / r;
+    omn = rho2 / (r * (r + D));
+  } else {
+    omn = (float)(1.0 - p.cos_theta[iT]);
+  }
+  const float adt = fabsf((float)(p.dt - dzd) + omn * dz - nx * dx - ny * dy);
+  const double wa = p.omega[0], wb = p.omega[p.n_omega - 1u];
+  const float wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
+  return !((float)fmax(fabs(wa), fabs(wb)) * adt < kPiLo) && !(wmin * adt > kPiHi);
+}
+
 // Sets *many where the phase limit cuts more than 1/32 of 128 sampled
-// (direction, step) pairs (to FP32, for the choice of a kernel only).
+// (direction, step) pairs.
 template <bool NEAR>
 __device__ __forceinline__ void adj_cut_share(const FarMixedParams &p, unsigned int *many) {
-  const uint32_t i = threadIdx.x, nT = p.n_theta;
-  constexpr uint32_t kSamples = 128;
-  const uint32_t t = (uint32_t)((uint64_t)(i % kSamples) * p.n_tracks / kSamples);
-  const uint32_t n = track_body(p, t);
-  bool cut = false;
-  if (i < kSamples && n > 1u) {
-    const uint32_t s = 1u + (i * 2654435761u >> 8) % (n - 1u), d = (i * 40503u) % (nT * p.n_phi);
-    const uint32_t iT = d % nT, iP = d / nT;
-    const float c0 = (float)(p.sin_theta[iT] * p.cos_phi[iP]);
-    const float c1 = (float)(p.sin_theta[iT] * p.sin_phi[iP]);
-    const int64_t g = p.offsets[t] + s;
-    auto ld = [&](const void *a, int64_t k) {
-      return p.track_f32 ? (double)((const float *)a)[k] : ((const double *)a)[k];
-    };
-    const double z = ld(p.z, g), dzd = z - ld(p.z, g - 1);
-    const float x = (float)ld(p.x, g), y = (float)ld(p.y, g), dz = (float)dzd;
-    const float dx = x - (float)ld(p.x, g - 1), dy = y - (float)ld(p.y, g - 1);
-    float nx = c0, ny = c1, omn;  // direction to the observer, 1 - n_z
-    if (NEAR) {
-      const float rx = c0 - x, ry = c1 - y, D = (float)(p.L_screen - z);
-      const float rho2 = rx * rx + ry * ry, r = sqrtf(rho2 + D * D);
-      nx = rx / r;
-      ny = ry / r;
-      omn = rho2 / (r * (r + D));
-    } else {
-      omn = (float)(1.0 - p.cos_theta[iT]);
-    }
-    const float adt = fabsf((float)(p.dt - dzd) + omn * dz - nx * dx - ny * dy);
-    const double wa = p.omega[0], wb = p.omega[p.n_omega - 1u];
-    const float wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
-    cut = !((float)fmax(fabs(wa), fabs(wb)) * adt < kPiLo) && !(wmin * adt > kPiHi);
-  }
-  if (__syncthreads_count(cut) > (int)kSamples / 32 && i == 0) *many = 1u;
+  const int cut = __syncthreads_count(sampled_cut<NEAR>(p, threadIdx.x));
+  if (32 * cut > (int)kCutSamples && threadIdx.x == 0) *many = 1u;
 }
 
 // The one-block preparations in one launch (three blocks of 1024 threads).

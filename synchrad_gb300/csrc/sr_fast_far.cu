@@ -58,6 +58,7 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
     return l;
   const uint64_t mean = (uint64_t)total_steps / c.n_tracks;
   l.on = true;
+  l.n_sm = (uint32_t)c.n_sm;
   const int np = near ? 3 : 1;
   l.n_bands = (c.n_omega + kFastMaxBand - 1) / kFastMaxBand;
   l.nb = (c.n_omega + l.n_bands - 1) / l.n_bands;
@@ -116,6 +117,12 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
       l.split = true;
       l.seg_steps = (uint32_t)std::min<uint64_t>(seg, 0xffffff00u);
       l.n_segs = (uint32_t)((uint64_t)total_steps / seg + c.n_tracks);
+      // lists that hold a whole segment, where they fit 4 GiB: one that fills up
+      // is emptied by its warp, which the others then wait for (near, 87 tracks of
+      // 600 steps, 5 a period, 140 directions, 512 frequencies: 14.5 ms, now 4.7)
+      const uint32_t fixed = l.list;
+      use_list((uint32_t)std::max<uint64_t>(fixed, std::min<uint64_t>(seg, 1u << 20) + 32));
+      if ((uint64_t)l.n_segs * l.n_dwb * l.slice_bytes > (4ull << 30)) use_list(fixed);
     }
   }
   if (n_snaps > 1) {
@@ -161,7 +168,9 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
 
 size_t fast_workspace(const FastLayout &l) {
   if (!l.on) return 0;
-  return up256(kFastTables) + up256((size_t)l.slices * 4) + (size_t)l.slices * l.slice_bytes;
+  return up256(kFastTables) + up256((size_t)l.slices * 4) +
+         (l.split ? up256((size_t)l.slices * 32 * sizeof(uint2)) : 0) +
+         (size_t)l.slices * l.slice_bytes;
 }
 
 void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char *base,
@@ -175,6 +184,9 @@ void fast_bind(FarMixedParams &p, const FastLayout &l, bool near, unsigned char 
   base += up256(kFastTables);
   f.dirty = (unsigned int *)base;
   base += up256((size_t)l.slices * 4);
+  f.work = (uint2 *)base;
+  f.n_work = (unsigned int *)(status + 200);
+  if (l.split) base += up256((size_t)l.slices * 32 * sizeof(uint2));
   f.scratch = base;
   f.slice_bytes = l.slice_bytes;
   f.n_dwb = l.n_dwb;

@@ -44,6 +44,8 @@ struct FastParams {
   double *deconv;        // 1 / transform of the spreading kernel, per frequency index
   float4 *twiddle;       // [M/32][32] exp(2 pi i a l / M): cos, sin, and their low parts
   unsigned int *dirty;   // per slice: directions whose direct sums hold something
+  uint2 *work;           // lists left to fast_lists_kernel: 32 slice + lane, entries
+  unsigned int *n_work;  // their number, and behind it the next to be taken
   unsigned char *scratch;
   unsigned long long slice_bytes;
   uint32_t n_bands, nb;  // omega bands and the frequencies of one
@@ -120,6 +122,7 @@ struct FastLayout {
   bool on;     // worth it for these sizes
   bool split;  // steps and transforms in two kernels (few tracks, one snapshot)
   uint32_t n_bands, nb, M, n_dwb, n_sub, n_segs, seg_steps, block, slices, dirs_per_warp, list;
+  uint32_t n_sm;
   size_t slice_bytes;
 };
 FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, int n_out,
