@@ -187,12 +187,17 @@ typedef struct sr_config {
   int32_t steps_per_stage;      /* step records per TMA stage (far field) */
   int32_t track_subsets;        /* tracks are split into this many subsets */
   int32_t ctas;                 /* CTAs of the persistent launch */
-  int32_t reserved;
+  int32_t transforms;           /* 1: even omega axes with steps enough are summed by
+                                   transforms, the shape serves the rest; 0: the shape
+                                   serves every even axis */
   double ms;                    /* time on the tuning sample (0: not timed) */
 } sr_config;
 
-/* Times candidate work shapes (points per lane and lanes per direction, then
- * steps per stage, then track subsets) with CUDA events on a sample of the
+/* Where the problem is summed by transforms, times them against the default
+ * term-by-term shape and keeps them unless that is faster; otherwise times
+ * candidate work shapes (points per lane and lanes per direction, then
+ * steps per stage, then track subsets; the subsets only on an uneven omega axis,
+ * whose kernel takes nothing else from the shape) with CUDA events on a sample of the
  * problem (its leading tracks, about budget_ms / 100 of work each run) and
  * caches the fastest for problems of exactly these sizes; later sr_spectrum
  * and sr_workspace_bytes calls for such problems use it (query the workspace
@@ -215,8 +220,9 @@ int sr_config_get(const sr_tracks *tracks, const sr_grid *grid, int comp, int pr
  * [32, 512]) and track_subsets (0: default, at most 64) are used, the rest is
  * derived.  A shape whose shared memory would exceed a CTA's 227 KB is
  * refused with SR_ERR_INVALID.  The shape is that of the term-by-term kernels:
- * a pinned problem is summed term by term, without the transforms that even
- * omega axes are summed by otherwise. */
+ * with config->transforms 0 the problem is summed term by term, without the
+ * transforms that even omega axes are summed by otherwise.  A config as
+ * sr_config_get or sr_autotune gave it takes the same path again. */
 int sr_config_set(const sr_tracks *tracks, const sr_grid *grid, int comp, int precision,
                   const sr_config *config);
 

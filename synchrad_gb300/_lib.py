@@ -93,12 +93,12 @@ class SrConfig(ctypes.Structure):
         ("steps_per_stage", ctypes.c_int32),
         ("track_subsets", ctypes.c_int32),
         ("ctas", ctypes.c_int32),
-        ("reserved", ctypes.c_int32),
+        ("transforms", ctypes.c_int32),
         ("ms", ctypes.c_double),
     ]
 
     def as_dict(self) -> dict:
-        return {k: getattr(self, k) for k, _ in self._fields_ if k != "reserved"}
+        return {k: getattr(self, k) for k, _ in self._fields_}
 
 
 EXPORTS = (

@@ -390,9 +390,9 @@ def run_spectrum(batch: TrackBatch, grid: GridDevice, comp: str, precision: int,
 def autotune(batch: TrackBatch, grid: GridDevice, comp: str = "total",
              precision: int = _lib.SR_PREC_MIXED, budget_ms: float = 3000.0,
              stream=None) -> dict:
-    """Tune the work shape of the persistent mixed-precision launch for this
-    batch's sizes (``sr_autotune``); later ``run_spectrum`` calls with the same
-    sizes use the choice.  Returns {'best': ..., 'default': ...} shapes with
+    """Tune the mixed-precision path for this batch's sizes (``sr_autotune``:
+    transforms or a work shape of the term-by-term launch); later ``run_spectrum``
+    calls with the same sizes use the choice.  Returns {'best': ..., 'default': ...} shapes with
     their times on the tuning sample."""
     L = _lib.lib()
     ts, gs = batch.c_struct(), grid.c_struct()
@@ -419,10 +419,11 @@ def current_config(batch: TrackBatch, grid: GridDevice, comp: str = "total",
 def set_config(batch: TrackBatch, grid: GridDevice, comp: str = "total",
                precision: int = _lib.SR_PREC_MIXED, points_per_lane: int = 32,
                lanes_per_direction: int = 32, steps_per_stage: int = 128,
-               track_subsets: int = 0) -> None:
-    """Pin a work shape for this batch's sizes (``sr_config_set``)."""
-    c = _lib.SrConfig(points_per_lane, lanes_per_direction, steps_per_stage, track_subsets, 0, 0,
-                      0.0)
+               track_subsets: int = 0, transforms: bool = False) -> None:
+    """Pin a work shape for this batch's sizes (``sr_config_set``); without
+    ``transforms`` the sum is taken term by term."""
+    c = _lib.SrConfig(points_per_lane, lanes_per_direction, steps_per_stage, track_subsets, 0,
+                      int(transforms), 0.0)
     ts, gs = batch.c_struct(), grid.c_struct()
     _lib.check(_lib.lib().sr_config_set(ctypes.byref(ts), ctypes.byref(gs), _lib.COMP_IDS[comp],
                                         precision, ctypes.byref(c)))

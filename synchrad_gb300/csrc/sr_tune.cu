@@ -8,7 +8,10 @@
 // times candidates with CUDA events on a bounded sample of the problem (the
 // leading tracks), by coordinate search: (K, L) first, then the stage size,
 // then the subsets, and caches the fastest per problem shape; sr_spectrum and
-// sr_workspace_bytes then use the cached choice for that shape.
+// sr_workspace_bytes then use the cached choice for that shape.  Where the problem
+// is summed by transforms, which have no free parameters, they are timed against
+// the default term-by-term shape, and shapes are searched only if that is faster;
+// on an uneven axis the subsets are all that its kernel takes from the shape.
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
@@ -66,8 +69,20 @@ void to_public(const FarMixedConfig &c, double ms, sr_config *o) {
   o->steps_per_stage = c.stage;
   o->track_subsets = c.n_sub;
   o->ctas = c.grid;
-  o->reserved = 0;
+  o->transforms = c.direct ? 0 : 1;
   o->ms = ms;
+}
+
+// The axis test of the record pass (fast_tables).
+bool even_axis(const std::vector<double> &w) {
+  const size_t n = w.size();
+  if (n < 2) return true;
+  const double dw = (w[n - 1] - w[0]) / (double)(n - 1);
+  if (!(std::fabs(dw) > 0.0) || !std::isfinite(dw)) return false;
+  for (size_t j = 0; j < n; ++j)
+    if (!(std::fabs(w[j] - (w[0] + (double)j * dw)) <= 1e-12 * std::fabs(w[j]) + 1e-300))
+      return false;
+  return true;
 }
 
 size_t workspace_of(const sr_tracks *t, const sr_grid *g, int n_out, const FarMixedConfig &c) {
@@ -166,7 +181,7 @@ extern "C" int sr_config_set(const sr_tracks *t, const sr_grid *g, int comp, int
                            c->track_subsets)
           : near_mixed_make(g->n_omega, n_dirs, t->n_tracks, device_sm_count(), K, L,
                             c->track_subsets);
-  cfg.direct = true;  // a shape is that of the term-by-term kernels
+  cfg.direct = c->transforms == 0;
   std::lock_guard<std::mutex> lk(g_tmu);
   g_cache[key_of(t, g, comp)] = cfg;
   return SR_OK;
@@ -211,10 +226,14 @@ extern "C" int sr_autotune(const sr_tracks *t, const sr_grid *g, int comp, int p
   // stream, which does not wait for non-blocking streams, and could read the
   // buffer before the copy landed.
   std::vector<int64_t> off(t->n_tracks + 1);
+  std::vector<double> om(g->n_omega);
   cudaError_t e = cudaMemcpyAsync(off.data(), t->offsets, off.size() * sizeof(int64_t),
                                   cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(om.data(), g->omega, om.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
-  if (e != cudaSuccess) return cuda_fail(e, "offsets read");
+  if (e != cudaSuccess) return cuda_fail(e, "offsets and frequencies read");
+  const bool even = even_axis(om);
   const double target = std::max(1e9, budget_ms / 100.0 * 2e9);
   uint32_t n_s = 1;
   while (n_s < t->n_tracks && (double)off[n_s] * (double)P < target) ++n_s;
@@ -222,16 +241,22 @@ extern "C" int sr_autotune(const sr_tracks *t, const sr_grid *g, int comp, int p
   ts.n_tracks = n_s;
   ts.total_steps = off[n_s];
   const bool full = (n_s == t->n_tracks);
+  const uint32_t ns = t->n_snaps;
+  // whether the problem, and the sample, are summed by transforms
+  const bool fast = even && fast_layout(dflt, !far, t->total_steps, n_out, ns).on;
 
   // candidates
   std::vector<FarMixedConfig> kl;
-  if (far) {
+  if (!even) {
+    // uneven_axis_kernel: its own points per lane
+  } else if (far) {
     for (int K : {32, 24, 16, 8})
       for (int L : {32, 16, 8}) {
         const uint64_t tile = (uint64_t)K * L;
         const uint64_t tiles = (g->n_omega + tile - 1) / tile;
         if ((double)(tiles * tile) > 1.34 * g->n_omega + 8.0 * L) continue;  // idle lanes
         kl.push_back(far_mixed_make(g->n_omega, n_dirs, n_s, n_sm, K, L, dflt.stage, 0));
+        kl.back().direct = true;
       }
   } else {
     for (int K : {16, 8})
@@ -240,11 +265,20 @@ extern "C" int sr_autotune(const sr_tracks *t, const sr_grid *g, int comp, int p
         const uint64_t tiles = (g->n_omega + tile - 1) / tile;
         if ((double)(tiles * tile) > 1.34 * g->n_omega + 8.0 * L) continue;
         kl.push_back(near_mixed_make(g->n_omega, n_dirs, n_s, n_sm, K, L, 0));
+        kl.back().direct = true;
       }
   }
-  const FarMixedConfig dflt_s =
+  FarMixedConfig dflt_s =
       far ? far_mixed_make(g->n_omega, n_dirs, n_s, n_sm, dflt.K, dflt.L, dflt.stage, 0)
           : near_mixed_make(g->n_omega, n_dirs, n_s, n_sm, dflt.K, dflt.L, 0);
+  dflt_s.direct = even && !fast;  // the sample takes the problem's path
+  const bool fast_s = fast && fast_layout(dflt_s, !far, ts.total_steps, n_out, ns).on;
+  if (fast && !fast_s) {
+    kl.clear();  // the sample has too few tracks for the transforms: nothing to compare
+  } else if (fast) {
+    kl.insert(kl.begin(), dflt_s);
+    kl.front().direct = true;
+  }
   kl.insert(kl.begin(), dflt_s);  // the default is always timed, first
 
   // scratch: outputs and the largest workspace any candidate can need
@@ -292,24 +326,28 @@ extern "C" int sr_autotune(const sr_tracks *t, const sr_grid *g, int comp, int p
     rc = consider(kl[i]);
     if (rc) break;
     if (i == 0) dflt_ms = best_ms;
+    if (fast && i == (fast_s ? 1u : 0u) && !best.direct) break;  // the transforms win
   }
+  const bool shapes = even && !(fast && !best.direct);
   // steps per stage
-  if (rc == SR_OK && far)
+  if (rc == SR_OK && far && shapes)
     for (int st : {64, 256}) {
       if (elapsed_ms() > budget_ms) break;
       FarMixedConfig c = far_mixed_make(g->n_omega, n_dirs, n_s, n_sm, best.K, best.L, st, 0);
+      c.direct = true;
       rc = consider(c);
       if (rc) break;
     }
   // track subsets
   int sub_scale_num = 1, sub_scale_den = 1;
-  if (rc == SR_OK) {
+  if (rc == SR_OK && (shapes || !even)) {
     const int h = best.n_sub;
     for (int v : {h / 2, h * 2}) {
       if (v < 1 || v > 64 || v > (int)n_s || v == h || elapsed_ms() > budget_ms) continue;
       FarMixedConfig c =
           far ? far_mixed_make(g->n_omega, n_dirs, n_s, n_sm, best.K, best.L, best.stage, v)
               : near_mixed_make(g->n_omega, n_dirs, n_s, n_sm, best.K, best.L, v);
+      c.direct = even;
       const int before = best.n_sub;
       rc = consider(c);
       if (rc) break;
@@ -340,6 +378,7 @@ extern "C" int sr_autotune(const sr_tracks *t, const sr_grid *g, int comp, int p
     chosen = far ? far_mixed_make(g->n_omega, n_dirs, t->n_tracks, n_sm, best.K, best.L,
                                   best.stage, nsub)
                  : near_mixed_make(g->n_omega, n_dirs, t->n_tracks, n_sm, best.K, best.L, nsub);
+    chosen.direct = best.direct;
   }
   {
     std::lock_guard<std::mutex> lk(g_tmu);
