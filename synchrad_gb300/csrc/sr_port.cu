@@ -86,9 +86,17 @@ __device__ __forceinline__ void sincos_of(float v, float &sn, float &cs) {
 
 // Which values a (direction, step) leaves in shared memory.
 //   V_TAU: time - n.x (far), time + r (near): the phase is omega times it
-//   V_RC, V_RS (FP64): exp(i d_omega tau)
+//   V_RC, V_RS (FP64, several points a lane): exp(i d_omega tau); FP32 near: 1/r
 //   V_A0..: far: the step's amplitude, near: (beta - n)/r and n/r^2
-enum { V_TAU = 0, V_RC = 1, V_RS = 2, V_A0 = 3, V_MAX = 9 };
+enum { V_TAU = 0, V_RC = 1, V_RS = 2 };
+template <bool F64, bool NEAR, int K>
+constexpr int first_amplitude() {
+  return F64 ? (K > 1 ? 3 : 1) : (NEAR ? 2 : 1);
+}
+template <bool F64, bool NEAR, int K>
+constexpr int shared_values() {
+  return first_amplitude<F64, NEAR, K>() + (NEAR ? 6 : 3);
+}
 
 // One warp's 32 / L directions, K consecutive omega points per lane.
 //
@@ -115,6 +123,8 @@ template <typename T, int COMP, bool NEAR, bool NATIVE, int K>
 __global__ void __launch_bounds__(128) port_kernel(PortParams p, int L) {
   using M = Math<T, NATIVE>;
   constexpr bool F64 = sizeof(T) == 8;
+  constexpr bool ROT = F64 && K > 1;  // phasors by rotation from the first point's
+  constexpr int V_A0 = first_amplitude<F64, NEAR, K>(), V_MAX = shared_values<F64, NEAR, K>();
   // total needs the two transverse components only (n.A is rounding noise,
   // ~1e-11 of A: 1e-22 of |A|^2)
   constexpr int NC = (!NEAR && COMP == 0 && F64) ? 2 : 3;
@@ -289,7 +299,7 @@ __global__ void __launch_bounds__(128) port_kernel(PortParams p, int L) {
             v[(V_A0 + 5) * 32] = rr * e2;
           }
           v[V_TAU * 32] = tau;
-          if constexpr (F64) {
+          if constexpr (ROT) {
             const T pr = dw * tau;
             const T e = fma(dw, tau, -pr);
             T sn, cs;
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(128) port_kernel(PortParams p, int L) {
               re[2][m] += A2 * cs; im[2][m] += A2 * sn;
             }
           };
-          if constexpr (F64) {
+          if constexpr (ROT) {
             const float dmax = dcoef * tf;  // bound of |delta|
             if (__all_sync(0xffffffffu, dmax < 1e-5f)) {
               // exp(i omega_0 tau) of the exact product, then rotations
@@ -408,6 +418,8 @@ __global__ void __launch_bounds__(128) port_kernel(PortParams p, int L) {
               if constexpr (NATIVE) {
                 sn = M::sn(phase);
                 cs = M::cs(phase);
+              } else if constexpr (F64) {
+                sincos(phase, &sn, &cs);
               } else {
                 sincos_of(phase, sn, cs);
               }
@@ -437,11 +449,17 @@ int launch_shape(const PortParams &p, int L, cudaStream_t s) {
   const uint64_t tiles = ((uint64_t)p.n_omega + (uint64_t)L * K - 1) / ((uint64_t)L * K);
   const uint64_t tasks = (((uint64_t)p.n_1 * p.n_phi + dpw - 1) / dpw) * tiles;
   // few tasks: one warp per CTA, so that they spread over the SMs
-  const int w = tasks >= 16ull * device_sm_count() ? 4 : 1;
-  const size_t smem = (size_t)w * dpw * (V_MAX * 32 + 1) * sizeof(T);
+  const int w = tasks >= 16ull * device_sm_count() && dpw <= 4 ? 4 : 1;
+  const size_t smem =
+      (size_t)w * dpw * (shared_values<sizeof(T) == 8, NEAR, K>() * 32 + 1) * sizeof(T);
   const uint64_t blocks = (tasks + w - 1) / w;
   if (blocks > 0x7fffffffull)
     return fail(SR_ERR_INVALID, "grid needs %llu blocks", (unsigned long long)blocks);
+  if (smem > 48u << 10) {
+    const cudaError_t e =
+        allow_smem((const void *)port_kernel<T, COMP, NEAR, NATIVE, K>, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "port smem attribute");
+  }
   port_kernel<T, COMP, NEAR, NATIVE, K><<<(unsigned)blocks, w * 32, smem, s>>>(p, L);
   return cuda_fail(cudaGetLastError(), "port kernel launch");
 }
@@ -453,6 +471,9 @@ int launch_shape(const PortParams &p, int L, cudaStream_t s) {
 // fullest SM: 16 per resident warp in FP64, at least the ~64 of a dependent
 // chain (FP32: 1/4 per warp, at least 6).  Measured, 64 omega points on 480
 // screen points: K = 2 with four warps per SM 23.8 ms, K = 4 with two 35.6 ms.
+// FP64 at one point per lane takes down to one lane per direction: 1 omega point on
+// 16384 directions, 1000 steps, far 14.2 ms with 8 lanes (one at work), 3.3 now;
+// near 16.0, 3.9 (a thread per point, without shared values: 10.4, 8.8).
 template <typename T, int COMP, bool NEAR, bool NATIVE>
 int launch_comp(const PortParams &p, cudaStream_t s) {
   constexpr bool F64 = sizeof(T) == 8;
@@ -463,13 +484,17 @@ int launch_comp(const PortParams &p, cudaStream_t s) {
   int bK = 1, bL = 32;
   double best = 1e300;
   for (int K = KM; K >= 1; K /= 2)
-    for (int L = 32; L >= 8; L /= 2) {
+    for (int L = 32; L >= (F64 && K == 1 ? 1 : 8); L /= 2) {
       const int dpw = 32 / L;
       const uint64_t tiles = ((uint64_t)p.n_omega + (uint64_t)L * K - 1) / ((uint64_t)L * K);
       const uint64_t tasks = ((dirs + dpw - 1) / dpw) * tiles;
       const double warps = (double)((tasks + n_sm - 1) / n_sm);
-      const double cycles = F64 ? std::max(16.0 * warps, 64.0) : std::max(0.25 * warps, 6.0);
-      const double cost = cycles * (K * c + seed + 4.0 * dpw);
+      // FP64 warps an SM holds, by their shared values
+      const double held = std::min(warps, 232448.0 / (dpw * (NEAR ? 9 : 6) * 32.0 * 8.0));
+      const double cycles =
+          F64 ? warps * std::max(16.0, 64.0 / held) : std::max(0.25 * warps, 6.0);
+      const double shared = F64 && K == 1 ? 3.0 : 4.0;
+      const double cost = cycles * (K * c + seed + shared * dpw);
       if (cost < best) {
         best = cost;
         bK = K;
