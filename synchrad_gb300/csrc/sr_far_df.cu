@@ -222,7 +222,8 @@ constexpr int kDSeries = 52;            // terms of I0 at kDBeta
 constexpr int kDSpreadWarps = 4;
 
 struct DfFast {
-  unsigned int *uneven;  // the axis is not even: everything term by term
+  // [0] the axis is not even, [1] sampled steps that the phase limit cuts
+  unsigned int *uneven;
   float4 *taps;          // [kDNodes + 1][kDRow] Taylor coefficients, pairs of taps
   double *deconv;        // [257] 1 / transform of the kernel, |index from the centre|
   double2 *twiddle;      // [M] exp(2 pi i k / M)
@@ -247,6 +248,17 @@ __device__ __forceinline__ uint64_t df_cell(const FarMixedParams &p, const DfFas
   return ((unit * 32u + dir % 32u) * f.M + j) * 4u;
 }
 
+// Whether the transforms are taken.  Where the |dphase| < pi rule cuts more than a
+// sixth of the sampled (direction, step) pairs, the cut steps' kernel would walk
+// most chunks anyway and everything is left to the term-by-term kernel (20 tracks,
+// 900 steps of which 9 make a period, 144 directions, 100 frequencies: 3.5 ms with the
+// transforms, 2.7 without; 40 tracks of 1200 steps, 16 a period, a quarter cut, 144
+// directions, 16 frequencies: 4.7 and 3.7).
+constexpr uint32_t kDSamples = 1024;
+__device__ __forceinline__ bool df_by_transform(const DfFast &f) {
+  return f.uneven[0] == 0u && 6u * f.uneven[1] <= kDSamples;
+}
+
 // Largest |omega| of a band.
 __device__ __forceinline__ float df_band_max(const FarMixedParams &p, const DfFast &f,
                                              uint32_t band) {
@@ -254,10 +266,35 @@ __device__ __forceinline__ float df_band_max(const FarMixedParams &p, const DfFa
   return (float)fmax(fabs(p.omega[j0]), fabs(p.omega[j1]));
 }
 
-// Tables, and whether the axis is even (one thread per entry).
-__global__ void df_fast_tables_kernel(FarMixedParams p, DfFast f, double c_last, double inv_i0) {
+// Tables, whether the axis is even (one thread per entry), and the sampled steps (the
+// first kDSamples threads).
+__global__ void __launch_bounds__(32) df_fast_tables_kernel(FarMixedParams p, DfFast f,
+                                                            const DfRecord *rec, double c_last,
+                                                            double inv_i0) {
   const uint32_t n = p.n_omega;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kDSamples) {  // whole warps
+    const uint32_t nT = p.n_theta, n_dirs = nT * p.n_phi;
+    const uint32_t t = (uint32_t)((uint64_t)i * p.n_tracks / kDSamples);
+    const uint32_t nb = track_body(p, t);
+    bool cut = false;
+    if (nb > 1) {
+      const uint32_t s = 1u + (i * 2654435761u >> 8) % (nb - 1u), d = (i * 40503u) % n_dirs;
+      const uint32_t iT = d % nT, iP = d / nT;
+      const double omc = 1.0 - p.cos_theta[iT], n0 = p.sin_theta[iT] * p.cos_phi[iP],
+                   n1 = p.sin_theta[iT] * p.sin_phi[iP];
+      const DfRecord &a = rec[p.offsets[t] + s], &b = rec[p.offsets[t] + s - 1];
+      const float adt = (float)fabs(df_tau(a.q, a.x, a.y, a.z, omc, n0, n1) -
+                                    df_tau(b.q, b.x, b.y, b.z, omc, n0, n1));
+      const double wa = p.omega[0], wb = p.omega[n - 1u];
+      const float wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
+      cut = !((float)fmax(fabs(wa), fabs(wb)) * adt < kPiLo) && !(wmin * adt > kPiHi);
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, cut);
+    if (threadIdx.x == 0 && m) atomicAdd(f.uneven + 1, (uint32_t)__popc(m));
+    return;
+  }
+  i -= kDSamples;
   const uint32_t n_tap = (kDNodes + 1) * kDTaps;
   if (i < n_tap) {
     // I0(beta sqrt(1 - (2x/W)^2)) = F(y), F(y) = sum y^k / k!^2, y quadratic in
@@ -298,35 +335,21 @@ __global__ void df_fast_tables_kernel(FarMixedParams p, DfFast f, double c_last,
   }
   const double w0 = p.omega[0], dw = (p.omega[n - 1] - w0) / (double)(n - 1);
   bool bad = !(fabs(dw) > 0.0) || !isfinite(dw);
-  for (uint32_t j = i; j < n; j += gridDim.x * blockDim.x) {
+  for (uint32_t j = i; j < n; j += gridDim.x * blockDim.x - kDSamples) {
     const double wj = p.omega[j];
     if (!(fabs(wj - (w0 + (double)j * dw)) <= 1e-12 * fabs(wj) + 1e-300)) bad = true;
   }
   if (bad) atomicOr(f.uneven, 1u);
 }
 
-// Where the |dphase| < pi rule cuts more than a quarter of 1024 sampled
-// (direction, step) pairs, the cut steps' kernel would walk most chunks anyway:
-// everything is left to it (20 tracks, 900 steps of which 9 make a period, 144
-// directions, 100 frequencies: 3.5 ms with the transforms, 2.7 without).
-__global__ void df_cut_share_kernel(FarMixedParams p, DfFast f, const DfRecord *rec) {
-  const uint32_t i = threadIdx.x, nT = p.n_theta, n_dirs = nT * p.n_phi;
-  const uint32_t t = (uint32_t)((uint64_t)i * p.n_tracks / blockDim.x);
-  const uint32_t n = track_body(p, t);
-  bool cut = false;
-  if (n > 1) {
-    const uint32_t s = 1u + (i * 2654435761u >> 8) % (n - 1u), d = (i * 40503u) % n_dirs;
-    const uint32_t iT = d % nT, iP = d / nT;
-    const double omc = 1.0 - p.cos_theta[iT], n0 = p.sin_theta[iT] * p.cos_phi[iP],
-                 n1 = p.sin_theta[iT] * p.sin_phi[iP];
-    const DfRecord &a = rec[p.offsets[t] + s], &b = rec[p.offsets[t] + s - 1];
-    const float adt = (float)fabs(df_tau(a.q, a.x, a.y, a.z, omc, n0, n1) -
-                                  df_tau(b.q, b.x, b.y, b.z, omc, n0, n1));
-    const double wa = p.omega[0], wb = p.omega[p.n_omega - 1u];
-    const float wmin = (wa <= 0.0) != (wb <= 0.0) ? 0.f : (float)fmin(fabs(wa), fabs(wb));
-    cut = !((float)fmax(fabs(wa), fabs(wb)) * adt < kPiLo) && !(wmin * adt > kPiHi);
-  }
-  if (__syncthreads_count(cut) > (int)blockDim.x / 4 && i == 0) atomicOr(f.uneven, 2u);
+// The circles cleared (a memset would write up to 4 GiB also where the cut steps take
+// the transforms off, and a warp alone its 32 circles too slowly).
+__global__ void __launch_bounds__(256) df_clear_kernel(const DfFast f, uint64_t n) {
+  if (!df_by_transform(f)) return;
+  double2 *c = reinterpret_cast<double2 *>(f.cells);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    c[i] = make_double2(0.0, 0.0);
 }
 
 // Adds a float to a double in memory; the conversion by integer operations
@@ -373,7 +396,7 @@ struct DfSpreadSmem {
 __global__ void __launch_bounds__(kDSpreadWarps * 32, 2)
     df_spread_kernel(const __grid_constant__ FarMixedParams p, const DfFast f,
                      const DfRecord *__restrict__ rec, const float4 *__restrict__ gtab) {
-  if (*f.uneven) return;
+  if (!df_by_transform(f)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   DfSpreadSmem &sm = *reinterpret_cast<DfSpreadSmem *>(smem_raw);
   for (int i = threadIdx.x; i < (kDNodes + 1) * kDRow; i += blockDim.x) sm.taps[i] = f.taps[i];
@@ -417,7 +440,6 @@ __global__ void __launch_bounds__(kDSpreadWarps * 32, 2)
   const int M = (int)f.M;
   const float Mf = (float)M;
   double *cells = f.cells + ((uint64_t)unit * 32u + lane) * (uint64_t)M * 4u;
-
   df2 acc[kDPairs][4];  // cells cur - 6 .. cur + 7 in pairs: theta re, im, phi re, im
 #pragma unroll
   for (int j = 0; j < kDPairs; ++j)
@@ -601,7 +623,7 @@ __global__ void __launch_bounds__(kDSpreadWarps * 32, 2)
 // from one buffer to the other, in FP64.
 __global__ void __launch_bounds__(128) df_transform_kernel(const __grid_constant__ FarMixedParams p,
                                                            const DfFast f) {
-  if (*f.uneven) return;
+  if (!df_by_transform(f)) return;
   extern __shared__ __align__(16) double2 tsm[];
   const uint32_t M = f.M, nT = p.n_theta, n_dirs = nT * p.n_phi;
   const uint32_t dir = blockIdx.x % n_dirs, tb = blockIdx.x / n_dirs;
@@ -656,12 +678,14 @@ struct DfAcc {  // pairs of points, 4 sums each: A_theta re/im, A_phi re/im
 };
 
 // FAST: the steps that include the whole band come from the transforms; this
-// kernel adds the cut ones and writes the comps (everything on an uneven axis).
+// kernel adds the cut ones and writes the comps.  Where the transforms are not
+// taken the other instance does everything.
 template <int K, bool FAST>
 __global__ void __launch_bounds__(kDW * 32, 1)
     far_df_kernel(FarMixedParams p, const DfRecord *__restrict__ rec,
                   const float4 *__restrict__ gtab, DfFast df_) {
   static_assert(K == 8, "K (more points per lane spill at 255 registers)");
+  if (df_.uneven != nullptr && df_by_transform(df_) != FAST) return;
   constexpr int KP = K / 2;
   __shared__ float4 tab[kTab];
   __shared__ DirConstDf dcs[kDW][kDMaxDpw];
@@ -720,7 +744,7 @@ __global__ void __launch_bounds__(kDW * 32, 1)
     wabs_max = fmaxf(wabs_max, (float)fabs(wm));
   }
   if (nv == 0) { wabs_min = 0.f; wabs_max = 0.f; }
-  const bool fast = FAST && *df_.uneven == 0u;
+  constexpr bool fast = FAST;
   const uint32_t band = FAST ? (uint32_t)min(j0, (int)nO - 1) / df_.nb : 0u;
   const float band_max = FAST ? df_band_max(p, df_, band) : 0.f;
   __syncthreads();  // table and direction constants
@@ -1056,9 +1080,8 @@ int launch_df_tables(const FarMixedParams &p, const DfFast &f, const DfRecord *r
   }
   double c_last = 1.0;
   for (int k = 1; k <= kDSeries; ++k) c_last /= (double)k * k;
-  const uint32_t n = (kDNodes + 1) * kDTaps + f.M + f.nb / 2 + 1;
-  df_fast_tables_kernel<<<(n + 31) / 32, 32, 0, s>>>(p, f, c_last, 1.0 / i0);
-  df_cut_share_kernel<<<1, 1024, 0, s>>>(p, f, rec);
+  const uint32_t n = kDSamples + (kDNodes + 1) * kDTaps + f.M + f.nb / 2 + 1;
+  df_fast_tables_kernel<<<(n + 31) / 32, 32, 0, s>>>(p, f, rec, c_last, 1.0 / i0);
   cudaError_t e = allow_smem((const void *)df_spread_kernel, (int)sizeof(DfSpreadSmem));
   if (e == cudaSuccess) e = allow_smem((const void *)df_transform_kernel, (int)(4 * 1024 * 16));
   return cuda_fail(e, "far_df smem attribute");
@@ -1068,8 +1091,10 @@ int launch_df_tables(const FarMixedParams &p, const DfFast &f, const DfRecord *r
 int launch_df_fast(const FarMixedParams &p, const DfFast &f, const DfRecord *rec,
                    const float4 *tab, size_t zero_bytes, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(f.any, 0, zero_bytes, s);
-  if (e != cudaSuccess) return cuda_fail(e, "circles reset");
-  const uint64_t units = (uint64_t)f.n_segs * f.n_dwb;
+  if (e != cudaSuccess) return cuda_fail(e, "cut flags reset");
+  const uint64_t units = (uint64_t)f.n_segs * f.n_dwb, pairs = units * 64u * f.M;
+  df_clear_kernel<<<(unsigned)std::min<uint64_t>((pairs + 255) / 256, 8ull * device_sm_count()),
+                    256, 0, s>>>(f, pairs);
   df_spread_kernel<<<(unsigned)((units + kDSpreadWarps - 1) / kDSpreadWarps), kDSpreadWarps * 32,
                      sizeof(DfSpreadSmem), s>>>(p, f, rec, tab);
   df_transform_kernel<<<p.n_tracks * p.n_theta * p.n_phi * f.n_bands, 128, 4 * f.M * 16, s>>>(p, f);
@@ -1222,9 +1247,10 @@ int launch_far_df(FarMixedParams p, const FarMixedConfig &shape, void *ws, size_
       q.it_end += t;
       q.snap_its += (size_t)t * p.snap_stride;
       if (q.save_A) q.save_A += (size_t)t * p.n_snaps * P * 4;
-      rc = launch_df_fast(q, f, rec, tab, lay.total - lay.any, stream);
+      rc = launch_df_fast(q, f, rec, tab, lay.cells - lay.any, stream);
       if (!rc) rc = launch_df_main<8, true>(q, rec, tab, f, stream);
     }
+    if (!rc) rc = launch_df_main<8, false>(p, rec, tab, f, stream);
   } else {
     rc = launch_df_main<8, false>(p, rec, tab, DfFast{}, stream);
   }

@@ -170,19 +170,51 @@ def test_gradient_with_least_scratch(mode, monkeypatch):
         assert 0 < np.linalg.norm(x - y) <= 6e-6 * np.linalg.norm(y)
 
 
+def _uneven(o):
+    return np.geomspace(o[0], o[-1], o.size)
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("mode", ["far", "near"])
-def test_uneven_axis_takes_the_least(mode):
+@pytest.mark.parametrize("mode,prec", [("far", "mixed"), ("near", "mixed"), ("far", "df")])
+def test_uneven_axis_takes_the_least(mode, prec):
+    """... and given everything (a caller that does not know its axis) the kernels
+    find it uneven and sum the same way, to the bit."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from synchrad_gb300 import batch as bt
-    batch, grid, n, _, _ = _problem(mode, axis=lambda o: np.geomspace(o[0], o[-1], o.size))
+    batch, grid, n, _, _ = _problem(mode, axis=_uneven)
+    pid = _lib.SR_PREC_MIXED if prec == "mixed" else _lib.SR_PREC_DF
     L = _lib.lib()
     ts, gs = batch.c_struct(), grid.c_struct()
-    args = (ctypes.byref(ts), ctypes.byref(gs), 0, _lib.SR_PREC_MIXED)
+    args = (ctypes.byref(ts), ctypes.byref(gs), 0, pid)
     ws = Workspace("cuda")
     out = torch.zeros((1,) + n[::-1], dtype=torch.float64, device="cuda")
-    bt.run_spectrum(batch, grid, "total", _lib.SR_PREC_MIXED, [out], workspace=ws)
+    bt.run_spectrum(batch, grid, "total", pid, [out], workspace=ws)
     assert ws.buf.numel() == L.sr_workspace_bytes_min(*args) < L.sr_workspace_bytes(*args)
     assert np.array_equal(out.cpu().numpy(),
-                          _raw(batch, grid, n, _lib.SR_PREC_MIXED, L.sr_workspace_bytes(*args))[1])
+                          _raw(batch, grid, n, pid, L.sr_workspace_bytes(*args))[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["far", "near"])
+def test_gradient_on_an_uneven_axis(mode):
+    """As above, for the saved forward and the backward."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from synchrad_gb300 import autograd as sag
+    _, _, n, axes, w = _problem(mode, axis=_uneven)
+
+    def gradients(known):
+        lay = sag.make_layout([900] * 4, w.time_step, axes, n, mode=mode,
+                              L_screen=w.L_screen or 0.0)
+        assert not lay.grid.even
+        lay.grid.even = not known
+        ts = [torch.tensor(np.concatenate([t[k] for t in w.tracks]), device="cuda",
+                           requires_grad=True) for k in range(6)]
+        wt = torch.ones(4, dtype=torch.float64, device="cuda", requires_grad=True)
+        sag.total_spectrum_fn(mode)(*ts, wt, lay).sum().backward()
+        return [t.grad.cpu().numpy() for t in ts + [wt]], lay.workspace.buf.numel()
+
+    (a, small), (b, big) = gradients(True), gradients(False)
+    assert small < big
+    assert all(np.array_equal(x, y) for x, y in zip(a, b))
