@@ -660,7 +660,7 @@ def main():
     _lib.check(L.sr_probe_fp32_peak(ctypes.byref(tf_s), ctypes.byref(tf_p),
                                     ctypes.c_void_p(stream.cuda_stream)))
     kern_avg_ms = kern_ms.value / max(kern_n.value, 1)
-    pinned = args.shape is not None
+    pinned = not shape["transforms"]  # summed term by term
     fpu = (flops_per_unit(w) if pinned else
            transform_flops(mode, w.args["grid"][-1][0], batch.total_steps / len(w.tracks)))
     fpu_exec = executed_flops_per_unit(w) if pinned else fpu

@@ -87,11 +87,13 @@ FastLayout fast_layout(const FarMixedConfig &c, bool near, int64_t total_steps, 
   l.dirs_per_warp = std::max(1u, 512u / l.M);
   const uint64_t P = (uint64_t)c.n_omega * c.n_dirs;
   // Few (track, 32 directions) units: their steps are split in segments of a
-  // block, after which a whole track's window is written out too, so that the
-  // sums come out the same either way (a batch streamed in chunks
-  // gives what one call gives).  Larger circles and the near field's three take
-  // longer segments: each one is cleared and read once per segment (~4 TB/s) while a
-  // step takes ~0.4 us, shortest together at sqrt(steps x bytes / (4e12 x 0.4e-6))
+  // block, after which a whole track's window is written out too, so that far-field
+  // sums of up to 128 frequencies come out the same either way where no step is cut
+  // (other sizes, and chunks of a batch that take another path than the whole,
+  // agree to the precision's tolerance only).  Larger circles and the near field's
+  // three take longer segments: each one is cleared and read once per segment
+  // (~4 TB/s) while a step takes ~0.4 us, shortest together at
+  // sqrt(steps x bytes / (4e12 x 0.4e-6))
   // (near, 8 tracks of 1280 steps, 1024 directions, 16 frequencies: 0.63 of the
   // term-by-term kernel's speed with segments of a block, 1.5 times it now).  Where that
   // leaves more than four units per resident warp or 4 GiB, segments grow for

@@ -322,9 +322,10 @@ __device__ void unit_init(const FarMixedParams &p, uint32_t dwb, int lane, FastS
 }
 
 // a x + b y for double-floats a, b, rounded once: the rounding of cos and sin
-// would be the same at every step of a phi and not average out (spectra of
-// betatron tracks 1.35e-6 from 64 bits with it, 1.19e-6 without; a phi's record
-// serves all its directions, so it costs no measurable time).
+// would be the same at every step of a phi and not average out (spectra of one
+// batch of 16 betatron tracks 1.35e-6 from 64 bits with it, 1.19e-6 without; ten
+// batches 0.8e-6 to 1.6e-6, mean 1.15e-6, term by term 1.22e-6).  A phi's record
+// serves all its directions, so it costs no measurable time.
 __device__ __forceinline__ float turned(float a, float al, float x, float b, float bl, float y) {
   const float p = a * x, q = b * y;
   const df s = two_sum(p, q);
@@ -367,7 +368,10 @@ __device__ __forceinline__ void stage_records(const FarMixedParams &p, int64_t g
   __syncwarp();
 }
 
-// 1/d to FP32 rounding: the hardware estimate and one Newton step.
+// 1/d to FP32 rounding: the hardware estimate and one Newton step, 5 % of the
+// spreading faster than __frcp_rn.  For every d of a binade and every estimate
+// within its 1 ulp of error the step ends at the correctly rounded value or, once
+// in a million, beside it (0.5 ulp + 1e-7).
 __device__ __forceinline__ float rcp_newton(float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
