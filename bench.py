@@ -532,9 +532,10 @@ def adjoint_main(args):
                 "adjoint": {"forward_ms": fwd_ms, "backward_ms": bwd_ms,
                             "backward_over_forward": bwd_ms / fwd_ms,
                             "adjoint_kernel_ms": kern_avg, "forward_autotune": tune},
-                # forward: records, sums, uneven axes, reduction; backward: records, two
-                # preparations, weights, fields, gradients, uneven axes, final
-                "e2e": None, "gpu_launches": 12 * args.steps,
+                # forward: records, sums, those of longer tracks, uneven axes, reduction;
+                # backward: records, two preparations, weights, fields, gradients in two
+                # variants, uneven axes, final (of one batch of cells: at least)
+                "e2e": None, "gpu_launches": 14 * args.steps,
                 "clocks": clocks.summary(),
                 "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
                              "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
