@@ -508,13 +508,12 @@ __device__ __forceinline__ uint32_t cut_interval(const FarMixedParams &p, uint32
 constexpr int kPairF = 20;  // floats a staged pair takes (14, padded)
 template <bool NEAR, int NK>
 __device__ __forceinline__ void drain_one(const FarMixedParams &p, FastSlice<NEAR> sl,
-                                          uint32_t slot0, uint32_t j0, int nb, int64_t base,
-                                          uint32_t it_start, int d, int n, bool add, float *pairs,
-                                          int lane) {
+                                          uint32_t slot0, uint32_t j0, int nb, double dw,
+                                          int64_t base, uint32_t it_start, int d, int n, bool add,
+                                          float *pairs, int lane) {
   constexpr int NP = NEAR ? 3 : 1;
   constexpr int KB = NK < 8 ? NK : 8;
   const double w0 = p.omega[0];
-  const double dw = (p.omega[p.n_omega - 1] - w0) / (double)(p.n_omega - 1);
   const double inv2pi = 0.15915494309189533577;
   const df f32 = df_from_double(32.0 * dw * inv2pi);
   const float w0f = (float)(w0 + (double)j0 * dw), dwf = (float)dw;
@@ -635,6 +634,12 @@ __device__ __forceinline__ void drain_one(const FarMixedParams &p, FastSlice<NEA
   __syncwarp();
 }
 
+// d_omega (an FP64 division: once for all lists that a warp empties; the lists'
+// kernel forms it per list, kept in registers there it cost 8 %).
+__device__ __forceinline__ double axis_step(const FarMixedParams &p) {
+  return (p.omega[p.n_omega - 1] - p.omega[0]) / (double)(p.n_omega - 1);
+}
+
 // The lists of every lane of the warp.
 template <bool NEAR, int NK>
 __device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<NEAR> sl,
@@ -643,10 +648,11 @@ __device__ __forceinline__ void drain_lists(const FarMixedParams &p, FastSlice<N
                                             int lane) {
   __syncwarp();
   const uint32_t old = __ballot_sync(0xffffffffu, dirty);
+  const double dw = axis_step(p);
 #pragma unroll 1
   for (uint32_t m = __ballot_sync(0xffffffffu, n_list > 0); m; m &= m - 1) {
     const int d = __ffs(m) - 1;
-    drain_one<NEAR, NK>(p, sl, slot0, j0, nb, base, it_start, d,
+    drain_one<NEAR, NK>(p, sl, slot0, j0, nb, dw, base, it_start, d,
                         __shfl_sync(0xffffffffu, n_list, d), (old >> d) & 1u,
                         reinterpret_cast<float *>(sm.rec), lane);
   }
@@ -1309,6 +1315,7 @@ fast_lists_kernel(const __grid_constant__ FarMixedParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const FastParams &f = p.fast;
   const uint32_t n_work = f.n_work[0];
+  if (n_work == 0u) return;
   for (;;) {
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(f.n_work + 1, 1u);
@@ -1320,8 +1327,8 @@ fast_lists_kernel(const __grid_constant__ FarMixedParams p) {
     const uint32_t j0 = dwb % f.n_bands * f.nb;
     const bool add = (__ldcg(f.dirty + unit) >> d) & 1u;
     drain_one<NEAR, R1 / 2>(p, FastSlice<NEAR>(f, unit), dwb / f.n_bands * 32u, j0,
-                            (int)min(f.nb, p.n_omega - j0), p.offsets[t], p.it_start[t], (int)d,
-                            (int)w.y, add, pairs[warp], lane);
+                            (int)min(f.nb, p.n_omega - j0), axis_step(p), p.offsets[t],
+                            p.it_start[t], (int)d, (int)w.y, add, pairs[warp], lane);
     if (lane == 0) atomicOr(f.dirty + unit, 1u << d);
   }
 }
